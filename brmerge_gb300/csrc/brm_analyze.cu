@@ -218,6 +218,10 @@ __global__ void __launch_bounds__(kAnaThreads) k_analyze(CsrDev A, CsrDev B, Pla
             mx = grp_max<TW>(mx, gm);
             if (gl == 0)
                 P.crange[row] = make_int2(mn, mx);
+            // rows placed by rank, where their lists and column range allow
+            const int rc = rank_class(f, a1 - a0, (long long)mx - mn);
+            if (rc >= 0)
+                bin = kBinRank0 + rc;
             if ((bin == kBinMidWarp && (long long)mx - mn >= (1ll << kMwRangeBits)) ||
                 (bin == kBinMidGroup && (long long)mx - mn >= (1ll << kMgRangeBits)) ||
                 ((bin == kBinMidTile || bin == kBinMidTile2) &&
@@ -236,11 +240,7 @@ __global__ void __launch_bounds__(kAnaThreads) k_analyze(CsrDev A, CsrDev B, Pla
             if (bin == kBinHeavy)
                 P.seg_base[row] = atomicAdd(&P.cnt->seg_cap, seg_bound(f, B.N, P.seg_cut));
             P.mid_flop[row] = bin == kBinBatch ? max((int)f, 2 * nl) : 0;  // batch weight
-            P.mw_flop[row] =
-                (bin == kBinMidWarp || bin == kBinMidGroup || bin == kBinMidTile ||
-                 bin == kBinMidTile2 || bin == kBinMidGroup2)
-                    ? (int)f
-                    : 0;
+            P.mw_flop[row] = bin >= kBinMidWarp ? (int)f : 0;
             P.spill[row] = 0;
             if (bin == kBinEmpty)
                 P.nnz[row] = 0;

@@ -631,23 +631,19 @@ __global__ void __launch_bounds__(256) k_mid_compact(PlanDev P, int M, const int
     const int r1 = min(M, P.r_hi);
     // warp and group rows from their row lists, then (only when there are
     // batches) the batched mid rows by a sweep over the rows
-    const int nw1 = P.cnt->bin_count[kBinMidWarp];
-    const int nw4 = P.cnt->bin_count[kBinMidGroup];
-    const int nwt = P.cnt->bin_count[kBinMidTile];
-    const int nwt2 = P.cnt->bin_count[kBinMidTile2];
-    const int nw5 = P.cnt->bin_count[kBinMidGroup2];
-    const int nlist = nw1 + nw4 + nwt + nwt2 + nw5;
+    int nlist = 0;
+#pragma unroll
+    for (int b = kBinMidWarp; b < kNumBins; b++)
+        nlist += P.cnt->bin_count[b];
     const int nsweep = P.cnt->n_batch > 0 ? r1 - P.r_lo : 0;
     for (int it = gw; it < nlist + nsweep; it += nwarps) {
         int row;
         long long src;
         if (it < nlist) {
-            row = it < nw1              ? P.rows[(size_t)kBinMidWarp * M + it]
-                  : it < nw1 + nw4       ? P.rows[(size_t)kBinMidGroup * M + (it - nw1)]
-                  : it < nw1 + nw4 + nwt ? P.rows[(size_t)kBinMidTile * M + (it - nw1 - nw4)]
-                  : it < nw1 + nw4 + nwt + nwt2
-                      ? P.rows[(size_t)kBinMidTile2 * M + (it - nw1 - nw4 - nwt)]
-                      : P.rows[(size_t)kBinMidGroup2 * M + (it - nw1 - nw4 - nwt - nwt2)];
+            int b = kBinMidWarp, i = it;
+            while (i >= P.cnt->bin_count[b])
+                i -= P.cnt->bin_count[b++];
+            row = P.rows[(size_t)b * M + i];
             if (row < P.r_lo || row >= r1)
                 continue;
             src = P.mid_pre[M] + P.mw_pre[row];

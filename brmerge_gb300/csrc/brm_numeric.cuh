@@ -5,7 +5,7 @@
 
 #include "brm_kernels.h"
 #include "brm_mid.cuh"
-#include "brm_midwarp.cuh"
+#include "brm_midrank.cuh"
 #include "brm_seg.cuh"
 #include "brm_rows.cuh"
 

@@ -33,7 +33,8 @@ constexpr int kMidMaxLists = kMidCap / 2;
 constexpr int kMidMaxK = 255;
 constexpr int kMidMaxRows = kMidCap / (kWarpMaxFlop + 1) + 2;
 
-// Warp mid rows: more than kWarpMaxFlop and at most kMwF products, at most
+// Merged mid rows, where the rank rows below do not take them.  Warp mid rows:
+// more than kWarpMaxFlop and at most kMwF products, at most
 // kMwMaxK A entries, columns within a range below 2^kMwRangeBits; one warp
 // each.  Group rows: up to kMgF products and kMwMaxK A entries, range below
 // 2^kMgRangeBits, four warps each; longer group rows (up to kMg2F products,
@@ -51,6 +52,36 @@ constexpr int kMgF = 3072;
 constexpr int kMgRangeBits = 20;
 constexpr int kMg2F = 5888;       // second group class: two groups a CTA fit 2 CTAs an SM
 constexpr int kMg2RangeBits = 19;
+// Rank rows (brm_midrank.cuh): rows of at most 64 lists whose products are
+// placed by population counts instead of sorted; they take precedence over the
+// tile, warp and group rows above, which keep the rows of 65 to 255 lists and
+// the wide ranges (the bitmap's summary outgrows a row's shared memory there).
+// R-MAT n=2^18: rows of 769..3072 products 0.35 -> 0.28 ms, of 3073..5888 0.40
+// -> 0.37 (the rows of more than 32 lists still merged).
+// The most products of a row of each class:
+constexpr int kRkF0 = 128;
+constexpr int kRkF1 = 384;
+constexpr int kRkF2 = 768;
+constexpr int kRkF3 = 1536;
+constexpr int kRkF4 = 3072;
+constexpr int kRkF5 = 6144;
+constexpr int kRkNarrowK = 32;      // lists of the rows with one mask word a column
+constexpr int kRkMaxK = 64;
+constexpr int kRkRangeBits0 = 18;   // column range, class 0
+constexpr int kRkRangeBits = 19;    // the others
+// The class of a row of f products, k lists and columns within `range` of the
+// first, -1 where it has none.
+__host__ __device__ inline int rank_class(long long f, int k, long long range)
+{
+    if (f <= 0 || f > kRkF5 || k > kRkMaxK || range < 0 || range >= (1ll << kRkRangeBits))
+        return -1;
+    if (k <= kRkNarrowK) {
+        if (f <= kRkF0)
+            return range < (1ll << kRkRangeBits0) ? 0 : -1;
+        return f <= kRkF1 ? 1 : f <= kRkF2 ? 2 : f <= kRkF3 ? 3 : f <= kRkF4 ? 4 : 5;
+    }
+    return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f <= kRkF4 ? 7 : -1;
+}
 // Subsets of the mid-row kernels (they can run on different streams).
 constexpr int kMidGroups = 1;     // the batched mid rows and the four-warp group rows
 constexpr int kMidWarps = 2;      // the warp and tile rows
@@ -111,8 +142,14 @@ enum RowBin : int {
     kBinMidTile = 8,  // half a warp per row, products sorted in registers (brm_midwarp.cuh)
     kBinMidTile2 = 9, // the same with twice the products
     kBinMidGroup2 = 10,  // four warps per row, longer rows (brm_midwarp.cuh)
-    kNumBins = 11,
+    kBinRank0 = 11,      // rank rows, classes 0 .. 7 (brm_midrank.cuh)
+    kNumBins = 19,
 };
+
+constexpr int kRankClasses = kNumBins - kBinRank0;
+// work counters of the mid-row kernels: the merge shapes, then the rank classes
+constexpr int kMwRankCounter = 3;
+constexpr int kMwCounters = kMwRankCounter + kRankClasses;
 
 // Device counters (one struct in device memory, zeroed per phase).
 struct Counters {
@@ -152,8 +189,8 @@ struct Counters {
     // shape) and the groups of a launch that have finished; the last group
     // of a launch sets both back to zero, so every launch starts from zero
     // whatever phase or pipeline runs it
-    int work_mw[3];
-    int done_mw[3];
+    int work_mw[kMwCounters];
+    int done_mw[kMwCounters];
 };
 
 // Descriptor slots reserved for a heavy row with F products and the cut
@@ -278,7 +315,8 @@ constexpr unsigned kLiveAll = 0xffffffffu;
 constexpr unsigned live_bit(int bin) { return 1u << bin; }
 constexpr unsigned kLiveMidRows = live_bit(kBinBatch) | live_bit(kBinMidWarp) |
                                   live_bit(kBinMidGroup) | live_bit(kBinMidTile) |
-                                  live_bit(kBinMidTile2) | live_bit(kBinMidGroup2);
+                                  live_bit(kBinMidTile2) | live_bit(kBinMidGroup2) |
+                                  (live_bit(kNumBins) - live_bit(kBinRank0));
 inline bool plan_live(const PlanDev &P, unsigned bits) { return (P.live & bits) != 0; }
 
 // Capacities of a captured batch pipeline: every buffer sized by a count the

@@ -1,7 +1,7 @@
 // brm_symbolic.cu -- symbolic phase launchers (exact row nnz, spill routing).
 #include "brm_kernels.h"
 #include "brm_mid.cuh"
-#include "brm_midwarp.cuh"
+#include "brm_midrank.cuh"
 #include "brm_rows.cuh"
 #include "brm_seg.cuh"
 
