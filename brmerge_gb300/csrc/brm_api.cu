@@ -840,7 +840,7 @@ int host_call(bool upper, const int *arpt, const int *acol, const T *aval, const
         BRM_TRY(alloc_results());
         t_num0 = now_sec();
         ev_record(ctx, timed, kEvCopy0);
-        brm::launch_compact(dtype == BRM_F64 ? 0 : 1, ctx->plan, (const int *)ctx->bar_col.p,
+        brm::launch_compact(dtype == BRM_F64 ? 0 : 1, ctx->plan, cnnz, (const int *)ctx->bar_col.p,
                             ctx->bar_val.p, (const int *)ctx->io_crpt.p, dcol, dval, s);
         ev_record(ctx, timed, kEvCopy1);
         BRM_CK(cudaGetLastError());
@@ -1422,7 +1422,7 @@ int brm_upper_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const b
     }
     double t4 = now_sec();
     ev_record(ctx, timed, kEvCopy0);
-    brm::launch_compact(dtype == BRM_F64 ? 0 : 1, ctx->plan, (const int *)ctx->bar_col.p,
+    brm::launch_compact(dtype == BRM_F64 ? 0 : 1, ctx->plan, cnnz, (const int *)ctx->bar_col.p,
                         ctx->bar_val.p, crpt, ccol, cval, ctx->stream);
     ev_record(ctx, timed, kEvCopy1);
     st = read_err(ctx);

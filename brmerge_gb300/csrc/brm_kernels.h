@@ -89,8 +89,9 @@ void launch_symbolic(const CsrDev &A, const CsrDev &B, const PlanDev &P, int num
 void launch_seg_partition(const PlanDev &P, const int *pb, int nparts, int *cnt, int *fill,
                           int *out, int *ranges, int num_sms, cudaStream_t s);
 
-// Upper compaction: C[crpt[i]..] = C_bar[scan_flop[i]..] (spgemm.h:429-444).
-void launch_compact(int dtype, const PlanDev &P, const int *bar_col, const void *bar_val,
+// Upper compaction: C[crpt[i]..] = C_bar[scan_flop[i]..] (spgemm.h:429-444),
+// nnz entries.
+void launch_compact(int dtype, const PlanDev &P, int nnz, const int *bar_col, const void *bar_val,
                     const int *crpt, int *ccol, void *cval, cudaStream_t s);
 
 // Input validation: row pointers monotone and in range, columns in range and
