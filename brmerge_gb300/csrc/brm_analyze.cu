@@ -49,249 +49,271 @@ __device__ __forceinline__ T grp_min(T v, unsigned gm)
     return v;
 }
 
-// A group of TW lanes per row (TW = 8 when rows are short, 32 otherwise),
-// kAnaRowsPerGroup rows per group.  With TW = 8, rows of more than
-// kAnaLongK entries are listed and left to a second, warp-wide pass
-// (LISTED: the rows are P.longk_rows[0 .. n_longk)).
+// Rows of more than kAnaLongK entries are left, by groups of fewer than 32
+// lanes, to the block's whole warps (a second pass in the same launch).
 constexpr int kAnaLongK = 64;
 
-template <int TW, bool LISTED>
+// What a block gathers of its rows before it takes places in the global lists.
+template <int RPB>
+struct AnaBlock {
+    int cnt[kNumBins];
+    int base[kNumBins];
+    int bin[RPB];
+    int idx[RPB];
+    unsigned long long off[RPB];   // place among the block's scratch entries
+    unsigned long long foff[RPB];  // place among the block's products
+    int longs[RPB];
+    int nlong;
+    int max_k;
+    unsigned long long mw, mid, flop, mw_base, flop_base;
+};
+
+// One row by a group of TW lanes (lane gl of it, mask gm): its products, list
+// table entries (P.abs, P.alen), class and column range.  LONG: eight entries
+// a lane in flight, and the first and last column of every list (the column
+// range) taken in the same pass, so their long lists are walked once.
+template <int TW, bool LONG, int RPB>
+__device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, const PlanDev &P,
+                                            int row, int slot, int gl, unsigned gm,
+                                            AnaBlock<RPB> &S)
+{
+    const int M = A.M, K = B.M;
+    int a0 = A.rpt[row];
+    int a1 = A.rpt[row + 1];
+    long long f = 0;
+    int nl = 0, leaf = -1;
+    bool bad = false;
+    if (a0 < 0 || a1 < a0 || a1 > A.nnz) {  // malformed row pointers: treat the row as empty
+        bad = true;
+        a0 = a1 = 0;
+    }
+    constexpr int UN = LONG ? 8 : 4;
+    int mn = INT_MAX, mx = -1;
+    for (int jb = a0 + gl; jb < a1; jb += UN * TW) {
+        int b[UN], bs[UN], be[UN];
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            const int j = jb + u * TW;
+            b[u] = j < a1 ? A.col[j] : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            const int j = jb + u * TW;
+            bs[u] = be[u] = 0;
+            if (j < a1) {
+                if ((unsigned)b[u] < (unsigned)K) {
+                    bs[u] = B.rpt[b[u]];
+                    be[u] = B.rpt[b[u] + 1];
+                } else {
+                    bad = true;
+                }
+            }
+        }
+        if (LONG) {
+            int c0[UN], c1[UN];
+#pragma unroll
+            for (int u = 0; u < UN; u++) {
+                c0[u] = INT_MAX;
+                c1[u] = -1;
+                if (be[u] > bs[u]) {
+                    c0[u] = B.col[bs[u]];
+                    c1[u] = B.col[be[u] - 1];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < UN; u++) {
+                mn = min(mn, c0[u]);
+                mx = max(mx, c1[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UN; u++) {
+            const int j = jb + u * TW;
+            if (j < a1) {
+                const int len = be[u] - bs[u];
+                P.abs[j] = bs[u];
+                P.alen[j] = len;
+                f += len;
+                if (len > 0) {
+                    nl++;
+                    leaf = max(leaf, j - a0);
+                }
+            }
+        }
+    }
+    f = grp_sum<TW>(f, gm);
+    nl = grp_sum<TW>(nl, gm);
+    leaf = grp_max<TW>(leaf, gm);
+    bad = (__ballot_sync(gm, bad) & gm) != 0u;
+    const bool ovf = f > INT_MAX;
+    if (ovf)
+        f = INT_MAX;
+    // row class (f, nl, a0, a1 are uniform in the group)
+    int bin;
+    if (f == 0)
+        bin = kBinEmpty;
+    else if (nl == 1)
+        bin = kBinCopy;
+    else if (f <= kWarpMaxFlop)
+        bin = kBinWarp;
+    else if (f <= kMg2F && a1 - a0 <= kMidMaxK)  // unless the column range is too wide
+        bin = f <= kMtF    ? kBinMidTile
+              : f <= kMt2F ? kBinMidTile2
+              : (f <= kMwF && a1 - a0 <= kMwMaxK) ? kBinMidWarp
+              : (f <= kMgF && a1 - a0 <= kMwMaxK) ? kBinMidGroup
+                           : kBinMidGroup2;
+    else if (f <= P.mid_limit && 2 * nl <= P.mid_limit && a1 - a0 <= kMidMaxK)
+        bin = kBinBatch;
+    else if (a1 - a0 <= kSegMaxK)
+        bin = kBinHeavy;  // segmented (brm_seg.cuh)
+    else
+        bin = kBinMid;    // row CTA / spill path
+    if (bin == kBinHeavy || bin >= kBinMidWarp) {
+        // column range of the row for the segment planning and the mid rows'
+        // keys and bitmaps: the first and last column of every nonempty list
+        for (int jb = a0 + gl; !LONG && jb < a1; jb += 4 * TW) {
+            int c0[4], c1[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int j = jb + u * TW;
+                c0[u] = INT_MAX;
+                c1[u] = -1;
+                if (j < a1) {
+                    const int len = P.alen[j];
+                    if (len > 0) {
+                        const int bs = P.abs[j];
+                        c0[u] = B.col[bs];
+                        c1[u] = B.col[bs + len - 1];
+                    }
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                mn = min(mn, c0[u]);
+                mx = max(mx, c1[u]);
+            }
+        }
+        mn = grp_min<TW>(mn, gm);
+        mx = grp_max<TW>(mx, gm);
+        if (gl == 0)
+            P.crange[row] = make_int2(mn, mx);
+        // rows placed by rank, where their lists and column range allow
+        const int rc = rank_class(f, a1 - a0, (long long)mx - mn);
+        if (rc >= 0)
+            bin = kBinRank0 + rc;
+        if ((bin == kBinMidWarp && (long long)mx - mn >= (1ll << kMwRangeBits)) ||
+            (bin == kBinMidGroup && (long long)mx - mn >= (1ll << kMgRangeBits)) ||
+            ((bin == kBinMidTile || bin == kBinMidTile2) &&
+             (long long)mx - mn >= (1ll << kMtRangeBits)) ||
+            (bin == kBinMidGroup2 && (long long)mx - mn >= (1ll << kMg2RangeBits)))
+            bin = (f <= P.mid_limit && 2 * nl <= P.mid_limit) ? kBinBatch : kBinHeavy;
+        if (bin == kBinHeavy && a1 - a0 > kSegMaxK)
+            bin = kBinMid;
+    }
+    if (gl != 0)
+        return;
+    if (bad)
+        atomicOr(&P.cnt->err, kErrBadInput);
+    if (ovf)
+        atomicOr(&P.cnt->err, kErrOverflow);
+    P.flop[row] = (int)f;
+    if (bin == kBinHeavy)
+        P.seg_base[row] = atomicAdd(&P.cnt->seg_cap, seg_bound(f, B.N, P.seg_cut));
+    const int weight = bin == kBinBatch ? max((int)f, 2 * nl) : 0;  // batch weight
+    P.mid_flop[row] = weight;
+    P.spill[row] = 0;
+    if (bin == kBinEmpty)
+        P.nnz[row] = 0;
+    else if (bin == kBinCopy) {
+        P.nnz[row] = (int)f;
+        P.copy_leaf[row] = leaf;
+    }
+    if (bin == kBinHeavy && f > kHugeFlop) {
+        // the planning takes these first, so the longest rows do not
+        // start last and finish after every other block
+        const int h = atomicAdd(&P.cnt->n_huge, 1);
+        if (BRM_IN(P.cnt, M - 1 - h, M))
+            P.rows[(size_t)kBinHeavy * M + (M - 1 - h)] = row;
+        bin = -2;
+    }
+    S.bin[slot] = bin;
+    S.idx[slot] = bin < 0 || bin == kBinEmpty ? 0 : atomicAdd(&S.cnt[bin], 1);
+    S.foff[slot] = atomicAdd(&S.flop, (unsigned long long)f);
+    if (bin == kBinWarp || bin >= kBinMidWarp)
+        S.off[slot] = atomicAdd(&S.mw, (unsigned long long)f);
+    if (weight)
+        atomicAdd(&S.mid, (unsigned long long)weight);
+    atomicMax(&S.max_k, a1 - a0);
+}
+
+// A group of TW lanes per row (TW = 8 when rows are short, 32 otherwise),
+// kAnaRowsPerGroup rows per group.
+template <int TW>
 __global__ void __launch_bounds__(kAnaThreads) k_analyze(CsrDev A, CsrDev B, PlanDev P)
 {
     constexpr int NW = kAnaThreads / 32;
     constexpr int NGR = kAnaThreads / TW;  // groups per block
-    constexpr int RPG = LISTED ? 1 : kAnaRowsPerGroup;  // rows per group (one listed long row)
-    constexpr int RPB = NGR * RPG;
-    __shared__ int s_cnt[kNumBins];
-    __shared__ int s_base[kNumBins];
-    __shared__ int s_bin[RPB];
-    __shared__ int s_idx[RPB];
-    __shared__ unsigned long long s_flop[NW];
-    __shared__ int s_maxk[NW];
+    constexpr int RPB = NGR * kAnaRowsPerGroup;
+    __shared__ AnaBlock<RPB> S;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int gl = threadIdx.x & (TW - 1);    // lane in the group
     const int grp = threadIdx.x / TW;         // group in the block
     const unsigned gm = TW == 32 ? kFull : (((1u << TW) - 1u) << (lane & ~(TW - 1)));
     if (threadIdx.x < kNumBins)
-        s_cnt[threadIdx.x] = 0;
-    __syncthreads();
-    const int M = A.M, K = B.M;
-    const int nrows = LISTED ? P.cnt->n_longk : M;
-    const int row0 = blockIdx.x * RPB;
-    unsigned long long gflop = 0;
-    int gmaxk = 0;
-    for (int r = 0; r < RPG; r++) {
-        const int slot = grp * RPG + r;
-        if (row0 + slot >= nrows) {
-            if (gl == 0)
-                s_bin[slot] = -1;
-            continue;
-        }
-        const int row = LISTED ? P.longk_rows[row0 + slot] : row0 + slot;
-        int a0 = A.rpt[row];
-        int a1 = A.rpt[row + 1];
-        if (TW < 32 && a1 - a0 > kAnaLongK && a0 >= 0 && a1 <= A.nnz) {
-            if (gl == 0) {
-                P.longk_rows[atomicAdd(&P.cnt->n_longk, 1)] = row;
-                s_bin[slot] = -1;
-            }
-            continue;
-        }
-        long long f = 0;
-        int nl = 0, leaf = -1;
-        bool bad = false;
-        if (a0 < 0 || a1 < a0 || a1 > A.nnz) {  // malformed row pointers: treat the row as empty
-            bad = true;
-            a0 = a1 = 0;
-        }
-        // UN entries a lane in flight; the listed long rows also take the
-        // first and last column of every nonempty list in the same pass (the
-        // column range), so their long lists are walked once
-        constexpr int UN = LISTED ? 8 : 4;
-        int mn = INT_MAX, mx = -1;
-        for (int jb = a0 + gl; jb < a1; jb += UN * TW) {
-            int b[UN], bs[UN], be[UN];
-#pragma unroll
-            for (int u = 0; u < UN; u++) {
-                const int j = jb + u * TW;
-                b[u] = j < a1 ? A.col[j] : -1;
-            }
-#pragma unroll
-            for (int u = 0; u < UN; u++) {
-                const int j = jb + u * TW;
-                bs[u] = be[u] = 0;
-                if (j < a1) {
-                    if ((unsigned)b[u] < (unsigned)K) {
-                        bs[u] = B.rpt[b[u]];
-                        be[u] = B.rpt[b[u] + 1];
-                    } else {
-                        bad = true;
-                    }
-                }
-            }
-            if (LISTED) {
-                int c0[UN], c1[UN];
-#pragma unroll
-                for (int u = 0; u < UN; u++) {
-                    c0[u] = INT_MAX;
-                    c1[u] = -1;
-                    if (be[u] > bs[u]) {
-                        c0[u] = B.col[bs[u]];
-                        c1[u] = B.col[be[u] - 1];
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < UN; u++) {
-                    mn = min(mn, c0[u]);
-                    mx = max(mx, c1[u]);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < UN; u++) {
-                const int j = jb + u * TW;
-                if (j < a1) {
-                    const int len = be[u] - bs[u];
-                    P.abs[j] = bs[u];
-                    P.alen[j] = len;
-                    f += len;
-                    if (len > 0) {
-                        nl++;
-                        leaf = max(leaf, j - a0);
-                    }
-                }
-            }
-        }
-        f = grp_sum<TW>(f, gm);
-        nl = grp_sum<TW>(nl, gm);
-        leaf = grp_max<TW>(leaf, gm);
-        bad = (__ballot_sync(gm, bad) & gm) != 0u;
-        const bool ovf = f > INT_MAX;
-        if (ovf)
-            f = INT_MAX;
-        // row class (f, nl, a0, a1 are uniform in the group)
-        int bin;
-        if (f == 0)
-            bin = kBinEmpty;
-        else if (nl == 1)
-            bin = kBinCopy;
-        else if (f <= kWarpMaxFlop)
-            bin = kBinWarp;
-        else if (f <= kMg2F && a1 - a0 <= kMidMaxK)  // unless the column range is too wide
-            bin = f <= kMtF    ? kBinMidTile
-                  : f <= kMt2F ? kBinMidTile2
-                  : (f <= kMwF && a1 - a0 <= kMwMaxK) ? kBinMidWarp
-                  : (f <= kMgF && a1 - a0 <= kMwMaxK) ? kBinMidGroup
-                               : kBinMidGroup2;
-        else if (f <= P.mid_limit && 2 * nl <= P.mid_limit && a1 - a0 <= kMidMaxK)
-            bin = kBinBatch;
-        else if (a1 - a0 <= kSegMaxK)
-            bin = kBinHeavy;  // segmented (brm_seg.cuh)
-        else
-            bin = kBinMid;    // row CTA / spill path
-        if (bin == kBinHeavy || bin == kBinMidWarp || bin == kBinMidGroup || bin == kBinMidTile ||
-            bin == kBinMidTile2 || bin == kBinMidGroup2) {
-            // column range of the row for the segment planning and the warp
-            // mid rows' keys: the first and last column of every nonempty list
-            for (int jb = a0 + gl; !LISTED && jb < a1; jb += 4 * TW) {
-                int c0[4], c1[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int j = jb + u * TW;
-                    c0[u] = INT_MAX;
-                    c1[u] = -1;
-                    if (j < a1) {
-                        const int len = P.alen[j];
-                        if (len > 0) {
-                            const int bs = P.abs[j];
-                            c0[u] = B.col[bs];
-                            c1[u] = B.col[bs + len - 1];
-                        }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    mn = min(mn, c0[u]);
-                    mx = max(mx, c1[u]);
-                }
-            }
-            mn = grp_min<TW>(mn, gm);
-            mx = grp_max<TW>(mx, gm);
-            if (gl == 0)
-                P.crange[row] = make_int2(mn, mx);
-            // rows placed by rank, where their lists and column range allow
-            const int rc = rank_class(f, a1 - a0, (long long)mx - mn);
-            if (rc >= 0)
-                bin = kBinRank0 + rc;
-            if ((bin == kBinMidWarp && (long long)mx - mn >= (1ll << kMwRangeBits)) ||
-                (bin == kBinMidGroup && (long long)mx - mn >= (1ll << kMgRangeBits)) ||
-                ((bin == kBinMidTile || bin == kBinMidTile2) &&
-                 (long long)mx - mn >= (1ll << kMtRangeBits)) ||
-                (bin == kBinMidGroup2 && (long long)mx - mn >= (1ll << kMg2RangeBits)))
-                bin = (f <= P.mid_limit && 2 * nl <= P.mid_limit) ? kBinBatch : kBinHeavy;
-            if (bin == kBinHeavy && a1 - a0 > kSegMaxK)
-                bin = kBinMid;
-        }
-        if (gl == 0) {
-            if (bad)
-                atomicOr(&P.cnt->err, kErrBadInput);
-            if (ovf)
-                atomicOr(&P.cnt->err, kErrOverflow);
-            P.flop[row] = (int)f;
-            if (bin == kBinHeavy)
-                P.seg_base[row] = atomicAdd(&P.cnt->seg_cap, seg_bound(f, B.N, P.seg_cut));
-            P.mid_flop[row] = bin == kBinBatch ? max((int)f, 2 * nl) : 0;  // batch weight
-            P.mw_flop[row] = bin >= kBinMidWarp ? (int)f : 0;
-            P.spill[row] = 0;
-            if (bin == kBinEmpty)
-                P.nnz[row] = 0;
-            else if (bin == kBinCopy) {
-                P.nnz[row] = (int)f;
-                P.copy_leaf[row] = leaf;
-            }
-            if (bin == kBinHeavy && f > kHugeFlop) {
-                // the planning takes these first, so the longest rows do not
-                // start last and finish after every other block
-                const int h = atomicAdd(&P.cnt->n_huge, 1);
-                if (BRM_IN(P.cnt, M - 1 - h, M))
-                    P.rows[(size_t)kBinHeavy * M + (M - 1 - h)] = row;
-                bin = -2;
-            }
-            s_bin[slot] = bin;
-            s_idx[slot] = (bin < 0 || bin == kBinEmpty || bin == kBinBatch) ? 0 : atomicAdd(&s_cnt[bin], 1);
-            gflop += (unsigned long long)f;
-            gmaxk = max(gmaxk, a1 - a0);
-        }
-    }
-    // per warp: the groups' totals (held by their first lanes)
-    {
-        unsigned long long wf = grp_sum<32>(gflop, kFull);
-        int wk = grp_max<32>(gmaxk, kFull);
-        if (lane == 0) {
-            s_flop[w] = wf;
-            s_maxk[w] = wk;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < kNumBins)
-        s_base[threadIdx.x] =
-            s_cnt[threadIdx.x] ? atomicAdd(&P.cnt->bin_count[threadIdx.x], s_cnt[threadIdx.x]) : 0;
+        S.cnt[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
-        unsigned long long t = 0;
-        int mk = 0;
-        for (int i = 0; i < NW; i++) {
-            t += s_flop[i];
-            mk = max(mk, s_maxk[i]);
+        S.nlong = S.max_k = 0;
+        S.mw = S.mid = S.flop = 0;
+    }
+    __syncthreads();
+    const int M = A.M;
+    const int row0 = blockIdx.x * RPB;
+    for (int r = 0; r < kAnaRowsPerGroup; r++) {
+        const int slot = grp * kAnaRowsPerGroup + r;
+        const int row = row0 + slot;
+        if (row >= M) {
+            if (gl == 0)
+                S.bin[slot] = -1;
+            continue;
         }
-        if (t)
-            atomicAdd(&P.cnt->total_flop, t);
-        atomicMax(&P.cnt->max_k, mk);
+        const int a0 = A.rpt[row], a1 = A.rpt[row + 1];
+        if (TW < 32 && a1 - a0 > kAnaLongK && a0 >= 0 && a1 <= A.nnz) {
+            if (gl == 0)
+                S.longs[atomicAdd(&S.nlong, 1)] = slot;
+            continue;
+        }
+        analyze_row<TW, false, RPB>(A, B, P, row, slot, gl, gm, S);
+    }
+    __syncthreads();
+    if (TW < 32 && S.nlong) {
+        for (int i = w; i < S.nlong; i += NW)
+            analyze_row<32, true, RPB>(A, B, P, row0 + S.longs[i], S.longs[i], lane, kFull, S);
+        __syncthreads();
+    }
+    if (threadIdx.x < kNumBins)
+        S.base[threadIdx.x] =
+            S.cnt[threadIdx.x] ? atomicAdd(&P.cnt->bin_count[threadIdx.x], S.cnt[threadIdx.x]) : 0;
+    if (threadIdx.x == 32) {
+        S.flop_base = S.flop ? atomicAdd(&P.cnt->total_flop, S.flop) : 0ull;
+        S.mw_base = S.mw ? atomicAdd(&P.cnt->mw_total, S.mw) : 0ull;
+        if (S.mid)
+            atomicAdd(&P.cnt->mid_total, S.mid);
+        if (S.max_k > 0)
+            atomicMax(&P.cnt->max_k, S.max_k);
     }
     __syncthreads();
     for (int slot = threadIdx.x; slot < RPB; slot += kAnaThreads) {
-        int bin = s_bin[slot];
-        if (bin > kBinEmpty && bin != kBinBatch && BRM_IN(P.cnt, s_base[bin] + s_idx[slot], M))
-            P.rows[(size_t)bin * M + s_base[bin] + s_idx[slot]] =
-                LISTED ? P.longk_rows[row0 + slot] : row0 + slot;
+        const int bin = S.bin[slot], row = row0 + slot;
+        if (bin == -1)
+            continue;
+        if (P.upper)
+            P.scan_flop[row] = (long long)(S.flop_base + S.foff[slot]);
+        if (bin <= kBinEmpty || bin == kBinBatch)
+            continue;
+        if (bin == kBinWarp || bin >= kBinMidWarp)
+            P.mw_pre[row] = (long long)(S.mw_base + S.off[slot]);
+        if (BRM_IN(P.cnt, S.base[bin] + S.idx[slot], M))
+            P.rows[(size_t)bin * M + S.base[bin] + S.idx[slot]] = row;
     }
 }
 
@@ -300,29 +322,28 @@ void launch_analyze(const CsrDev &A, const CsrDev &B, const PlanDev &P, cudaStre
     if (A.M <= 0)
         return;
     constexpr int RPB32 = (kAnaThreads / 32) * kAnaRowsPerGroup;
-    // eight lanes a row when rows average at most 12 entries; the few long
-    // rows then go to a warp-wide pass over their list (at most all rows)
+    // eight lanes a row when rows average at most 12 entries
     if ((long long)A.nnz <= 12ll * A.M) {
         constexpr int RPB = (kAnaThreads / 8) * kAnaRowsPerGroup;
-        k_analyze<8, false><<<(A.M + RPB - 1) / RPB, kAnaThreads, 0, s>>>(A, B, P);
-        count_launch();
-        const long long most = std::min<long long>(A.M, (long long)A.nnz / (kAnaLongK + 1));
-        constexpr int RPBL = kAnaThreads / 32;  // one listed row per warp
-        const int g = (int)std::max<long long>(1, (most + RPBL - 1) / RPBL);
-        k_analyze<32, true><<<g, kAnaThreads, 0, s>>>(A, B, P);
+        k_analyze<8><<<(A.M + RPB - 1) / RPB, kAnaThreads, 0, s>>>(A, B, P);
     } else {
-        k_analyze<32, false><<<(A.M + RPB32 - 1) / RPB32, kAnaThreads, 0, s>>>(A, B, P);
+        k_analyze<32><<<(A.M + RPB32 - 1) / RPB32, kAnaThreads, 0, s>>>(A, B, P);
     }
     count_launch();
 }
 
 // ---------------------------------------------------------------------------
-// Exclusive scan (reduce, scan of tile sums, downsweep), out[n] = total.
-// Replaces opt_prefix_sum (spgemm.h:179-187) for crpt and scan_floprC.
+// Exclusive scan, out[n] = total, in two launches (tile sums, then every block
+// adds up the sums before its tile), or in one where the blocks before a tile
+// are few enough for it to add up their items itself.  Replaces
+// opt_prefix_sum (spgemm.h:179-187) for crpt.
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 512;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
+// tiles up to which one launch does it: the last block then reads at most
+// 28672 items before its own, which takes less than a launch
+constexpr int kScanOneLaunch = 8;
 
 __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int *in, int n,
                                                               long long *tile_sums)
@@ -341,24 +362,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_reduce(const int *in, int
         tile_sums[blockIdx.x] = t;
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(long long *tile_sums, int ntiles)
-{
-    __shared__ long long ws[kScanThreads / 32 + 1];
-    long long carry = 0;
-    for (int base = 0; base < ntiles; base += kScanThreads) {
-        int idx = base + threadIdx.x;
-        long long v = idx < ntiles ? tile_sums[idx] : 0;
-        long long tot;
-        long long ex = block_excl_scan<kScanThreads>(v, ws, &tot);
-        if (idx < ntiles)
-            tile_sums[idx] = carry + ex;
-        carry += tot;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        tile_sums[ntiles] = carry;
-}
-
+// tile_sums: the tiles' sums, or nullptr to add up the items before the tile.
 template <typename OutT>
 __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int *in, int n,
                                                             const long long *tile_sums,
@@ -366,6 +370,15 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int *in, int n
 {
     __shared__ long long ws[kScanThreads / 32 + 1];
     const long long base = (long long)blockIdx.x * kScanTile;
+    long long before = 0;
+    if (tile_sums) {
+        for (int i = threadIdx.x; i < (int)blockIdx.x; i += kScanThreads)
+            before += tile_sums[i];
+    } else {
+#pragma unroll 8
+        for (long long i = threadIdx.x; i < base; i += kScanThreads)
+            before += in[i];
+    }
     // blocked arrangement: thread t owns items [t*I, t*I+I) of the tile
     long long v[kScanItems];
     long long s = 0;
@@ -375,9 +388,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int *in, int n
         v[i] = idx < n ? in[idx] : 0;
         s += v[i];
     }
+    before = block_sum<kScanThreads>(before, ws);
+    __syncthreads();
     long long tot;
     long long ex = block_excl_scan<kScanThreads>(s, ws, &tot);
-    long long run = tile_sums[blockIdx.x] + ex;
+    long long run = before + ex;
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         long long idx = base + (long long)threadIdx.x * kScanItems + i;
@@ -393,7 +408,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_down(const int *in, int n
         run += v[i];
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
-        long long total = tile_sums[gridDim.x];
+        long long total = before + tot;
         if (cnt)
             cnt->cnnz = total;
         if (sizeof(OutT) == 4 && total > INT_MAX) {
@@ -419,10 +434,12 @@ static void scan_impl(const int *in, OutT *out, int n, Counters *cnt, void *tmp,
     int tiles = (n + kScanTile - 1) / kScanTile;
     if (tiles == 0)
         tiles = 1;
-    k_scan_reduce<<<tiles, kScanThreads, 0, s>>>(in, n, ts);
-    count_launch();
-    k_scan_tiles<<<1, kScanThreads, 0, s>>>(ts, tiles);
-    count_launch();
+    if (tiles <= kScanOneLaunch) {
+        ts = nullptr;
+    } else {
+        k_scan_reduce<<<tiles, kScanThreads, 0, s>>>(in, n, ts);
+        count_launch();
+    }
     k_scan_down<OutT><<<tiles, kScanThreads, 0, s>>>(in, n, ts, out, cnt);
     count_launch();
 }
@@ -598,7 +615,7 @@ __global__ void k_pipe_admit(PlanDev P, int M, PipeCaps caps, int stage)
     bool bad;
     if (stage == 0)
         bad = (long long)c->total_flop > caps.products || (long long)c->seg_cap > caps.seg_slots ||
-              P.mid_pre[M] + P.mw_pre[M] > caps.products;
+              (long long)(c->mw_total + c->mid_total) > caps.products + caps.nnz_a;
     else
         bad = (long long)c->table_cap > caps.table || (long long)c->spill_bytes > caps.spill_bytes;
     if (bad) {

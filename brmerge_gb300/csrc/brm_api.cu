@@ -79,7 +79,6 @@ struct brm_context_s {
     int *d_bad = nullptr;
     brm::Counters *h_cnt = nullptr;  // pinned mirror of the device counters
     int *h_bad = nullptr;            // pinned
-    long long *h_mid = nullptr;      // pinned: entries of the mid-row scratch (batched, warp)
     // per-A-entry list metadata (B-row start and length)
     DevBuf ameta;
     // heavy-row segments: descriptors + written list, the split table and the
@@ -90,6 +89,11 @@ struct brm_context_s {
     int *mid_col = nullptr;
     void *mid_val = nullptr;
     bool mid_ready = false;
+    // the plan has cleared the counters of the numeric phase and nothing has
+    // used them since
+    bool fresh = false;
+    // nnz(C) and the plan's errors are still on the device (plan_phase)
+    bool deferred = false;
     // spill scratch
     DevBuf spill;
     // Upper upper-bound buffer
@@ -187,12 +191,10 @@ size_t workspace_bytes(int M)
     b += a256(m);                           // spill flags
     b += a256(4 * m);                       // spill_rows
     b += a256(8 * m);                       // spill_off
-    b += a256(8 * (m + 1));                 // scan_flop
+    b += a256(8 * m);                       // scan_flop
     b += a256(4 * m);                       // mid_flop
     b += a256(8 * (m + 1));                 // mid_pre
-    b += a256(4 * m);                       // mw_flop
-    b += a256(8 * (m + 1));                 // mw_pre
-    b += a256(4 * m);                       // longk_rows
+    b += a256(8 * m);                       // mw_pre
     b += a256(4 * (m + 1));                 // batch_start
     b += a256(8 * m);                       // seg_base
     b += a256(4 * m);                       // seg_n
@@ -235,12 +237,10 @@ int ensure_workspace(brm_context ctx, int M)
     P.spill = (unsigned char *)take(m);
     P.spill_rows = (int *)take(4 * m);
     P.spill_off = (unsigned long long *)take(8 * m);
-    P.scan_flop = (long long *)take(8 * (m + 1));
+    P.scan_flop = (long long *)take(8 * m);
     P.mid_flop = (int *)take(4 * m);
     P.mid_pre = (long long *)take(8 * (m + 1));
-    P.mw_flop = (int *)take(4 * m);
-    P.mw_pre = (long long *)take(8 * (m + 1));
-    P.longk_rows = (int *)take(4 * m);
+    P.mw_pre = (long long *)take(8 * m);
     P.batch_start = (int *)take(4 * (m + 1));
     P.seg_base = (unsigned long long *)take(8 * m);
     P.seg_n = (int *)take(4 * m);
@@ -336,10 +336,10 @@ double ev_sec(brm_context ctx, int a, int b)
 }
 
 // Planning phase fields of the timing structs, from the events of a timed
-// plan_phase.  Precise: compute_flop = row analysis and binning,
-// prefix_sum_flop = prefix sums of the mid-row products and batch starts,
-// load_balance = host read of the bin counts and sizing of the segment and
-// scratch buffers, symbolic = exact row nnz (heavy-row planning included),
+// plan_phase.  Precise: compute_flop = row analysis, binning and offsets,
+// prefix_sum_flop = copy of the totals and class counts to the host,
+// load_balance = the wait for it and sizing of the segment and scratch
+// buffers, symbolic = exact row nnz (heavy-row planning included),
 // prefix_sum_nnz = crpt scan.
 void plan_times(brm_context ctx, brm_precise_timing *t)
 {
@@ -351,7 +351,7 @@ void plan_times(brm_context ctx, brm_precise_timing *t)
 }
 
 // Upper (spgemm.h:220-457 has no symbolic pass): compute_flop = row
-// analysis, prefix_sum_flop = the mid-row prefix sums and the scan_flop scan,
+// analysis and offsets, prefix_sum_flop = copy of the totals to the host,
 // load_balance = buffer sizing plus the heavy-row planning that cuts long
 // rows into balanced segments.
 void plan_times_upper(brm_context ctx, brm_upper_timing *t)
@@ -361,15 +361,56 @@ void plan_times_upper(brm_context ctx, brm_upper_timing *t)
     t->load_balance = ev_sec(ctx, kEvPre, kEvSym);
 }
 
+// Products up to which a one-call Precise allocates C for every product (24
+// MB in float64) instead of waiting for nnz(C): one host round trip less where
+// a whole call takes about 100 us (the ER product of 2^20 products 0.205 ->
+// 0.114 ms with it and the launches saved).
+constexpr unsigned long long kDeferProducts = 2ull << 20;
+
+// Few rows: the smaller rank classes go along in the launch of the largest
+// that has rows, as long as its groups of warps hold all rows at once (a
+// launch costs about 5 us and each class at least 15 us on its own, rows of
+// another class a little more than in theirs).
+void plan_rank_spans(brm::PlanDev &P, const brm::Counters &c, int num_sms)
+{
+    // rows of each narrow class on one SM at a time (brm_midrank.cuh)
+    constexpr int kRows[6] = {40, 24, 10, 7, 4, 2};
+    std::memset(P.rank_span, 0, sizeof(P.rank_span));
+    P.rank_taken = 0;
+    auto take = [&](int lo, int hi) {  // classes lo .. hi: true when one takes them all
+        int top = -1;
+        long long rows = 0;
+        for (int k = lo; k <= hi; k++) {
+            rows += c.bin_count[brm::kBinRank0 + k];
+            if (c.bin_count[brm::kBinRank0 + k])
+                top = k;
+        }
+        if (top < 0 || rows > (long long)num_sms * kRows[top])
+            return top < 0;
+        P.rank_span[top] = top - lo;
+        for (int k = lo; k < top; k++)
+            P.rank_taken |= 1u << k;
+        return true;
+    };
+    if (!take(0, 5)) {
+        take(0, 2);
+        take(3, 5);
+    }
+}
+
 // Analysis + symbolic (+ crpt scan for Precise).  Leaves ctx->h_cnt filled.
 // Timed: events kEvStart, kEvAna, kEvPre, kEvSized, kEvSym, kEvScan.
-// fused_dtype >= 0 (one-call Precise only): the mid rows are computed here,
-// values included, into ctx->midbuf, and the numeric phase only moves them.
+// fused_dtype >= 0 (one-call Precise only): the warp and mid rows are computed
+// here, values included, into ctx->midbuf, and the numeric phase only moves
+// them.  may_defer: a small call without heavy rows does not wait for nnz(C)
+// and the plan's errors (ctx->deferred; the caller reads the counters at the
+// end, and the numeric phase does nothing when the plan has failed).
 int plan_phase(brm_context ctx, const brm_csr *A, const brm_csr *B, int *crpt, bool upper,
-               bool timed, int fused_dtype = -1)
+               bool timed, int fused_dtype = -1, bool may_defer = false)
 {
     const bool fused = fused_dtype >= 0 && !upper;
     ctx->mid_ready = false;
+    ctx->deferred = false;
     BRM_TRY(ensure_workspace(ctx, A->M));
     BRM_TRY(ensure_ameta(ctx, A->nnz));
     if (ctx->validate)
@@ -380,45 +421,42 @@ int plan_phase(brm_context ctx, const brm_csr *A, const brm_csr *B, int *crpt, b
     ctx->plan.r_hi = A->M;
     ctx->plan.seg_range = nullptr;
     ctx->plan.live = brm::kLiveAll;
+    ctx->plan.upper = upper;
     brm::PlanDev P = ctx->plan;
     cudaStream_t s = ctx->stream;
     ev_record(ctx, timed, kEvStart);
     BRM_CK(cudaMemsetAsync(P.cnt, 0, sizeof(brm::Counters), s));
     brm::launch_analyze(a, b, P, s);
     ev_record(ctx, timed, kEvAna);
-    brm::launch_batches(P, A->M, ctx->scan_tmp, s);
-    ev_record(ctx, timed, kEvPre);
-    // the segment descriptors of heavy rows are sized by the analysis
+    // the analysis counts the rows of every class and sizes the segment
+    // descriptors and the scratch
     BRM_CK(cudaGetLastError());
     BRM_CK(cudaMemcpyAsync(ctx->h_cnt, P.cnt, sizeof(brm::Counters), cudaMemcpyDeviceToHost, s));
-    if (fused) {
-        BRM_CK(cudaMemcpyAsync(ctx->h_mid, P.mid_pre + A->M, sizeof(long long),
-                               cudaMemcpyDeviceToHost, s));
-        BRM_CK(cudaMemcpyAsync(ctx->h_mid + 1, P.mw_pre + A->M, sizeof(long long),
-                               cudaMemcpyDeviceToHost, s));
-    }
+    ev_record(ctx, timed, kEvPre);
     BRM_CK(cudaStreamSynchronize(s));
+    const brm::Counters &hc = *ctx->h_cnt;
     {
         // row classes with rows (the analysis has binned every row): the
         // kernels of the others are not launched
-        const brm::Counters &hc = *ctx->h_cnt;
         unsigned live = 0;
         for (int b = 0; b < brm::kNumBins; b++)
             if (hc.bin_count[b] > 0)
                 live |= brm::live_bit(b);
-        // batched mid rows are counted in batches, the longest heavy rows apart
-        if (hc.n_batch > 0)
-            live |= brm::live_bit(brm::kBinBatch);
+        // the longest heavy rows are counted apart
         if (hc.n_huge > 0)
             live |= brm::live_bit(brm::kBinHeavy);
         if (live & brm::live_bit(brm::kBinHeavy))
             live |= brm::kLiveSegs;  // until the planning says no row was segmented
-        P.live = ctx->plan.live = live;
+        ctx->plan.live = live;
+        plan_rank_spans(ctx->plan, hc, ctx->num_sms);
+        P = ctx->plan;
     }
+    if (brm::plan_live(P, brm::live_bit(brm::kBinBatch)))
+        brm::launch_batches(P, A->M, ctx->scan_tmp, s);
     if (fused) {
-        // batched mid rows at mid_pre[row], warp mid rows after them
-        const long long tot = ctx->h_mid[0] + ctx->h_mid[1];
-        const size_t n = (size_t)(tot > 0 ? tot : 1);
+        // warp, tile, merge and rank rows at mw_pre[row], batched mid rows
+        // after them
+        const size_t n = (size_t)std::max(1ull, hc.mw_total + hc.mid_total);
         const size_t b_col = a256(4 * n);
         BRM_TRY(grow(ctx, ctx->midbuf, b_col + vsize((brm_dtype)fused_dtype) * n));
         ctx->mid_col = (int *)ctx->midbuf.p;
@@ -426,7 +464,7 @@ int plan_phase(brm_context ctx, const brm_csr *A, const brm_csr *B, int *crpt, b
         P.mid_cap = ctx->plan.mid_cap = (long long)n;
     }
     {
-        const size_t cap = (size_t)ctx->h_cnt->seg_cap + 1;
+        const size_t cap = (size_t)hc.seg_cap + 1;
         const size_t b_run = a256(cap * sizeof(brm::SegRun));
         BRM_TRY(grow(ctx, ctx->segbuf, b_run + cap * (sizeof(brm::SegDesc) + sizeof(int))));
         P.run = (brm::SegRun *)ctx->segbuf.p;
@@ -438,48 +476,47 @@ int plan_phase(brm_context ctx, const brm_csr *A, const brm_csr *B, int *crpt, b
     }
     ev_record(ctx, timed, kEvSized);
     if (fused) {
-        // the batched and four-warp group mid rows (values into the scratch)
-        // on the second stream, beside the warp-row counts, the heavy-row
-        // planning and then the warp and tile mid rows; the planning is
-        // enqueued first, so its longest rows start before the mid rows
-        // take the SMs
+        // the batched and group mid rows (values into the scratch) on the
+        // second stream, beside the heavy-row planning and then the warp and
+        // tile mid rows; the planning is enqueued first, so its longest rows
+        // start before the mid rows take the SMs
         const brm::Fork &fk = ctx->fork;
-        BRM_CK(cudaEventRecord(fk.fork, s));
+        const auto scratch = fused_dtype == BRM_F64 ? brm::launch_mid_scratch_f64
+                                                    : brm::launch_mid_scratch_f32;
+        const bool fork = brm::plan_live(P, brm::kLiveGroups);
+        if (fork)
+            BRM_CK(cudaEventRecord(fk.fork, s));
         brm::launch_symbolic(a, b, P, ctx->num_sms, upper, fused, s);
-        BRM_CK(cudaStreamWaitEvent(fk.aux, fk.fork, 0));
-        if (fused_dtype == BRM_F64)
-            brm::launch_mid_scratch_f64(a, b, P, ctx->mid_col, ctx->mid_val, ctx->num_sms, fk.aux,
-                                        brm::kMidGroups);
-        else
-            brm::launch_mid_scratch_f32(a, b, P, ctx->mid_col, ctx->mid_val, ctx->num_sms, fk.aux,
-                                        brm::kMidGroups);
-        BRM_CK(cudaEventRecord(fk.join, fk.aux));
+        if (fork) {
+            BRM_CK(cudaStreamWaitEvent(fk.aux, fk.fork, 0));
+            scratch(a, b, P, ctx->mid_col, ctx->mid_val, ctx->num_sms, fk.aux, brm::kMidGroups);
+            BRM_CK(cudaEventRecord(fk.join, fk.aux));
+        }
+        scratch(a, b, P, ctx->mid_col, ctx->mid_val, ctx->num_sms, s, brm::kMidWarps);
+        if (fork)
+            BRM_CK(cudaStreamWaitEvent(s, fk.join, 0));
     } else {
         brm::launch_symbolic(a, b, P, ctx->num_sms, upper, fused, s);
     }
-    if (fused) {
-        if (fused_dtype == BRM_F64)
-            brm::launch_mid_scratch_f64(a, b, P, ctx->mid_col, ctx->mid_val, ctx->num_sms, s,
-                                        brm::kMidWarps);
-        else
-            brm::launch_mid_scratch_f32(a, b, P, ctx->mid_col, ctx->mid_val, ctx->num_sms, s,
-                                        brm::kMidWarps);
-        BRM_CK(cudaStreamWaitEvent(s, ctx->fork.join, 0));
-    }
     ev_record(ctx, timed, kEvSym);
-    if (upper)
-        brm::launch_scan_i64(P.flop, P.scan_flop, A->M, ctx->scan_tmp, s);
-    else
+    if (!upper)
         brm::launch_scan_i32(P.nnz, crpt, A->M, P.cnt, ctx->scan_tmp, s);
     ev_record(ctx, timed, kEvScan);
     BRM_CK(cudaGetLastError());
-    BRM_CK(cudaMemcpyAsync(ctx->h_cnt, P.cnt, sizeof(brm::Counters), cudaMemcpyDeviceToHost, s));
-    BRM_CK(cudaStreamSynchronize(s));
-    ctx->last_err = ctx->h_cnt->err;
-    BRM_TRY(device_err_status(ctx->h_cnt->err));
-    if (ctx->h_cnt->n_seg == 0)
+    ctx->deferred = fused && may_defer && hc.err == 0 && hc.total_flop <= kDeferProducts &&
+                    !brm::plan_live(P, brm::live_bit(brm::kBinHeavy) |
+                                           brm::live_bit(brm::kBinMid));
+    if (!ctx->deferred) {
+        BRM_CK(cudaMemcpyAsync(ctx->h_cnt, P.cnt, sizeof(brm::Counters), cudaMemcpyDeviceToHost,
+                               s));
+        BRM_CK(cudaStreamSynchronize(s));
+        ctx->last_err = hc.err;
+        BRM_TRY(device_err_status(hc.err));
+    }
+    if (hc.n_seg == 0)
         ctx->plan.live &= ~brm::kLiveSegs;
     ctx->planned = true;
+    ctx->fresh = true;
     ctx->a_rpt = A->rpt;
     ctx->a_col = A->col;
     ctx->b_rpt = B->rpt;
@@ -487,7 +524,7 @@ int plan_phase(brm_context ctx, const brm_csr *A, const brm_csr *B, int *crpt, b
     ctx->pM = A->M;
     ctx->pK = A->N;
     ctx->pN = B->N;
-    ctx->spill_bytes = ctx->h_cnt->spill_bytes;
+    ctx->spill_bytes = hc.spill_bytes;
     ctx->mid_ready = fused;
     return BRM_SUCCESS;
 }
@@ -552,9 +589,14 @@ int numeric_launch(brm_context ctx, brm_dtype dtype, bool upper, const brm_csr *
     P.seg_range = part.seg_range;
     if (part.seg_list)
         P.seg_list = (int *)part.seg_list;
-    // work_num and (unless the errors of earlier parts must survive) err
-    BRM_CK(cudaMemsetAsync(&P.cnt->work_num, 0, (clear_err ? 2 : 1) * sizeof(int), s));
-    BRM_CK(cudaMemsetAsync(&P.cnt->work_bnum, 0, 2 * sizeof(int), s));  // work_bnum, work_seg
+    // the phase's counters and (unless the errors of earlier parts must
+    // survive) err, unless the plan has just cleared them (the batched mid rows
+    // of a one-call plan use work_bnum)
+    if (!ctx->fresh || sizes || brm::plan_live(P, brm::live_bit(brm::kBinBatch))) {
+        char *from = (char *)(clear_err ? &P.cnt->err : &P.cnt->work_num);
+        BRM_CK(cudaMemsetAsync(from, 0, (char *)(&P.cnt->long_elems + 1) - from, s));
+    }
+    ctx->fresh = false;
     BRM_TRY(grow(ctx, ctx->splitbuf, ((size_t)sz.table_cap + 1) * sizeof(int)));
     P.split = (int *)ctx->splitbuf.p;
     ctx->plan.split = P.split;
@@ -572,10 +614,12 @@ int numeric_launch(brm_context ctx, brm_dtype dtype, bool upper, const brm_csr *
         P.long_val = q + b_col + b_leaf;
         P.long_cap_cols = cols;
         P.long_cap_elems = elems;
-        static_assert(offsetof(brm::Counters, long_elems) ==
-                          offsetof(brm::Counters, long_cols) + sizeof(unsigned long long),
-                      "the two long-column counters are cleared together");
-        BRM_CK(cudaMemsetAsync(&P.cnt->long_cols, 0, 2 * sizeof(unsigned long long), s));
+        static_assert(offsetof(brm::Counters, work_num) ==
+                              offsetof(brm::Counters, err) + sizeof(int) &&
+                          offsetof(brm::Counters, long_elems) + sizeof(unsigned long long) -
+                                  offsetof(brm::Counters, err) ==
+                              4 * sizeof(int) + 2 * sizeof(unsigned long long),
+                      "err and the counters of the numeric phase are cleared together");
     }
     brm::CsrDev a = to_dev(A), b = to_dev(B);
     const int *mcol = mid ? ctx->mid_col : nullptr;
@@ -602,6 +646,17 @@ int read_err(brm_context ctx)
                                cudaMemcpyDeviceToHost, ctx->stream));
         BRM_CK(cudaStreamSynchronize(ctx->stream));
     }
+    ctx->last_err = ctx->h_cnt->err;
+    return device_err_status(ctx->h_cnt->err);
+}
+
+// All counters and the error status after the numeric phase of a plan that did
+// not wait for them.
+int read_counters(brm_context ctx)
+{
+    BRM_CK(cudaMemcpyAsync(ctx->h_cnt, ctx->plan.cnt, sizeof(brm::Counters),
+                           cudaMemcpyDeviceToHost, ctx->stream));
+    BRM_CK(cudaStreamSynchronize(ctx->stream));
     ctx->last_err = ctx->h_cnt->err;
     return device_err_status(ctx->h_cnt->err);
 }
@@ -909,6 +964,7 @@ int brm::numeric_async(brm_context ctx, brm_dtype dtype, const brm_csr *A, const
     BRM_TRY(check_pair(A, B));
     if (!plan_matches(ctx, A, B))
         return BRM_ERR_NOT_PLANNED;
+    ctx->fresh = false;  // a captured launch clears its counters at every replay
     return numeric_launch(ctx, dtype, false, A, B, crpt, ccol, cval);
 }
 
@@ -960,7 +1016,8 @@ int brm::reserve_pipe(brm_context ctx, brm_dtype dtype, const brm::PipeCaps &c)
         ctx->plan.seg_list = (int *)(ctx->plan.seg + cap);
     }
     {
-        const size_t n = (size_t)std::max(c.products, 1LL);
+        // a batched mid row weighs at most its products and its entries
+        const size_t n = (size_t)std::max(c.products + c.nnz_a, 1LL);
         const size_t b_col = a256(4 * n);
         BRM_TRY(grow(ctx, ctx->midbuf, b_col + vsize(dtype) * n));
         ctx->mid_col = (int *)ctx->midbuf.p;
@@ -989,6 +1046,10 @@ int brm::precise_pipe(brm_context ctx, brm_dtype dtype, const brm_csr *A, const 
     ctx->plan.r_hi = A->M;
     ctx->plan.seg_range = nullptr;
     ctx->plan.live = brm::kLiveAll;  // the counts are on the device only
+    ctx->plan.upper = 0;
+    std::memset(ctx->plan.rank_span, 0, sizeof(ctx->plan.rank_span));
+    ctx->plan.rank_taken = 0;
+    ctx->fresh = false;
     ctx->planned = false;
     const brm::PlanDev P = ctx->plan;
     cudaStream_t s = ctx->stream;
@@ -1074,8 +1135,6 @@ int brm_create(brm_context *out)
         e = cudaMallocHost(&ctx->h_cnt, sizeof(brm::Counters));
     if (e == cudaSuccess)
         e = cudaMallocHost(&ctx->h_bad, sizeof(int));
-    if (e == cudaSuccess)
-        e = cudaMallocHost(&ctx->h_mid, 2 * sizeof(long long));
     for (int i = 0; i < kNumEvents && e == cudaSuccess; i++)
         e = cudaEventCreate(&ctx->ev[i]);
     for (int i = 0; i < brm::kMaxParts && e == cudaSuccess; i++)
@@ -1138,8 +1197,6 @@ int brm_destroy(brm_context ctx)
         cudaFreeHost(ctx->h_cnt);
     if (ctx->h_bad)
         cudaFreeHost(ctx->h_bad);
-    if (ctx->h_mid)
-        cudaFreeHost(ctx->h_mid);
     for (int i = 0; i < kNumEvents; i++)
         if (ctx->ev[i])
             cudaEventDestroy(ctx->ev[i]);
@@ -1322,12 +1379,14 @@ int brm_precise_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const
     BRM_CK(cudaMallocAsync((void **)&crpt, 4 * ((size_t)A->M + 1), ctx->stream));
     double t1 = now_sec();
     ctx->planned = false;
-    int st = plan_phase(ctx, A, B, crpt, false, timed, dtype);
+    int st = plan_phase(ctx, A, B, crpt, false, timed, dtype, true);
     if (st != BRM_SUCCESS) {
         cudaFreeAsync(crpt, ctx->stream);
         return st;
     }
-    int cnnz = (int)ctx->h_cnt->cnnz;
+    // a small call has not waited for nnz(C): C has room for every product
+    const bool deferred = ctx->deferred;
+    int cnnz = deferred ? (int)ctx->h_cnt->total_flop : (int)ctx->h_cnt->cnnz;
     int *ccol = nullptr;
     void *cval = nullptr;
     double t2 = now_sec();
@@ -1335,6 +1394,7 @@ int brm_precise_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const
     if (e == cudaSuccess)
         e = cudaMallocAsync(&cval, vsize(dtype) * (size_t)(cnnz > 0 ? cnnz : 1), ctx->stream);
     if (e != cudaSuccess) {
+        ctx->planned = ctx->planned && !deferred;
         cudaFreeAsync(crpt, ctx->stream);
         if (ccol)
             cudaFreeAsync(ccol, ctx->stream);
@@ -1343,16 +1403,19 @@ int brm_precise_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const
     }
     double t3 = now_sec();
     ev_record(ctx, timed, kEvNum0);
+    ctx->h_cnt->cnnz = cnnz;
     st = numeric_launch(ctx, dtype, false, A, B, crpt, ccol, cval, true);
     ev_record(ctx, timed, kEvNum1);
     if (st == BRM_SUCCESS)
-        st = read_err(ctx);
+        st = deferred ? read_counters(ctx) : read_err(ctx);
     if (st != BRM_SUCCESS) {
+        ctx->planned = ctx->planned && !deferred;
         cudaFreeAsync(crpt, ctx->stream);
         cudaFreeAsync(ccol, ctx->stream);
         cudaFreeAsync(cval, ctx->stream);
         return st;
     }
+    cnnz = (int)ctx->h_cnt->cnnz;
     double t4 = now_sec();
     *crpt_ = crpt;
     *ccol_ = ccol;

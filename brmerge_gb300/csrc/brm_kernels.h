@@ -67,8 +67,8 @@ long long launches_so_far();
 // (replaces compute_flop and the static load balance, spgemm.h:31-56, :496-503).
 void launch_analyze(const CsrDev &A, const CsrDev &B, const PlanDev &P, cudaStream_t s);
 
-// Mid-row batches: scan of the mid products in row order and the first row
-// of every batch (Counters::n_batch batches).
+// Mid-row batches: scan of their weights in row order and the first row of
+// every batch (Counters::n_batch batches); needed where the class has rows.
 void launch_batches(const PlanDev &P, int M, void *tmp, cudaStream_t s);
 
 // Exclusive scans with out[n] = total.  The int32 form ORs kErrOverflow into
@@ -125,10 +125,10 @@ void launch_numeric_f32(bool upper, const CsrDev &A, const CsrDev &B, const Plan
                         unsigned long long spill_bytes, const int *mid_col, const void *mid_val,
                         int num_sms, cudaStream_t s, const Fork &fk);
 
-// One-call Precise: the mid rows' values and lengths (P.nnz) computed with
-// the plan, into a scratch of P.mid_pre[M] entries (row r at P.mid_pre[r]).
-// which: 1 = the batched mid rows and the four-warp group rows, 2 = the warp
-// and tile rows, 3 = all (the parts can run on different streams).
+// One-call Precise: the warp and mid rows' values and lengths (P.nnz) computed
+// with the plan, into a scratch (k_mid_compact says where).  which: 1 = the
+// batched mid rows and the group rows, 2 = the warp and tile rows, 3 = all
+// (the parts can run on different streams).
 void launch_mid_scratch_f64(const CsrDev &A, const CsrDev &B, const PlanDev &P, int *mid_col,
                             void *mid_val, int num_sms, cudaStream_t s, int which);
 void launch_mid_scratch_f32(const CsrDev &A, const CsrDev &B, const PlanDev &P, int *mid_col,

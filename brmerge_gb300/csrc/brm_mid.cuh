@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(kMidThreads) k_mid_numeric(CsrDev A, CsrDev B,
                 enter(p);
                 const int e = sb[p];
                 const int row = t.s_row[s_cur];
-                const long long base = SCRATCH ? P.mid_pre[row]
+                const long long base = SCRATCH ? (long long)P.cnt->mw_total + P.mid_pre[row]
                                        : (UPPER ? P.scan_flop[row] : (long long)crpt[row]);
                 const long long o = base + (h - s_hb[s_cur]);
                 int q = p + 1;
@@ -614,49 +614,73 @@ __global__ void __launch_bounds__(256) k_batch_starts(PlanDev P, int M)
         P.cnt->n_batch = (int)((hi + W - 1) / W);
 }
 
-// Moves the mid rows written by k_mid_numeric<..., SCRATCH> (row at
-// P.mid_pre[row]) and k_mid_warp<..., kMwScratch> (row at P.mid_pre[M] +
-// P.mw_pre[row]), P.nnz[row] entries each, from the scratch to C at
-// crpt[row].  One warp per row; rows that are not mid rows are skipped.
-template <typename T>
-__global__ void __launch_bounds__(256) k_mid_compact(PlanDev P, int M, const int *__restrict__ scol,
+// Moves the rows written to the one-call scratch -- k_mid_numeric<..., SCRATCH>
+// (row at Counters::mw_total + P.mid_pre[row]), the warp, merge and rank
+// kernels (row at P.mw_pre[row]), P.nnz[row] entries each -- to C at crpt[row].
+// One warp per row.  COPY: the copy rows (one nonempty list, C row = a * B
+// row) in the same launch.
+template <typename T, bool COPY>
+__global__ void __launch_bounds__(256) k_mid_compact(CsrDev A, CsrDev B, PlanDev P,
+                                                     const int *__restrict__ scol,
                                                      const T *__restrict__ sval, const int *crpt,
                                                      int *__restrict__ ccol, T *__restrict__ cval)
 {
-    if (P.cnt->abort)  // a capacity check of a captured pipeline failed
+    // a capacity check of a captured pipeline failed, or the plan did (row
+    // lengths may then be missing)
+    if (P.cnt->abort || P.cnt->err)
         return;
     const int lane = threadIdx.x & 31;
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int M = A.M;
     const int r1 = min(M, P.r_hi);
-    // warp and group rows from their row lists, then (only when there are
-    // batches) the batched mid rows by a sweep over the rows
+    // rows from their class lists, then (only when there are batches) the
+    // batched mid rows by a sweep over the rows
+    constexpr int B0 = COPY ? kBinCopy : kBinWarp;
+    auto listed = [](int b) { return b <= kBinWarp || b >= kBinMidWarp; };
     int nlist = 0;
 #pragma unroll
-    for (int b = kBinMidWarp; b < kNumBins; b++)
-        nlist += P.cnt->bin_count[b];
+    for (int b = B0; b < kNumBins; b++)
+        nlist += listed(b) ? P.cnt->bin_count[b] : 0;
     const int nsweep = P.cnt->n_batch > 0 ? r1 - P.r_lo : 0;
     for (int it = gw; it < nlist + nsweep; it += nwarps) {
         int row;
+        const int *sc = scol;
+        const T *sv = sval;
         long long src;
+        T a = T(0);
+        bool copy = false;
         if (it < nlist) {
-            int b = kBinMidWarp, i = it;
-            while (i >= P.cnt->bin_count[b])
-                i -= P.cnt->bin_count[b++];
+            int b = B0, i = it;
+            for (;; b++) {
+                const int c = listed(b) ? P.cnt->bin_count[b] : 0;
+                if (i < c)
+                    break;
+                i -= c;
+            }
             row = P.rows[(size_t)b * M + i];
             if (row < P.r_lo || row >= r1)
                 continue;
-            src = P.mid_pre[M] + P.mw_pre[row];
+            copy = COPY && b == kBinCopy;
+            if (copy) {
+                const int j = A.rpt[row] + P.copy_leaf[row];
+                a = ((const T *)A.val)[j];
+                sc = B.col;
+                sv = (const T *)B.val;
+                src = P.abs[j];
+            } else {
+                src = P.mw_pre[row];
+            }
         } else {
             row = P.r_lo + (it - nlist);
             if (P.mid_flop[row] == 0)
                 continue;
-            src = P.mid_pre[row];
+            src = (long long)P.cnt->mw_total + P.mid_pre[row];
         }
         const long long dst = crpt[row];
         int n = P.nnz[row];
-        if (n > 0 && !(BRM_IN(P.cnt, dst + n - 1, P.c_cap) && BRM_IN(P.cnt, src + n - 1, P.mid_cap)))
-            n = 0;  // checked build: a row outside C or the scratch is skipped
+        if (n > 0 && !(BRM_IN(P.cnt, dst + n - 1, P.c_cap) && BRM_IN(P.cnt, src + n - 1, copy ? (long long)B.nnz : P.mid_cap)))
+            n = 0;  // checked build: a row outside C, B or the scratch is skipped
         // four elements per lane in flight before the stores
         int i = lane;
         for (; i + 96 < n; i += 128) {
@@ -664,18 +688,18 @@ __global__ void __launch_bounds__(256) k_mid_compact(PlanDev P, int M, const int
             T v[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                c[u] = scol[src + i + 32 * u];
-                v[u] = sval[src + i + 32 * u];
+                c[u] = sc[src + i + 32 * u];
+                v[u] = sv[src + i + 32 * u];
             }
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 ccol[dst + i + 32 * u] = c[u];
-                cval[dst + i + 32 * u] = v[u];
+                cval[dst + i + 32 * u] = copy ? vmul(a, v[u]) : v[u];
             }
         }
         for (; i < n; i += 32) {
-            ccol[dst + i] = scol[src + i];
-            cval[dst + i] = sval[src + i];
+            ccol[dst + i] = sc[src + i];
+            cval[dst + i] = copy ? vmul(a, sv[src + i]) : sv[src + i];
         }
     }
 }

@@ -260,8 +260,19 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
     int *gs = (int *)(ws + S::o_gs);          // scan scratch, then row, F, counts
     int *gm = gs + G + 1;
     const int M = A.M;
-    const int n = P.cnt->bin_count[S::BIN];
-    const int *rows = P.rows + (size_t)S::BIN * M;
+    // rows of this class, then of the smaller ones it takes along
+    const int b0 = S::BIN - P.rank_span[S::BIN - kBinRank0];
+    int n = 0;
+    for (int b = b0; b <= S::BIN; b++)
+        n += P.cnt->bin_count[b];
+    auto row_at = [&](int i) {
+        if (i >= n)
+            return -1;
+        int b = S::BIN;
+        for (; i >= P.cnt->bin_count[b]; b--)
+            i -= P.cnt->bin_count[b];
+        return P.rows[(size_t)b * M + i];
+    };
     const int *__restrict__ bcol = B.col;
     const T *__restrict__ bval = (const T *)B.val;
     const T *__restrict__ aval = (const T *)A.val;
@@ -273,7 +284,7 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
     int row = -1, nrow = -1, nit = 0;
     if (t == 0) {
         nit = atomicAdd(work, claim);
-        nrow = nit < n ? rows[nit] : -1;
+        nrow = row_at(nit);
     }
     for (;;) {
         if (G > 1) {
@@ -303,7 +314,7 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
             if (mine && t == 0)  // the analysis bins prevent this
                 atomicOr(&P.cnt->err, kErrWindowOverflow);
             if (t == 0)
-                nrow = nit < n ? rows[nit] : -1;
+                nrow = row_at(nit);
             grp_sync<G>(gid);
             continue;
         }
@@ -351,7 +362,7 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
             }
         }
         if (t == 0)
-            nrow = nit < n ? rows[nit] : -1;
+            nrow = row_at(nit);
         grp_sync<G>(gid);
         if (G > 1)
             F = gm[1];
@@ -451,7 +462,7 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
         } else if (MODE == kMwUpper) {
             base = P.scan_flop[row];
         } else {
-            base = P.mid_pre[M] + P.mw_pre[row];
+            base = P.mw_pre[row];
         }
         if ((MODE == kMwUpper || MODE == kMwScratch) && t == 0)
             P.nnz[row] = U;
@@ -682,6 +693,8 @@ template <typename T, int MODE, class S>
 inline void launch_mid_rank(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int *crpt,
                             int *ccol, T *cval, int num_sms, cudaStream_t s)
 {
+    if (!plan_live(P, live_bit(S::BIN)) || (P.rank_taken >> (S::BIN - kBinRank0) & 1u))
+        return;
     cudaFuncSetAttribute(k_mid_rank<T, MODE, S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)S::bytes);
     k_mid_rank<T, MODE, S><<<num_sms * S::CTAS, S::THREADS, S::bytes, s>>>(A, B, P, crpt, ccol,
@@ -703,24 +716,16 @@ inline void launch_mid_warp(const CsrDev &A, const CsrDev &B, const PlanDev &P, 
             launch_mid_group<T, MODE, 5>(A, B, P, crpt, ccol, cval, num_sms, s);
         if (plan_live(P, live_bit(kBinMidGroup)))
             launch_mid_group<T, MODE, 4>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(Rank5::BIN)))
-            launch_mid_rank<T, MODE, Rank5>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(Rank7::BIN)))
-            launch_mid_rank<T, MODE, Rank7>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(Rank4::BIN)))
-            launch_mid_rank<T, MODE, Rank4>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(Rank3::BIN)))
-            launch_mid_rank<T, MODE, Rank3>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank5>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank7>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank4>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank3>(A, B, P, crpt, ccol, cval, num_sms, s);
     }
     if (which & kMidWarps) {
-        if (plan_live(P, live_bit(Rank6::BIN)))
-            launch_mid_rank<T, MODE, Rank6>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(Rank2::BIN)))
-            launch_mid_rank<T, MODE, Rank2>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(Rank1::BIN)))
-            launch_mid_rank<T, MODE, Rank1>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(Rank0::BIN)))
-            launch_mid_rank<T, MODE, Rank0>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank6>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank2>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank1>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank0>(A, B, P, crpt, ccol, cval, num_sms, s);
         if (plan_live(P, live_bit(kBinMidWarp)))
             launch_mid_group<T, MODE, 1>(A, B, P, crpt, ccol, cval, num_sms, s);
         if (plan_live(P, live_bit(kBinMidTile2)))

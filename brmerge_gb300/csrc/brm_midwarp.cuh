@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(mw_threads<SID>(), 2) k_mid_warp(CsrDev A, Csr
         } else if (MODE == kMwUpper) {
             base = P.scan_flop[row];
         } else {
-            base = P.mid_pre[M] + P.mw_pre[row];
+            base = P.mw_pre[row];
         }
         if ((MODE == kMwUpper || MODE == kMwScratch) && t == 0)
             P.nnz[row] = len;
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(kMwThreads, 2) k_mid_tile(CsrDev A, CsrDev B, 
         } else if (MODE == kMwUpper) {
             base = P.scan_flop[row];
         } else {
-            base = P.mid_pre[M] + P.mw_pre[row];
+            base = P.mw_pre[row];
         }
         if ((MODE == kMwUpper || MODE == kMwScratch) && lt == 0)
             P.nnz[row] = len;

@@ -19,37 +19,49 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
 {
     // copy, warp and mid rows on the aux stream (when there is one), beside
     // the split table and the segments of the heavy rows on s0
+    // (one stream when no row is segmented)
+    const bool segs = plan_live(P, kLiveSegs);
+    const bool fork = fk.aux && segs;
     cudaStream_t s = s0;
-    if (fk.aux) {
+    if (fork) {
         cudaEventRecord(fk.fork, s0);
         cudaStreamWaitEvent(fk.aux, fk.fork, 0);
         s = fk.aux;
     }
-    // (kernels of row classes without rows are not launched)
-    if (plan_live(P, live_bit(kBinCopy))) {
-        k_copy_numeric<T, UPPER><<<num_sms * 8, 256, 0, s>>>(A, B, P, crpt, ccol, cval);
-        count_launch();
-    }
-    if (plan_live(P, live_bit(kBinWarp))) {
-        k_warp_numeric<T, UPPER><<<num_sms * 8, 256, 0, s>>>(A, B, P, crpt, ccol, cval);
-        count_launch();
-    }
-    // The mid rows computed with the plan (one-call Precise) are moved into
-    // C by a bandwidth-bound copy.  With heavy-row segments it waits for the
-    // segment kernel (which holds every SM's registers) and runs beside the
-    // latency-bound column reducers that follow it (R-MAT n=2^18 one-call
+    // The warp and mid rows computed with the plan (one-call Precise) are moved
+    // into C by a bandwidth-bound copy.  With heavy-row segments it waits for
+    // the segment kernel (which holds every SM's registers) and runs beside
+    // the latency-bound column reducers that follow it (R-MAT n=2^18 one-call
     // Precise 2.875 -> 2.838 ms; the two reducers on separate streams as
     // well: 2.917 ms).  A numeric phase run in row parts (the host drop-in
-    // copies each part back while the next computes) keeps it first.
+    // copies each part back while the next computes) keeps it first.  Without
+    // segments it does the copy rows too, in one launch.
+    // (kernels of row classes without rows are not launched)
     const bool compact = mid_col && plan_live(P, kLiveMidRows);
-    const bool compact_late = compact && fk.aux && plan_live(P, kLiveSegs) && !P.seg_range;
-    if (mid_col) {
-        if (compact && !compact_late) {
-            k_mid_compact<T><<<num_sms * 8, 256, 0, s>>>(P, A.M, mid_col, (const T *)mid_val,
-                                                              crpt, ccol, cval);
+    const bool compact_late = compact && fork && !P.seg_range;
+    const bool copies = plan_live(P, live_bit(kBinCopy));
+    if (compact && !segs && copies) {
+        k_mid_compact<T, true><<<num_sms * 8, 256, 0, s>>>(A, B, P, mid_col, (const T *)mid_val,
+                                                           crpt, ccol, cval);
+        count_launch();
+    } else {
+        if (copies) {
+            k_copy_numeric<T, UPPER><<<num_sms * 8, 256, 0, s>>>(A, B, P, crpt, ccol, cval);
             count_launch();
         }
-    } else {
+        if (compact && !compact_late) {
+            k_mid_compact<T, false><<<num_sms * 8, 256, 0, s>>>(A, B, P, mid_col,
+                                                                (const T *)mid_val, crpt, ccol,
+                                                                cval);
+            count_launch();
+        }
+    }
+    if (!mid_col) {
+        if (plan_live(P, live_bit(kBinWarp))) {
+            k_warp_numeric<T, UPPER ? kWarpUpper : kWarpPrecise>
+                <<<num_sms * 8, 256, 0, s>>>(A, B, P, crpt, ccol, cval);
+            count_launch();
+        }
         launch_mid_warp<T, UPPER ? kMwUpper : kMwPrecise>(A, B, P, crpt, ccol, cval, num_sms,
                                                           s);
         if (plan_live(P, live_bit(kBinBatch))) {
@@ -61,10 +73,10 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
             count_launch();
         }
     }
-    if (fk.aux && !compact_late)
+    if (fork && !compact_late)
         cudaEventRecord(fk.join, fk.aux);
     s = s0;
-    if (plan_live(P, kLiveSegs)) {
+    if (segs) {
         k_split<0><<<num_sms * 8, 256, 0, s>>>(A, B, P);
         count_launch();
         const size_t ssm = SegLayout<T>::bytes;
@@ -87,9 +99,8 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
             // aux stream's first wait has already taken its earlier state)
             cudaEventRecord(fk.fork, s0);
             cudaStreamWaitEvent(fk.aux, fk.fork, 0);
-            k_mid_compact<T><<<num_sms * 8, 256, 0, fk.aux>>>(P, A.M, mid_col,
-                                                                (const T *)mid_val, crpt, ccol,
-                                                                cval);
+            k_mid_compact<T, false><<<num_sms * 8, 256, 0, fk.aux>>>(
+                A, B, P, mid_col, (const T *)mid_val, crpt, ccol, cval);
             count_launch();
             cudaEventRecord(fk.join, fk.aux);
         }
@@ -110,7 +121,7 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
             A, B, P, crpt, ccol, cval, (unsigned char *)spill_scratch, spill_bytes);
         count_launch();
     }
-    if (fk.aux)
+    if (fork)
         cudaStreamWaitEvent(s0, fk.join, 0);
 }
 
@@ -142,6 +153,11 @@ void launch_mid_scratch_t(const CsrDev &A, const CsrDev &B, const PlanDev &P, in
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)msm);
         k_mid_numeric<T, false, true><<<num_sms * 2, kMidThreads, msm, s>>>(
             A, B, P, nullptr, mid_col, (T *)mid_val);
+        count_launch();
+    }
+    if ((which & kMidWarps) && plan_live(P, live_bit(kBinWarp))) {
+        k_warp_numeric<T, kWarpScratch><<<num_sms * 8, 256, 0, s>>>(A, B, P, nullptr, mid_col,
+                                                                    (T *)mid_val);
         count_launch();
     }
     launch_mid_warp<T, kMwScratch>(A, B, P, nullptr, mid_col, (T *)mid_val, num_sms, s, which);

@@ -156,27 +156,30 @@ struct Counters {
     int bin_count[kNumBins];
     int spill_count;
     int work_sym;      // dynamic row counter of the symbolic row kernel
-    int work_num;      // dynamic row counter of the numeric row kernel
-    int err;           // OR of DevErr bits
     int max_k;         // longest A row
-    unsigned long long total_flop;
-    unsigned long long spill_bytes;  // scratch reserved for spill rows
-    long long cnnz;    // total nnz of C (int64 before the int32 check)
-    int n_batch;       // number of mid-row batches
-    int work_bsym;     // dynamic batch counter, symbolic
+    // err, then the counters of the numeric phase: cleared by one memset, with
+    // or without err
+    int err;           // OR of DevErr bits
+    int work_num;      // dynamic row counter of the numeric row kernel
     int work_bnum;     // dynamic batch counter, numeric
     int work_seg;      // dynamic segment counter, numeric
-    unsigned long long seg_cap;    // descriptor slots reserved by the analysis
-    unsigned long long table_cap;  // split-table entries reserved by the planning
-    int n_seg;         // segments written by the planning
-    int work_plan;     // dynamic row counter of the heavy-row planning
-    int n_huge;        // heavy rows above kHugeFlop products (listed from the end)
-    int n_longk;       // rows the narrow analysis left to the warp-wide pass
     // long columns of the segment kernel handed to the column reducers:
     // columns and elements reserved so far (two counters, so neither can
     // overflow into the other however many columns a call has)
     unsigned long long long_cols;
     unsigned long long long_elems;
+    unsigned long long total_flop;
+    unsigned long long mw_total;   // products of the warp, tile, merge and rank rows
+    unsigned long long mid_total;  // weights of the batched mid rows
+    unsigned long long spill_bytes;  // scratch reserved for spill rows
+    long long cnnz;    // total nnz of C (int64 before the int32 check)
+    int n_batch;       // number of mid-row batches
+    int work_bsym;     // dynamic batch counter, symbolic
+    unsigned long long seg_cap;    // descriptor slots reserved by the analysis
+    unsigned long long table_cap;  // split-table entries reserved by the planning
+    int n_seg;         // segments written by the planning
+    int work_plan;     // dynamic row counter of the heavy-row planning
+    int n_huge;        // heavy rows above kHugeFlop products (listed from the end)
     // set by the capacity checks of a captured batch pipeline when the batch
     // does not fit its buffers; every kernel that writes at data-dependent
     // offsets then returns at once (the call reports BRM_ERR_CAPACITY)
@@ -265,14 +268,14 @@ struct PlanDev {
     unsigned char *spill;  // [M] 1 if the row takes the spill path
     int *spill_rows;  // [M] spill row list
     unsigned long long *spill_off;  // [M] scratch byte offset per spill list entry
-    long long *scan_flop;  // [M+1] exclusive scan of flop (Upper)
+    long long *scan_flop;  // [M] offset of each row in C_bar (Upper)
     int *abs;              // [nnz(A)] start of B row acol[j] (list start of A entry j)
     int *alen;             // [nnz(A)] length of B row acol[j] (0 if acol[j] is out of range)
     int *mid_flop;         // [M] products of batched mid rows, 0 for other rows
     long long *mid_pre;    // [M+1] exclusive scan of mid_flop
-    int *mw_flop;          // [M] products of warp mid rows, 0 for other rows
-    long long *mw_pre;     // [M+1] exclusive scan of mw_flop (one-call scratch after mid_pre[M])
-    int *longk_rows;       // [M] rows with many A entries, analysed by whole warps
+    long long *mw_pre;     // [M] offset of each warp, tile, merge or rank row in the one-call
+                           // scratch (the batched mid rows lie behind them, at
+                           // Counters::mw_total + mid_pre)
     int *batch_start;      // [M+1] first row of each mid batch
     unsigned long long *seg_base;  // [M] first descriptor slot of each heavy row
     int *seg_n;            // [M] segments of each heavy row (0: not segmented)
@@ -295,6 +298,7 @@ struct PlanDev {
     // policy knobs (see kMinSegCut): heavy-row cut target, mid-row weight limit
     int seg_cut;
     int mid_limit;
+    int upper;  // the analysis writes scan_flop
     // entries of the arrays the numeric kernels write (C, or C_bar for
     // Upper) and of the one-call mid-row scratch; the bounds of the checked
     // build
@@ -302,8 +306,12 @@ struct PlanDev {
     long long mid_cap;
     Counters *cnt;
     // host side only: the launches the plan needs (kLive* bits); all ones
-    // when the host does not know the class counts (a captured pipeline)
+    // when the host does not know the class counts (a captured pipeline);
+    // rank_span[c]: rank classes below c whose few rows c's launch takes along,
+    // rank_taken their bits
     unsigned live;
+    int rank_span[kRankClasses];
+    unsigned rank_taken;
 };
 
 // Launch mask of a plan (PlanDev::live): bit b set when row class b (RowBin)
@@ -313,10 +321,15 @@ struct PlanDev {
 constexpr unsigned kLiveSegs = 1u << 30;
 constexpr unsigned kLiveAll = 0xffffffffu;
 constexpr unsigned live_bit(int bin) { return 1u << bin; }
-constexpr unsigned kLiveMidRows = live_bit(kBinBatch) | live_bit(kBinMidWarp) |
+// rows of the one-call scratch
+constexpr unsigned kLiveMidRows = live_bit(kBinWarp) | live_bit(kBinBatch) | live_bit(kBinMidWarp) |
                                   live_bit(kBinMidGroup) | live_bit(kBinMidTile) |
                                   live_bit(kBinMidTile2) | live_bit(kBinMidGroup2) |
                                   (live_bit(kNumBins) - live_bit(kBinRank0));
+constexpr unsigned kLiveGroups = live_bit(kBinBatch) | live_bit(kBinMidGroup) |
+                                 live_bit(kBinMidGroup2) | live_bit(kBinRank0 + 3) |
+                                 live_bit(kBinRank0 + 4) | live_bit(kBinRank0 + 5) |
+                                 live_bit(kBinRank0 + 7);  // kMidGroups
 inline bool plan_live(const PlanDev &P, unsigned bits) { return (P.live & bits) != 0; }
 
 // Capacities of a captured batch pipeline: every buffer sized by a count the

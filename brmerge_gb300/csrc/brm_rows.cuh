@@ -715,7 +715,10 @@ __global__ void __launch_bounds__(256) k_warp_symbolic(CsrDev A, CsrDev B, PlanD
     }
 }
 
-template <typename T, bool UPPER>
+// MODE: at crpt (kWarpPrecise), at the row's offset in C_bar (kWarpUpper) or
+// in the one-call scratch (kWarpScratch); the last two write the row's length.
+enum WarpRowMode : int { kWarpPrecise = 0, kWarpUpper = 1, kWarpScratch = 2 };
+template <typename T, int MODE>
 __global__ void __launch_bounds__(256) k_warp_numeric(CsrDev A, CsrDev B, PlanDev P,
                                                       const int *crpt, int *ccol, T *cval)
 {
@@ -779,16 +782,18 @@ __global__ void __launch_bounds__(256) k_warp_numeric(CsrDev A, CsrDev B, PlanDe
             node >>= 1;
         }
         const unsigned outm = __ballot_sync(kFull, active);
-        const long long base = UPPER ? P.scan_flop[row] : (long long)crpt[row];
+        const long long base = MODE == kWarpUpper     ? P.scan_flop[row]
+                               : MODE == kWarpScratch ? P.mw_pre[row]
+                                                      : (long long)crpt[row];
         if (active) {
             const long long o = base + __popc(outm & lanemask_lt());
-            if (BRM_IN(P.cnt, o, P.c_cap)) {
+            if (BRM_IN(P.cnt, o, MODE == kWarpScratch ? P.mid_cap : P.c_cap)) {
                 ccol[o] = c;
                 cval[o] = v;
             }
         }
         if (lane == 0) {
-            if (UPPER)
+            if (MODE != kWarpPrecise)
                 P.nnz[row] = __popc(outm);
             else if (__popc(outm) != crpt[row + 1] - crpt[row])
                 atomicOr(&P.cnt->err, kErrNnzMismatch);

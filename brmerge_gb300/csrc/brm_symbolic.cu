@@ -12,7 +12,6 @@ void launch_batches(const PlanDev &P, int M, void *tmp, cudaStream_t s)
     if (M <= 0)
         return;
     launch_scan_i64(P.mid_flop, P.mid_pre, M, tmp, s);
-    launch_scan_i64(P.mw_flop, P.mw_pre, M, tmp, s);
     k_batch_starts<0><<<(M + 1 + 255) / 256, 256, 0, s>>>(P, M);
     count_launch();
 }
@@ -23,7 +22,7 @@ void launch_symbolic(const CsrDev &A, const CsrDev &B, const PlanDev &P, int num
     if (A.M <= 0)
         return;
     if (!only_heavy) {
-        if (plan_live(P, live_bit(kBinWarp))) {
+        if (!skip_mid && plan_live(P, live_bit(kBinWarp))) {
             k_warp_symbolic<0><<<num_sms * 8, 256, 0, s>>>(A, B, P);
             count_launch();
         }

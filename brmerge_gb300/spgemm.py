@@ -312,7 +312,8 @@ class Context:
         tc = tcls._c()
         fn = self._L.brm_upper_device if upper else self._L.brm_precise_device
         _native.check(fn(self._h, code, C.byref(a), C.byref(b), C.byref(pr), C.byref(pc),
-                         C.byref(pv), C.byref(cnnz), C.byref(tc)),
+                         C.byref(pv), C.byref(cnnz),
+                         None if timing is None else C.byref(tc)),
                       "brm_upper_device" if upper else "brm_precise_device")
         n = cnnz.value
         dev = A.rpt.device

@@ -55,8 +55,9 @@ typedef enum brm_dtype { BRM_F64 = 0, BRM_F32 = 1 } brm_dtype;
 /* Phase times in seconds; the fields mirror Precise_Timing
  * (BRMerge-SpGEMM/inc/Timings.h:26-46).  GPU phases are timed with CUDA
  * events on the call's stream: compute_flop = row analysis and binning,
- * prefix_sum_flop = prefix sums of the mid-row products, load_balance = host
- * read of the bin counts and sizing of the segment buffers, symbolic = exact
+ * prefix_sum_flop = copy of the product totals and class counts to the host
+ * (the analysis gives the rows their offsets), load_balance = the wait for it
+ * and sizing of the segment buffers, symbolic = exact
  * row nnz (heavy rows cut into balanced segments), prefix_sum_nnz = crpt
  * scan, compute = numeric phase.  Device forms: pre_allocate and allocate_C
  * are host wall times of the output allocations.  Host drop-ins:
@@ -77,7 +78,8 @@ typedef struct brm_precise_timing {
 } brm_precise_timing;
 
 /* Mirrors Upper_Timing (BRMerge-SpGEMM/inc/Timings.h:4-24): compute_flop =
- * row analysis, prefix_sum_flop = the row-product scans, load_balance =
+ * row analysis (offsets in the upper-bound buffer included),
+ * prefix_sum_flop = copy of the totals to the host, load_balance =
  * buffer sizing and heavy-row segment planning, compute = merge into the
  * upper-bound buffer, prefix_sum_nnz = crpt scan, copy = compaction into C;
  * host drop-ins add pre_allocate = copies of A and B and cleanup = copy of
