@@ -210,6 +210,31 @@ class DeviceCSR:
                             self.val.data_ptr() if self.val.numel() else None)
 
 
+_CSR_ARRAY = np.dtype([("M", np.int32), ("N", np.int32), ("nnz", np.int32), ("pad", np.int32),
+                       ("rpt", np.uint64), ("col", np.uint64), ("val", np.uint64)])
+assert _CSR_ARRAY.itemsize == C.sizeof(_native.CsrC)
+
+
+def _csr_array(mats):
+    """The brm_csr array of many DeviceCSR (what c() gives one by one), filled
+    field by field: a batch of thousands of pairs makes no Python object per
+    matrix, and so does not set off the garbage collector on the caller's
+    tensors."""
+    a = np.zeros(len(mats), _CSR_ARRAY)
+    a["M"] = [m.M for m in mats]
+    a["N"] = [m.N for m in mats]
+    a["nnz"] = nnz = [m.col.numel() for m in mats]
+    a["rpt"] = [m.rpt.data_ptr() for m in mats]
+    a["col"] = [m.col.data_ptr() for m in mats]
+    a["val"] = [m.val.data_ptr() for m in mats]
+    if 0 in nnz:  # no entries: null arrays
+        a["col"][a["nnz"] == 0] = 0
+    a["val"][[m.val.numel() == 0 for m in mats]] = 0
+    p = a.ctypes.data_as(C.POINTER(_native.CsrC))
+    p._arr = a
+    return p
+
+
 class Context:
     """A brm_context bound to the current CUDA device and a stream."""
 
@@ -264,8 +289,8 @@ class Context:
         import torch
         n = len(pairs)
         code = _dtype_code(np.float64 if pairs[0][0].val.dtype == torch.float64 else np.float32)
-        As = (_native.CsrC * n)(*[a.c() for a, _ in pairs])
-        Bs = (_native.CsrC * n)(*[b.c() for _, b in pairs])
+        As = _csr_array([a for a, _ in pairs])
+        Bs = _csr_array([b for _, b in pairs])
         t = _native.TuningC()
         _native.check(self._L.brm_autotune(self._h, code, n, As, Bs, C.byref(t)), "brm_autotune")
         return {"seg_cut": t.seg_cut, "mid_flop": t.mid_flop, "long_scratch": t.long_scratch}
@@ -343,8 +368,8 @@ class Context:
         if any(a.val.dtype != dt or b.val.dtype != dt for a, b in pairs):
             raise TypeError("all pairs of a batch must have the same value type")
         code = _dtype_code(np.float64 if dt == torch.float64 else np.float32)
-        As = (_native.CsrC * n)(*[a.c() for a, _ in pairs])
-        Bs = (_native.CsrC * n)(*[b.c() for _, b in pairs])
+        As = _csr_array([a for a, _ in pairs])
+        Bs = _csr_array([b for _, b in pairs])
         out = _native.BatchC()
         _native.check(self._L.brm_batch_precise(self._h, code, n, As, Bs, C.byref(out)),
                       "brm_batch_precise")
@@ -474,8 +499,8 @@ class BatchGraph:
         n = len(self._pairs)
         dt = self._pairs[0][0].val.dtype
         code = _dtype_code(np.float64 if dt == torch.float64 else np.float32)
-        As = (_native.CsrC * n)(*[a.c() for a, _ in self._pairs])
-        Bs = (_native.CsrC * n)(*[b.c() for _, b in self._pairs])
+        As = _csr_array([a for a, _ in self._pairs])
+        Bs = _csr_array([b for _, b in self._pairs])
         out = _native.BatchC()
         _native.check(self._L.brm_batch_graph_create(ctx._h, code, n, As, Bs, C.byref(self._h),
                                                      C.byref(out)), "brm_batch_graph_create")
@@ -530,8 +555,8 @@ class BatchPipe:
             n = len(pairs)
             dt = pairs[0][0].val.dtype
             self._code = _dtype_code(np.float64 if dt == torch.float64 else np.float32)
-            As = (_native.CsrC * n)(*[a.c() for a, _ in pairs])
-            Bs = (_native.CsrC * n)(*[b.c() for _, b in pairs])
+            As = _csr_array([a for a, _ in pairs])
+            Bs = _csr_array([b for _, b in pairs])
             cc = _native.BatchCapsC()
             _native.check(self._L.brm_batch_caps_for(ctx._h, self._code, n, As, Bs,
                                                      float(headroom), C.byref(cc)),
@@ -553,8 +578,8 @@ class BatchPipe:
         import torch
         n = len(pairs)
         dt = pairs[0][0].val.dtype
-        As = (_native.CsrC * n)(*[a.c() for a, _ in pairs])
-        Bs = (_native.CsrC * n)(*[b.c() for _, b in pairs])
+        As = _csr_array([a for a, _ in pairs])
+        Bs = _csr_array([b for _, b in pairs])
         ptr = None
         if stream is not None:
             ptr = stream.cuda_stream if hasattr(stream, "cuda_stream") else int(stream)
