@@ -350,32 +350,21 @@ int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A,
         return BRM_SUCCESS;
     cudaStream_t s = brm::context_stream(ctx);
     const size_t vb = dtype == BRM_F64 ? 8 : 4;
-    // device scratch: the table, A_bd, B_bd (freed at the end)
-    Buf tab, abd, bbd;
-    auto cleanup = [&]() {
-        if (tab.p)
-            cudaFreeAsync(tab.p, s);
-        if (abd.p)
-            cudaFreeAsync(abd.p, s);
-        if (bbd.p)
-            cudaFreeAsync(bbd.p, s);
-    };
-    int st = grow_buf(tab, h.t.bytes, s);
+    // the table, A_bd and B_bd, in a buffer of the context
     const size_t a_rpt = a256(4 * (size_t)(ra + 1)), a_col = a256(4 * (size_t)std::max(na, 1LL));
     const size_t b_rpt = a256(4 * (size_t)(rb + 1)), b_col = a256(4 * (size_t)std::max(nb, 1LL));
-    if (st == BRM_SUCCESS)
-        st = grow_buf(abd, a_rpt + a_col + vb * (size_t)std::max(na, 1LL), s);
-    if (st == BRM_SUCCESS)
-        st = grow_buf(bbd, b_rpt + b_col + vb * (size_t)std::max(nb, 1LL), s);
-    if (st != BRM_SUCCESS) {
-        cleanup();
+    const size_t a_val = a256(vb * (size_t)std::max(na, 1LL)), t_all = a256(h.t.bytes);
+    void *buf = nullptr;
+    int st = brm::batch_scratch(
+        ctx, t_all + a_rpt + a_col + a_val + b_rpt + b_col + vb * (size_t)std::max(nb, 1LL), &buf);
+    if (st != BRM_SUCCESS)
         return st;
-    }
-    const BatchTable t = table_layout(tab.p, n);
-    int *A_rpt = (int *)abd.p, *A_col = (int *)((char *)abd.p + a_rpt);
-    void *A_val = (char *)abd.p + a_rpt + a_col;
-    int *B_rpt = (int *)bbd.p, *B_col = (int *)((char *)bbd.p + b_rpt);
-    void *B_val = (char *)bbd.p + b_rpt + b_col;
+    char *abd = (char *)buf + t_all, *bbd = abd + a_rpt + a_col + a_val;
+    const BatchTable t = table_layout(buf, n);
+    int *A_rpt = (int *)abd, *A_col = (int *)(abd + a_rpt);
+    void *A_val = abd + a_rpt + a_col;
+    int *B_rpt = (int *)bbd, *B_col = (int *)(bbd + b_rpt);
+    void *B_val = bbd + b_rpt + b_col;
     brm_csr Abd{(int)ra, (int)rb, (int)na, A_rpt, A_col, A_val};
     brm_csr Bbd{(int)rb, (int)cb, (int)nb, B_rpt, B_col, B_val};
     cudaError_t e = cudaMemcpyAsync(t.dims, h.t.dims, t.upload, cudaMemcpyHostToDevice, s);
@@ -387,7 +376,6 @@ int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A,
     }
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        cleanup();
         return BRM_ERR_CUDA;
     }
     // one Precise call on the stacked operands
@@ -395,10 +383,8 @@ int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A,
     void *cval = nullptr;
     int cnnz = 0;
     st = brm_precise_device(ctx, dtype, &Abd, &Bbd, &crpt, &ccol, &cval, &cnnz, nullptr);
-    if (st != BRM_SUCCESS) {
-        cleanup();
+    if (st != BRM_SUCCESS)
         return st;
-    }
     int *lrpt = nullptr;
     e = cudaMallocAsync((void **)&lrpt, sizeof(int) * (size_t)(ra + n), s);
     if (e == cudaSuccess) {
@@ -412,7 +398,6 @@ int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A,
                             cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess)
         e = cudaStreamSynchronize(s);
-    cleanup();
     if (!hf || !hr || e != cudaSuccess) {
         (void)cudaGetLastError();
         std::free(hf);
