@@ -529,63 +529,113 @@ __device__ __forceinline__ void copy_seg_run(SegRun *dst, const SegRun *src)
         cp_async16((unsigned char *)dst + 16 * q, (const unsigned char *)src + 16 * q);
 }
 
+constexpr int kSegNP = kSegCap / kSegThreads;  // products a lane
+static_assert(kSegCap % kSegThreads == 0 && kSegCap <= 4096, "12-bit columns, ranks and lists");
+
 template <typename T>
 struct SegLayout {
     static constexpr int NW = kSegThreads / 32;
-    static constexpr size_t o_loff = 0;
-    static constexpr size_t o_lbs = o_loff + mid_a16((kSegCap + 1) * 4);
-    static constexpr size_t o_lleaf = o_lbs + mid_a16(kSegCap * 4);
-    static constexpr size_t o_prc = o_lleaf + mid_a16(kSegCap * 2);
-    static constexpr size_t o_pval = o_prc + mid_a16(kSegCap * 4);
-    static constexpr size_t o_pleaf = o_pval + mid_a16(kSegCap * sizeof(T));
-    static constexpr size_t o_pu = o_pleaf + mid_a16(kSegCap * 2);
-    static constexpr size_t o_ia = o_pu + mid_a16(kSegCap * 2);
-    static constexpr size_t o_ib = o_ia + mid_a16(kSegCap * 2);
-    // the summary words of a wide segment and their ranks are dead before
-    // the scatter first writes ib, so they share its space
-    static constexpr size_t o_summ = o_ib;
+    // bitmap words, with the summary words of a wide segment and their ranks
+    // behind them; the values take their place
+    static constexpr size_t o_cw = 0;
+    static constexpr size_t o_val = 0;
+    static constexpr size_t o_summ = o_cw + mid_a16(kSegCap * 4);
     static constexpr size_t o_srank = o_summ + mid_a16(kSumWords * 4);
-    static_assert(kSumWords * 4 + kSumWords * 2 <= kSegCap * 2, "summary words fit in ib");
-    static constexpr size_t o_cw = o_ib + mid_a16(kSegCap * 2);
-    static constexpr size_t o_cwr = o_cw + mid_a16(kSegCap * 4);
-    static constexpr size_t o_long = o_cwr + mid_a16((kSegCap + 1) * 2);
-    static constexpr size_t o_ws = o_long + mid_a16(kLongMax * 2);
+    static constexpr size_t end_cw = o_srank + mid_a16(kSumWords * 2);
+    static constexpr size_t end_val = mid_a16(kSegCap * sizeof(T));
+    // list table: B offset less the product offset, then (dead) the order of a
+    // long column's products and the warps' bitmaps over the lists
+    static constexpr size_t o_lofs = end_cw > end_val ? end_cw : end_val;
+    static constexpr size_t o_ord = o_lofs;
+    static constexpr size_t o_bmp = o_ord + mid_a16(kSegCap * 2);
+    static constexpr size_t o_lleaf = o_lofs + mid_a16(kSegCap * 4);
+    static_assert(o_bmp + NW * kSegPWords * 6 <= o_lleaf, "the bitmaps fit in the list table");
+    static constexpr size_t o_pre = o_lleaf + mid_a16(kSegCap * 2);   // word prefixes, then runs
+    static constexpr size_t o_cnt = o_pre + mid_a16(kSegCap * 2);     // products of each column,
+    static constexpr size_t o_list = o_cnt;                           // then lists by position
+    static constexpr size_t o_ucol = o_cnt + mid_a16(kSegCap * 2);
+    // columns of two and of three or four products (from both ends), and of
+    // five to eight and more (the same)
+    static constexpr int n_a = kSegCap / 2, n_b = kSegCap / 5 + 2;
+    static constexpr size_t o_lista = o_ucol + mid_a16(kSegCap * 4);
+    static constexpr size_t o_listb = o_lista + mid_a16(n_a * 2);
+    static constexpr size_t o_llen = o_listb + mid_a16(n_b * 2);  // products of the long ones
+    static constexpr size_t o_sb = o_llen + mid_a16(kLongMax * 2);
+    static constexpr size_t o_ws = o_sb + mid_a16(kSegPWords * 4);
     static constexpr size_t o_misc = o_ws + mid_a16((NW + 1) * 8);
     static constexpr size_t o_run = o_misc + 64;  // the next segment's record
     static constexpr size_t bytes = o_run + sizeof(SegRun);
-    // per-warp p-bitmaps and their word prefixes live in cw once u is known
-    static_assert(NW * kSegPWords * 6 <= kSegCap * 4, "cw region holds the warp bitmaps");
 };
 
+// Prefix of the bit counts of words[0, n) into pre, a thread's words
+// consecutive (a multiple of four, so that threads 16 bytes apart in a phase
+// of a load fall on different banks); returns the total.
+template <int NT>
+__device__ __forceinline__ int seg_word_prefix(const unsigned *words, int n, unsigned short *pre,
+                                               int *ws)
+{
+    constexpr int MAXV = (kSegCap + 4 * NT - 1) / (4 * NT);  // 16-byte loads a thread
+    const int vt = (n + 4 * NT - 1) / (4 * NT);
+    int cnt[MAXV][4];
+    int sum = 0;
+#pragma unroll
+    for (int q = 0; q < MAXV; q++) {
+        const int i = 4 * (threadIdx.x * vt + q);
+        uint4 x = make_uint4(0, 0, 0, 0);
+        if (q < vt && i < n)
+            x = *(const uint4 *)&words[i];
+        cnt[q][0] = sum;
+        cnt[q][1] = cnt[q][0] + __popc(x.x);
+        cnt[q][2] = cnt[q][1] + __popc(x.y);
+        cnt[q][3] = cnt[q][2] + __popc(x.z);
+        sum = cnt[q][3] + __popc(x.w);
+    }
+    int tot;
+    const int ex = block_excl_scan<NT, int>(sum, ws, &tot);
+#pragma unroll
+    for (int q = 0; q < MAXV; q++) {
+        const int i = 4 * (threadIdx.x * vt + q);
+        if (q < vt && i < n)
+            *(ushort4 *)&pre[i] = make_ushort4(
+                (unsigned short)(ex + cnt[q][0]), (unsigned short)(ex + cnt[q][1]),
+                (unsigned short)(ex + cnt[q][2]), (unsigned short)(ex + cnt[q][3]));
+    }
+    return tot;
+}
+
 template <typename T, bool UPPER>
-__global__ void __launch_bounds__(kSegThreads, 512 / kSegThreads) k_seg_numeric(CsrDev A, CsrDev B, PlanDev P,
-                                                             const int *crpt, int *ccol, T *cval)
+__global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
+    k_seg_numeric(CsrDev A, CsrDev B, PlanDev P, const int *crpt, int *ccol, T *cval)
 {
     if (P.cnt->abort)  // a capacity check of a captured pipeline failed
         return;
-    constexpr int NT = kSegThreads;
+    constexpr int NT = kSegThreads, NP = kSegNP;
     using L = SegLayout<T>;
+    constexpr int NW = L::NW;
     extern __shared__ __align__(16) unsigned char smem[];
-    int *loff = (int *)(smem + L::o_loff);
-    int *ucnt = loff;  // per-column counts, then column starts (after staging)
-    int *lbs = (int *)(smem + L::o_lbs);
-    unsigned short *lleaf = (unsigned short *)(smem + L::o_lleaf);
-    int *prc = (int *)(smem + L::o_prc);
-    T *pval = (T *)(smem + L::o_pval);
-    unsigned short *pleaf = (unsigned short *)(smem + L::o_pleaf);
-    unsigned short *pu = (unsigned short *)(smem + L::o_pu);
-    unsigned short *ia = (unsigned short *)(smem + L::o_ia);
-    unsigned short *ib = (unsigned short *)(smem + L::o_ib);
+    unsigned *cw = (unsigned *)(smem + L::o_cw);
+    T *vals = (T *)(smem + L::o_val);
     unsigned *summ = (unsigned *)(smem + L::o_summ);
     unsigned short *srank = (unsigned short *)(smem + L::o_srank);
-    unsigned *cw = (unsigned *)(smem + L::o_cw);
-    unsigned short *cwr = (unsigned short *)(smem + L::o_cwr);
-    unsigned short *longu = (unsigned short *)(smem + L::o_long);
+    int *lofs = (int *)(smem + L::o_lofs);
+    unsigned short *ord = (unsigned short *)(smem + L::o_ord);
+    unsigned short *lleaf = (unsigned short *)(smem + L::o_lleaf);
+    unsigned short *pre = (unsigned short *)(smem + L::o_pre);
+    unsigned short *run = pre;
+    unsigned *cnt2 = (unsigned *)(smem + L::o_cnt);  // two 16-bit counts a word
+    const unsigned short *cnt = (const unsigned short *)(smem + L::o_cnt);
+    unsigned short *plist = (unsigned short *)(smem + L::o_list);
+    int *ucol = (int *)(smem + L::o_ucol);
+    unsigned short *lista = (unsigned short *)(smem + L::o_lista);
+    unsigned short *listb = (unsigned short *)(smem + L::o_listb);
+    unsigned short *llen = (unsigned short *)(smem + L::o_llen);
+    unsigned *sb = (unsigned *)(smem + L::o_sb);
     long long *ws = (long long *)(smem + L::o_ws);
     int *wsi = (int *)(smem + L::o_ws);
     int *misc = (int *)(smem + L::o_misc);
     SegRun *srun = (SegRun *)(smem + L::o_run);
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned ltm = lanemask_lt(), lem = ltm | (1u << lane);
     const int i0 = P.seg_range ? P.seg_range[0] : 0;
     const int nsegs = P.seg_range ? P.seg_range[1] : P.cnt->n_seg;
     const int *__restrict__ bcol = B.col;
@@ -605,32 +655,48 @@ __global__ void __launch_bounds__(kSegThreads, 512 / kSegThreads) k_seg_numeric(
             cp_async_wait_all();
             misc[0] = pf;
         }
+        if (tid < kSegPWords)
+            sb[tid] = 0;
         __syncthreads();
         const int item = misc[0];
         if (item >= nsegs)
             break;
         const SegRun d = *srun;
         if (tid == 0) {
-            pf = i0 + atomicAdd(&P.cnt->work_seg, 1);  // consumed after the staging
+            pf = i0 + atomicAdd(&P.cnt->work_seg, 1);  // consumed after the columns are read
             pf_copied = false;
         }
         const int row = d.row;
         const int a0 = d.a0;
         const int k = d.k;
         const int span = d.c_hi - d.c_lo;
-        // distinct columns of the row up to the next segment (checked at the end)
+        // distinct columns of the row up to the next segment (checked below)
         const int next_u = d.next_u;
         const int nsum = (span + 1023) >> 10;
         const int *sp0 = P.split + d.sp;
         const int *sp1 = sp0 + k;
-        // nonempty sub-lists of the segment, in leaf order (a thread takes
-        // four consecutive lists per pass: hub rows have thousands of lists
-        // and few products of each in one segment)
+        // a segment spanning at most 32 * kSegCap columns ranks its columns
+        // with one flat bitmap; wider ones with a summary bit per nonempty
+        // word and compressed words
+        const int nwf = (span + 31) >> 5;
+        const bool flat = nwf <= kSegCap;
+        {
+            uint4 *z = (uint4 *)(flat ? cw : summ);
+            const int nz = ((flat ? nwf : min(nsum, kSumWords)) + 3) >> 2;
+            for (int i = tid; i < nz; i += NT)
+                z[i] = make_uint4(0, 0, 0, 0);
+            for (int i = tid; i < kSegCap / 8; i += NT)
+                ((uint4 *)cnt2)[i] = make_uint4(0, 0, 0, 0);
+        }
+        // 1. nonempty sub-lists of the segment, in leaf order (a thread takes
+        //    four consecutive lists per pass: hub rows have thousands of lists
+        //    and few products of each in one segment), and a bit per list
+        //    start in product order
         constexpr int LPT = 4;
-        int lcarry = 0, pcarry = 0;
+        int nlists = 0, nprod = 0;
         for (int lb = 0; lb < k; lb += NT * LPT) {
             int st[LPT], len[LPT];
-            int cnt = 0, psum = 0;
+            int ne = 0, psum = 0;
 #pragma unroll
             for (int q = 0; q < LPT; q++) {
                 const int l = lb + tid * LPT + q;
@@ -640,436 +706,390 @@ __global__ void __launch_bounds__(kSegThreads, 512 / kSegThreads) k_seg_numeric(
                     st[q] = sp0[l];
                     len[q] = sp1[l] - st[q];
                 }
-                cnt += len[q] > 0;
+                ne += len[q] > 0;
                 psum += len[q];
             }
             long long tot;
             const long long ex = block_excl_scan<NT, long long>(
-                ((long long)cnt << 32) | (long long)psum, ws, &tot);
-            int li = lcarry + (int)(ex >> 32);
-            int po = pcarry + (int)(ex & 0xffffffffLL);
+                ((long long)ne << 32) | (long long)psum, ws, &tot);
+            int li = nlists + (int)(ex >> 32);
+            int po = nprod + (int)(ex & 0xffffffffLL);
 #pragma unroll
             for (int q = 0; q < LPT; q++) {
                 if (len[q] > 0) {
-                    if (li < kSegCap) {
-                        loff[li] = po;
-                        lbs[li] = st[q];
+                    if (li < kSegCap && po < kSegCap) {
+                        lofs[li] = st[q] - po;
                         lleaf[li] = (unsigned short)(lb + tid * LPT + q);
+                        atomicOr(&sb[po >> 5], 1u << (po & 31));
                     }
                     li++;
                     po += len[q];
                 }
             }
-            lcarry += (int)(tot >> 32);
-            pcarry += (int)(tot & 0xffffffffLL);
+            nlists += (int)(tot >> 32);
+            nprod += (int)(tot & 0xffffffffLL);
         }
-        const int nlists = lcarry, nprod = pcarry;
-        if (nprod > kSegCap || nprod != d.nprod || nsum > kSumWords || span <= 0) {
-            if (tid == 0)
+        if (nprod > kSegCap || nprod != d.nprod || nsum > kSumWords || span <= 0 || nprod == 0) {
+            // (the columns before a chunk's first cut may hold no product)
+            if (tid == 0 && !(nprod == 0 && d.nprod == 0 && next_u == d.u_off))
                 atomicOr(&P.cnt->err, kErrWindowOverflow);
+            __syncthreads();
             continue;
         }
-        if (tid == 0) {
-            loff[nlists] = nprod;
-            misc[1] = 0;  // long runs
-            misc[2] = 0;  // staged column out of range
-            misc[3] = 0;  // listed columns of three or four products
-            misc[4] = 0;  // listed columns of five to eight products
-        }
-        // a segment spanning at most 32 * kSegCap columns ranks its columns
-        // with one flat bitmap in cw (a prefix per word); wider ones with a
-        // summary bit per nonempty word and compressed words
-        const bool flat = span <= 32 * kSegCap;
-        const int nwf = (span + 31) >> 5;
-        if (flat) {
-            for (int i = tid; i < nwf; i += NT)
-                cw[i] = 0;
-        } else {
-            for (int i = tid; i < nsum; i += NT)
-                summ[i] = 0;
-        }
+        if (tid < 8)
+            misc[1 + tid] = 0;  // columns of each size, positions, an input error
         __syncthreads();
-        // stage products in list-major (= leaf) order; mark their words in the
-        // flat bitmap or in the summary
-        const int ipt = (nprod + NT - 1) / NT;
-        const int p0 = min(tid * ipt, nprod), p1 = min(p0 + ipt, nprod);
-        // a thread's products are column-sorted within each list, so runs of
-        // equal summary words are OR-ed in a register and flushed once
-        unsigned run_w = 0xffffffffu, run_b = 0;
-        if (p0 < p1) {
-            int j = last_le(loff, nlists, p0);
-            int lbeg = loff[j], lend = loff[j + 1], bsj = lbs[j];
-            for (int p = p0; p < p1; p += kGatherBatch) {
-                const int n = min(kGatherBatch, p1 - p);
-                int addr[kGatherBatch], lid[kGatherBatch], c[kGatherBatch];
-                T bv[kGatherBatch], av[kGatherBatch];
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; i++) {
-                    if (i < n) {
-                        while (p + i >= lend) {
-                            j++;
-                            lbeg = lend;
-                            lend = loff[j + 1];
-                            bsj = lbs[j];
-                        }
-                        addr[i] = bsj + (p + i - lbeg);
-                        lid[i] = j;
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; i++) {
-                    if (i < n) {
-                        const bool in = BRM_IN(P.cnt, addr[i], B.nnz);
-                        c[i] = in ? bcol[addr[i]] : d.c_lo;
-                        bv[i] = in ? bval[addr[i]] : T(0);
-                        av[i] = aval[a0 + lleaf[lid[i]]];
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; i++) {
-                    if (i < n) {
-                        const int e = p + i;
-                        int rc = c[i] - d.c_lo;
-                        if ((unsigned)rc >= (unsigned)span) {
-                            misc[2] = 1;
-                            rc = 0;
-                        }
-                        prc[e] = rc;
-                        pval[e] = vmul(av[i], bv[i]);
-                        pleaf[e] = lleaf[lid[i]];
-                        const unsigned sw = (unsigned)rc >> (flat ? 5 : 10);
-                        if (sw != run_w) {
-                            if (run_b)
-                                atomicOr(flat ? &cw[run_w] : &summ[run_w], run_b);
-                            run_w = sw;
-                            run_b = 0;
-                        }
-                        run_b |= 1u << ((rc >> (flat ? 0 : 5)) & 31);
-                    }
-                }
-            }
-            if (run_b)
-                atomicOr(flat ? &cw[run_w] : &summ[run_w], run_b);
+        // 2. this warp's words of 32 products, [w0, w0 + nw): columns into
+        //    registers, their bits into the bitmap or the summary.  Lanes
+        //    beyond the last product take no part from the counting on
+        const int nwd = (nprod + 31) >> 5;
+        const int npw = (nwd + NW - 1) / NW;
+        const int w0 = w * npw;
+        const int nw = min(npw, nwd - w0);
+        int jb = -1;  // lists that start before the word, less one
+        {
+            int x = 0;
+            for (int i = lane; i < w0 && i < nwd; i += 32)
+                x += __popc(sb[i]);
+            jb += __reduce_add_sync(kFull, x);
         }
+        int c[NP];        // column, from c_lo; then the product's turn in its column
+        unsigned pk[NP];  // list << 17 | word slot << 5 | column in the word; then list << 12 | u
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+            if (u < nw) {
+                const int e = min((w0 + u) * 32 + lane, nprod - 1);
+                const unsigned bits = sb[w0 + u];
+                const int j = jb + __popc(bits & lem);
+                jb += __popc(bits);
+                pk[u] = (unsigned)j << 17;
+                const int bi = lofs[j] + e;
+                c[u] = BRM_IN(P.cnt, bi, B.nnz) ? bcol[bi] : d.c_lo;
+            }
+        }
+        bool bad = false;
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+            if (u < nw) {
+                c[u] -= d.c_lo;
+                if ((unsigned)c[u] >= (unsigned)span) {
+                    bad = true;  // a column outside the segment: unsorted rows of B
+                    c[u] = 0;
+                }
+                const int x = flat ? c[u] : c[u] >> 5;
+                unsigned *q = (flat ? cw : summ) + (x >> 5);
+                const unsigned b = 1u << (x & 31);
+                if (flat)
+                    pk[u] |= (unsigned)c[u];
+                if (!(*q & b))
+                    atomicOr(q, b);
+            }
+        }
+        if (bad)
+            misc[6] = 1;
         __syncthreads();
         // every thread has read this segment's record: copy the next one
         if (tid == 0 && pf < nsegs) {
             copy_seg_run(srun, P.run + pf);
             pf_copied = true;
         }
-        if (misc[2]) {  // a column outside the segment: the plan does not match the input
+        if (misc[6]) {  // the plan does not match the input
             if (tid == 0)
                 atomicOr(&P.cnt->err, kErrBadInput);
+            __syncthreads();
             continue;
         }
-        // compressed words: one per nonempty 32-column word (flat: every word)
         int ncw = nwf;
         if (!flat) {
-            // SPT consecutive summary words a thread (nsum <= kSumWords)
-            constexpr int SPT = (kSumWords + NT - 1) / NT;
-            const int s0 = min(tid * SPT, nsum), s1 = min(s0 + SPT, nsum);
-            int sc = 0;
-            for (int i = s0; i < s1; i++)
-                sc += __popc(summ[i]);
-            long long ncw_t;
-            int sx = (int)block_excl_scan<NT, long long>(sc, ws, &ncw_t);
-            for (int i = s0; i < s1; i++) {
-                srank[i] = (unsigned short)sx;
-                sx += __popc(summ[i]);
-            }
-            ncw = (int)ncw_t;
-            for (int i = tid; i < ncw; i += NT)
-                cw[i] = 0;
-            for (int i = tid; i <= nprod; i += NT)  // the sub-list table is dead now
-                ucnt[i] = 0;
+            // slots of the nonempty words
+            ncw = seg_word_prefix<NT>(summ, nsum, srank, wsi);
+            for (int i = tid; i < (ncw + 3) >> 2; i += NT)
+                ((uint4 *)cw)[i] = make_uint4(0, 0, 0, 0);
             __syncthreads();
-        }
-        // mark the compressed words; keep each product's word index in pu
-        if (!flat) {
-            int run_ci = -1;
-            unsigned bits = 0;
-            for (int p = p0; p < p1; p++) {
-                const int rc = prc[p];
-                const int w = rc >> 5;
-                const int ci = srank[w >> 5] + __popc(summ[w >> 5] & ((1u << (w & 31)) - 1u));
-                pu[p] = (unsigned short)ci;
-                if (ci != run_ci) {
-                    if (bits)
-                        atomicOr(&cw[run_ci], bits);
-                    run_ci = ci;
-                    bits = 0;
+#pragma unroll
+            for (int u = 0; u < NP; u++) {
+                if (u < nw) {
+                    const int sw = c[u] >> 10;
+                    const unsigned b = 1u << (c[u] & 31);
+                    const int ci = srank[sw] + __popc(summ[sw] & ((1u << ((c[u] >> 5) & 31)) - 1u));
+                    pk[u] |= ((unsigned)ci << 5) | (unsigned)(c[u] & 31);
+                    if (!(cw[ci] & b))
+                        atomicOr(&cw[ci], b);
                 }
-                bits |= 1u << (rc & 31);
             }
-            if (bits)
-                atomicOr(&cw[run_ci], bits);
             __syncthreads();
-        } else {
-            // a flat segment clears the column counts here (the sub-list
-            // table they overwrite is dead since the staging barrier); the
-            // barrier of the rank scan below orders them before the counting
-            for (int i = tid; i <= nprod; i += NT)
-                ucnt[i] = 0;
         }
-        // ranks of the compressed words -> distinct columns before each word
-        long long U_t;
-        {
-            const int cpt = (ncw + NT - 1) / NT;
-            const int c0 = min(tid * cpt, ncw), c1 = min(c0 + cpt, ncw);
-            int cs = 0;
-            for (int i = c0; i < c1; i++)
-                cs += __popc(cw[i]);
-            int r = (int)block_excl_scan<NT, long long>(cs, ws, &U_t);
-            for (int i = c0; i < c1; i++) {
-                cwr[i] = (unsigned short)r;
-                r += __popc(cw[i]);
-            }
-        }
-        const int U = (int)U_t;
-        const bool nodup = (U == nprod);
-        __syncthreads();
-        // u = distinct-column rank of each product; count the products of
-        // every column (the rank within a column, from the atomic, is in
-        // arbitrary order and is put in leaf order when the column is reduced)
-        for (int p = p0; p < p1; p++) {
-            const int rc = prc[p];
-            const int ci = flat ? rc >> 5 : pu[p];
-            const int u = cwr[ci] + __popc(cw[ci] & ((1u << (rc & 31)) - 1u));
-            pu[p] = (unsigned short)u;
-            if (!nodup && BRM_IN(P.cnt, u, U))
-                ia[p] = (unsigned short)atomicAdd(&ucnt[u], 1);
-        }
-        __syncthreads();
-        const long long obase = (UPPER ? P.scan_flop[row] : (long long)crpt[row]) + d.u_off;
-        unsigned short *S = ib;
-        if (nodup) {
-            // every column has one contribution: position u holds product e
-            for (int p = p0; p < p1; p++)
-                if (BRM_IN(P.cnt, pu[p], nprod))
-                    S[pu[p]] = (unsigned short)p;
-        } else {
-            // exclusive scan of the column counts (in place), then scatter
-            const int cpt = (U + NT - 1) / NT;
-            const int c0 = min(tid * cpt, U), c1 = min(c0 + cpt, U);
-            int cs = 0;
-            for (int i = c0; i < c1; i++)
-                cs += ucnt[i];
-            long long tot;
-            int r = (int)block_excl_scan<NT, long long>(cs, ws, &tot);
-            for (int i = c0; i < c1; i++) {
-                const int c = ucnt[i];
-                ucnt[i] = r;
-                r += c;
-            }
+        // 3. distinct columns, and those before each word
+        const int U = seg_word_prefix<NT>(cw, ncw, pre, wsi);
+        const bool nodup = U == nprod;
+        if (U != next_u - d.u_off) {  // must produce exactly its share of the row's columns
             if (tid == 0)
-                ucnt[U] = nprod;
+                atomicOr(&P.cnt->err, kErrNnzMismatch);
             __syncthreads();
-            for (int p = p0; p < p1; p++)
-                if (BRM_IN(P.cnt, ucnt[pu[p]] + ia[p], nprod))
-                    S[ucnt[pu[p]] + ia[p]] = (unsigned short)p;
+            continue;
         }
         __syncthreads();
-        // one thread per output column of one or two products (consecutive
-        // columns -> coalesced stores); columns of three or four and of five to
-        // eight products are listed (at the front and the back of pu, dead
-        // after the scatter) and reduced by a second, dense pass, so that the
-        // lanes of a warp run the same code; longer columns go to longu
-        for (int u = tid; u < U; u += NT) {
-            int i0 = u, len = 1;
-            if (!nodup) {
-                i0 = ucnt[u];
-                len = ucnt[u + 1] - i0;
-            }
-            const int e0 = S[i0];
-            T v;
-            if (len == 1) {
-                v = pval[e0];
-            } else if (len == 2) {
-                const int e1 = S[i0 + 1];
-                v = pleaf[e0] < pleaf[e1] ? vadd(pval[e0], pval[e1])   // left + right
-                                          : vadd(pval[e1], pval[e0]);
-            } else if (len <= 4) {
-                pu[atomicAdd(&misc[3], 1)] = (unsigned short)u;
-                continue;
-            } else if (len <= 8) {
-                pu[kSegCap - 1 - atomicAdd(&misc[4], 1)] = (unsigned short)u;
-                continue;
-            } else {
-                const int li = atomicAdd(&misc[1], 1);
-                if (li < kLongMax)
-                    longu[li] = (unsigned short)u;
-                continue;
-            }
-            if (BRM_IN(P.cnt, obase + u, P.c_cap)) {
-                ccol[obase + u] = d.c_lo + prc[e0];
-                cval[obase + u] = v;
+        // 4. column rank of each product and its turn among the column's (in
+        //    arbitrary order)
+#pragma unroll
+        for (int u = 0; u < NP; u++) {
+            if (u < nw) {
+                const int ci = (int)((pk[u] >> 5) & 0xfffu);
+                const int r = pre[ci] + __popc(cw[ci] & ((1u << (pk[u] & 31u)) - 1u));
+                pk[u] = ((pk[u] >> 17) << 12) | (unsigned)r;
+                ucol[r] = c[u];
+                c[u] = 0;
+                if (!nodup && (w0 + u) * 32 + lane < nprod) {
+                    const int sh = 16 * (r & 1);
+                    c[u] = (int)((atomicAdd(&cnt2[r >> 1], 1u << sh) >> sh) & 0xffffu);
+                }
             }
         }
         __syncthreads();
-        const int n34 = misc[3], nmid = n34 + misc[4];
-        for (int i = tid; i < nmid; i += NT) {
-            const int u = i < n34 ? pu[i] : pu[kSegCap - 1 - (i - n34)];
-            const int i0 = ucnt[u], len = ucnt[u + 1] - i0;
-            const int e0 = S[i0];
-            T v;
-            if (len <= 4) {
-                // sort the (leaf, value) pairs in registers, then the closed form
-                const int e1 = S[i0 + 1], e2 = S[i0 + 2];
-                int l0 = pleaf[e0], l1 = pleaf[e1], l2 = pleaf[e2];
-                T v0 = pval[e0], v1 = pval[e1], v2 = pval[e2];
-                if (len == 3) {
+        // 5. columns of several products: positions for the second and further
+        //    ones (column u's i-th at run[u] + i, its first at u), lists by size
+        if (!nodup) {
+            for (int ib = w * 32; ib < U; ib += NT) {
+                const int u = ib + lane;
+                const int n = u < U ? cnt[u] : 0;
+                const unsigned mb = __ballot_sync(kFull, n > 1);
+                if (!mb)
+                    continue;
+                const int x = n > 1 ? n - 1 : 0;
+                const int inc = warp_incl_scan(x);
+                int at = 0;
+                if (lane == 31)
+                    at = atomicAdd(&misc[5], inc);
+                at = __shfl_sync(kFull, at, 31) + inc - x;
+                // one list position a column: a warp's columns of one size together
+                const int cls = n == 2 ? 0 : n <= 4 ? 1 : n <= 8 ? 2 : 3;
+                unsigned left = mb;
+                int o = 0;
+                while (left) {
+                    const int k0 = __shfl_sync(kFull, cls, __ffs(left) - 1);
+                    const unsigned same = __ballot_sync(kFull, n > 1 && cls == k0);
+                    int first = 0;
+                    if (lane == 0)
+                        first = atomicAdd(&misc[1 + k0], __popc(same));
+                    first = __shfl_sync(kFull, first, 0);
+                    if (cls == k0)
+                        o = first + __popc(same & ltm);
+                    left &= ~same;
+                }
+                if (n > 1) {
+                    run[u] = (unsigned short)(U - 1 + at);
+                    // (the size beside the column's 12 bits)
+                    if (cls == 0)
+                        lista[o] = (unsigned short)u;
+                    else if (cls == 1)
+                        lista[L::n_a - 1 - o] = (unsigned short)(u | ((n - 3) << 12));
+                    else if (cls == 2)
+                        listb[o] = (unsigned short)(u | ((n - 5) << 12));
+                    else {
+                        listb[L::n_b - 1 - o] = (unsigned short)u;
+                        llen[o] = (unsigned short)n;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        const int n2 = misc[1], n34 = misc[2], n58 = misc[3], nlong = misc[4];
+        // 6. values to their positions
+        {
+            constexpr int VB = 4;  // gathers in flight a lane
+            static_assert(NP % VB == 0, "whole batches");
+#pragma unroll
+            for (int ub = 0; ub < NP; ub += VB) {
+                if (ub < nw) {
+                    T bv[VB], av[VB];
+                    int lf[VB];
+#pragma unroll
+                    for (int q = 0; q < VB; q++) {
+                        const int u = ub + q;
+                        if (u < nw) {
+                            const int j = (int)(pk[u] >> 12);
+                            const int bi = lofs[j] + min((w0 + u) * 32 + lane, nprod - 1);
+                            lf[q] = lleaf[j];
+                            bv[q] = BRM_IN(P.cnt, bi, B.nnz) ? bval[bi] : T(0);
+                            av[q] = aval[a0 + lf[q]];
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < VB; q++) {
+                        const int u = ub + q;
+                        if (u < nw && (w0 + u) * 32 + lane < nprod) {
+                            int p = (int)(pk[u] & 0xfffu);
+                            if (c[u])
+                                p = run[p] + c[u];
+                            vals[p] = vmul(av[q], bv[q]);
+                            plist[p] = (unsigned short)(pk[u] >> 12);
+                        }
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        // 7. columns of several products, each size by its own loop so that
+        //    the lanes of a warp run the same code; the value to position u
+        if (!nodup) {
+            for (int i = tid; i < n2; i += NT) {
+                const int u = lista[i];
+                vals[u] = vadd(vals[u], vals[run[u] + 1]);
+            }
+            for (int i = tid; i < n34; i += NT) {
+                const int x = lista[L::n_a - 1 - i], u = x & 0xfff, p = run[u];
+                // sort the (list, value) pairs in registers, then the closed form
+                int l0 = plist[u], l1 = plist[p + 1], l2 = plist[p + 2];
+                T v0 = vals[u], v1 = vals[p + 1], v2 = vals[p + 2];
+                if (!(x >> 12)) {
                     leaf_cas(l0, v0, l1, v1);
                     leaf_cas(l1, v1, l2, v2);
                     leaf_cas(l0, v0, l1, v1);
-                    v = trie3(l0, l1, l2, v0, v1, v2);
+                    vals[u] = trie3<T>(lleaf[l0], lleaf[l1], lleaf[l2], v0, v1, v2);
                 } else {
-                    const int e3 = S[i0 + 3];
-                    int l3 = pleaf[e3];
-                    T v3 = pval[e3];
+                    int l3 = plist[p + 3];
+                    T v3 = vals[p + 3];
                     leaf_cas(l0, v0, l1, v1);
                     leaf_cas(l2, v2, l3, v3);
                     leaf_cas(l0, v0, l2, v2);
                     leaf_cas(l1, v1, l3, v3);
                     leaf_cas(l1, v1, l2, v2);
-                    v = trie4(l0, l1, l2, l3, v0, v1, v2, v3);
+                    vals[u] = trie4<T>(lleaf[l0], lleaf[l1], lleaf[l2], lleaf[l3], v0, v1, v2, v3);
                 }
-            } else {
+            }
+            for (int i = tid; i < n58; i += NT) {
+                const int y = listb[i], u = y & 0xfff, p = run[u], len = 5 + (y >> 12);
                 // sorting network and a register stack
                 int l8[8];
                 T v8[8];
 #pragma unroll
                 for (int j = 0; j < 8; j++) {
+                    l8[j] = INT_MAX;
+                    v8[j] = T(0);
                     if (j < len) {
-                        const int e = S[i0 + j];
-                        l8[j] = pleaf[e];
-                        v8[j] = pval[e];
-                    } else {
-                        l8[j] = INT_MAX;
-                        v8[j] = T(0);
+                        const int x = j ? p + j : u;
+                        l8[j] = plist[x];
+                        v8[j] = vals[x];
                     }
                 }
                 leaf_sort8(l8, v8);
                 RegShiftReduce<T, 8> sr;
-                sr.init(l8[0], v8[0]);
+                sr.init(lleaf[l8[0]], v8[0]);
 #pragma unroll
                 for (int j = 1; j < 8; j++)
                     if (j < len)
-                        sr.push(l8[j], v8[j]);
-                v = sr.finish();
+                        sr.push(lleaf[l8[j]], v8[j]);
+                vals[u] = sr.finish();
             }
-            if (BRM_IN(P.cnt, obase + u, P.c_cap)) {
-                ccol[obase + u] = d.c_lo + prc[e0];
-                cval[obase + u] = v;
+        }
+        // columns with more than eight products: one warp each puts them in
+        // list order with a bitmap over the lists and hands them to the column
+        // reducer through the long-column scratch; when the scratch is full
+        // it reduces them itself (across its lanes up to 32 products, in its
+        // first lane beyond)
+        const long long obase = (UPPER ? P.scan_flop[row] : (long long)crpt[row]) + d.u_off;
+        if (nlong > 0) {
+            unsigned *bmp = (unsigned *)(smem + L::o_bmp) + w * kSegPWords;
+            unsigned short *wpre =
+                (unsigned short *)((unsigned *)(smem + L::o_bmp) + NW * kSegPWords) + w * kSegPWords;
+            const int nwl = (nlists + 31) >> 5;
+            T *lval = (T *)P.long_val;
+            for (int lb = w; lb < nlong; lb += 32 * NW) {
+                // the warp's next (up to) 32 columns lb + j * NW: one
+                // reservation of long-column scratch covers all of them
+                const int lj = lb + lane * NW;
+                int lu = 0, ln = 0;
+                if (lj < nlong) {
+                    lu = listb[L::n_b - 1 - lj];
+                    ln = llen[lj];
+                }
+                const int ncol = __popc(__ballot_sync(kFull, lj < nlong));
+                const int lincl = warp_incl_scan(ln);
+                unsigned long long rcol = 0, relem = 0;
+                if (lane == 31) {
+                    rcol = atomicAdd(&P.cnt->long_cols, (unsigned long long)ncol);
+                    relem = atomicAdd(&P.cnt->long_elems, (unsigned long long)lincl);
+                }
+                rcol = __shfl_sync(kFull, rcol, 31);
+                relem = __shfl_sync(kFull, relem, 31);
+                for (int jc = 0; jc < ncol; jc++) {
+                    const int u = __shfl_sync(kFull, lu, jc);
+                    const int len = __shfl_sync(kFull, ln, jc);
+                    const int rp = run[u];
+                    const long long lci = (long long)rcol + jc;
+                    const long long leo =
+                        (long long)relem + __shfl_sync(kFull, lincl - ln, jc);
+                    const bool handoff = lci < P.long_cap_cols && leo + len <= P.long_cap_elems;
+                    for (int x = lane; x < nwl; x += 32)
+                        bmp[x] = 0;
+                    __syncwarp();
+                    for (int i = lane; i < len; i += 32) {
+                        const int l = plist[i ? rp + i : u];
+                        atomicOr(&bmp[l >> 5], 1u << (l & 31));
+                    }
+                    __syncwarp();
+                    {
+                        const int x0 = lane * 3;
+                        const int c0 = x0 < nwl ? __popc(bmp[x0]) : 0;
+                        const int c1 = x0 + 1 < nwl ? __popc(bmp[x0 + 1]) : 0;
+                        const int c2 = x0 + 2 < nwl ? __popc(bmp[x0 + 2]) : 0;
+                        const int ex = warp_incl_scan(c0 + c1 + c2) - (c0 + c1 + c2);
+                        if (x0 < nwl)
+                            wpre[x0] = (unsigned short)ex;
+                        if (x0 + 1 < nwl)
+                            wpre[x0 + 1] = (unsigned short)(ex + c0);
+                        if (x0 + 2 < nwl)
+                            wpre[x0 + 2] = (unsigned short)(ex + c0 + c1);
+                    }
+                    __syncwarp();
+                    for (int i = lane; i < len; i += 32) {
+                        const int x = i ? rp + i : u;
+                        const int l = plist[x];
+                        const int r = wpre[l >> 5] + __popc(bmp[l >> 5] & ((1u << (l & 31)) - 1u));
+                        if (handoff) {
+                            P.long_leaf[leo + r] = lleaf[l];
+                            lval[leo + r] = vals[x];
+                        } else {
+                            ord[r ? rp + r : u] = (unsigned short)x;
+                        }
+                    }
+                    if (lci < P.long_cap_cols && lane == 0) {
+                        LongCol lc;
+                        lc.out = obase + u;
+                        lc.off = leo;
+                        lc.col = d.c_lo + ucol[u];
+                        lc.len = handoff ? len : -1;
+                        P.long_col[lci] = lc;
+                    }
+                    __syncwarp();
+                    if (handoff)
+                        continue;
+                    if (len <= 32) {
+                        const int x = ord[lane > 0 && lane < len ? rp + lane : u];
+                        const T r = warp_trie<T>(lleaf[plist[x]], vals[x], len);
+                        __syncwarp();
+                        if (lane == 0)
+                            vals[u] = r;
+                    } else if (lane == 0) {
+                        ShiftReduce<T, 17> sr;
+                        sr.init(lleaf[plist[ord[u]]], vals[ord[u]]);
+                        for (int i = 1; i < len; i++)
+                            sr.push(lleaf[plist[ord[rp + i]]], vals[ord[rp + i]]);
+                        vals[u] = sr.finish();
+                    }
+                    __syncwarp();
+                }
             }
         }
         __syncthreads();
-        // columns with more than eight products: one warp each puts them in
-        // leaf order (= staging order p, which it ranks with a bitmap over
-        // p) and hands them to the column reducer through the long-column
-        // scratch; when the scratch is full it reduces them itself (across
-        // its lanes up to 32 products, in its first lane beyond)
-        const int nlong = min(misc[1], kLongMax);
-        {
-            const int lane = tid & 31, wid = tid >> 5;
-            unsigned *bmp = cw + wid * kSegPWords;
-            unsigned short *wpre = (unsigned short *)(cw + L::NW * kSegPWords) + wid * kSegPWords;
-            const int nwp = (nprod + 31) >> 5;
-            T *lval = (T *)P.long_val;
-            for (int lb = wid; lb < nlong; lb += 32 * L::NW) {
-              // the warp's next (up to) 32 columns lb + j * NW: one
-              // reservation of long-column scratch covers all of them
-              const int lj = lb + lane * L::NW;
-              int myu = 0, mylen = 0;
-              if (lj < nlong) {
-                  myu = longu[lj];
-                  mylen = ucnt[myu + 1] - ucnt[myu];
-              }
-              const int ncol = __popc(__ballot_sync(kFull, lj < nlong));
-              const int lincl = warp_incl_scan(mylen);
-              unsigned long long rcol = 0, relem = 0;
-              if (lane == 31) {
-                  rcol = atomicAdd(&P.cnt->long_cols, (unsigned long long)ncol);
-                  relem = atomicAdd(&P.cnt->long_elems, (unsigned long long)lincl);
-              }
-              rcol = __shfl_sync(kFull, rcol, 31);
-              relem = __shfl_sync(kFull, relem, 31);
-              for (int jc = 0; jc < ncol; jc++) {
-                const int u = __shfl_sync(kFull, myu, jc);
-                const int len = __shfl_sync(kFull, mylen, jc);
-                const int i0 = ucnt[u], i1 = i0 + len;
-                const long long lci = (long long)rcol + jc;
-                const long long leo = (long long)relem + __shfl_sync(kFull, lincl - mylen, jc);
-                const bool handoff = lci < P.long_cap_cols && leo + len <= P.long_cap_elems;
-                for (int w = lane; w < nwp; w += 32)
-                    bmp[w] = 0;
-                __syncwarp();
-                for (int i = i0 + lane; i < i1; i += 32) {
-                    const int p = S[i];
-                    atomicOr(&bmp[p >> 5], 1u << (p & 31));
-                }
-                __syncwarp();
-                {
-                    const int w0 = lane * 3;
-                    const int c0 = w0 < nwp ? __popc(bmp[w0]) : 0;
-                    const int c1 = w0 + 1 < nwp ? __popc(bmp[w0 + 1]) : 0;
-                    const int c2 = w0 + 2 < nwp ? __popc(bmp[w0 + 2]) : 0;
-                    const int ex = warp_incl_scan(c0 + c1 + c2) - (c0 + c1 + c2);
-                    if (w0 < nwp)
-                        wpre[w0] = (unsigned short)ex;
-                    if (w0 + 1 < nwp)
-                        wpre[w0 + 1] = (unsigned short)(ex + c0);
-                    if (w0 + 2 < nwp)
-                        wpre[w0 + 2] = (unsigned short)(ex + c0 + c1);
-                }
-                __syncwarp();
-                for (int i = i0 + lane; i < i1; i += 32) {
-                    const int p = S[i];
-                    const int r = wpre[p >> 5] + __popc(bmp[p >> 5] & ((1u << (p & 31)) - 1u));
-                    if (handoff) {
-                        P.long_leaf[leo + r] = pleaf[p];
-                        lval[leo + r] = pval[p];
-                    } else {
-                        if (BRM_IN(P.cnt, i0 + r, nprod))
-                            ia[i0 + r] = (unsigned short)p;
-                    }
-                }
-                if (lci < P.long_cap_cols && lane == 0) {
-                    LongCol c;
-                    c.out = obase + u;
-                    c.off = leo;
-                    c.col = d.c_lo + prc[S[i0]];
-                    c.len = handoff ? len : -1;
-                    P.long_col[lci] = c;
-                }
-                __syncwarp();
-                if (handoff)
-                    continue;
-                if (len <= 32) {
-                    const int e = ia[i0 + (lane < len ? lane : 0)];
-                    const T r = warp_trie<T>(pleaf[e], pval[e], len);
-                    if (lane == 0) {
-                        if (BRM_IN(P.cnt, obase + u, P.c_cap)) {
-                            ccol[obase + u] = d.c_lo + prc[e];
-                            cval[obase + u] = r;
-                        }
-                    }
-                } else if (lane == 0) {
-                    ShiftReduce<T, 17> sr;
-                    sr.init(pleaf[ia[i0]], pval[ia[i0]]);
-                    for (int i = i0 + 1; i < i1; i++)
-                        sr.push(pleaf[ia[i]], pval[ia[i]]);
-                    if (BRM_IN(P.cnt, obase + u, P.c_cap)) {
-                        ccol[obase + u] = d.c_lo + prc[ia[i0]];
-                        cval[obase + u] = sr.finish();
-                    }
-                }
-                __syncwarp();
-              }
+        // 8. the segment's columns (the column reducer overwrites those handed
+        //    to it)
+        for (int u = tid; u < U; u += NT) {
+            if (BRM_IN(P.cnt, obase + u, P.c_cap)) {
+                ccol[obase + u] = d.c_lo + ucol[u];
+                cval[obase + u] = vals[u];
             }
         }
-        // the segment must produce exactly its share of the row's columns
-        if (tid == 0 && U != next_u - d.u_off)
-            atomicOr(&P.cnt->err, kErrNnzMismatch);
         __syncthreads();
     }
 }
