@@ -351,4 +351,38 @@ __device__ __forceinline__ T warp_trie(int leaf, T v, int n)
     return v;
 }
 
+// The same for two columns at once, one per half warp (lane 16 h + j < 16 h + n
+// holds the j-th smallest of the n <= 16 leaves of half h's column); results in
+// lanes 0 and 16.  A round joins every adjacent pair whose split level is
+// below its neighbours' (such pairs are siblings too), in as many rounds as
+// the tree is deep or fewer.  Adjacent splits differ unless leaves are equal
+// (a list that repeats a column): then the last pair of the equal ones joins,
+// so every round joins some pair.
+template <typename T>
+__device__ __forceinline__ T half_trie(int leaf, T v, int n)
+{
+    const int lane = threadIdx.x & 31, hl = lane & 15, hb = lane & 16;
+    bool alive = hl < n;
+    for (;;) {
+        const unsigned am = (__ballot_sync(kFull, alive) >> hb) & 0xffffu;
+        if (!__any_sync(kFull, (am & (am - 1u)) != 0u))
+            break;
+        const unsigned after = am & ~((2u << hl) - 1u), before = am & ((1u << hl) - 1u);
+        const bool has = alive && after != 0u;
+        const int nl = has ? __ffs(after) - 1 + hb : lane;
+        const int pl = before ? 31 - __clz(before) + hb : lane;
+        const int kn = __shfl_sync(kFull, leaf, nl);
+        const T vn = __shfl_sync(kFull, v, nl);
+        const int s = has ? split_level(leaf, kn) : 64;
+        const int sp = __shfl_sync(kFull, s, pl), sn = __shfl_sync(kFull, s, nl);
+        const bool comb = has && s < sn && (!before || s <= sp);
+        if (comb)
+            v = vadd(v, vn);
+        const unsigned cm = __ballot_sync(kFull, comb);
+        if (before && ((cm >> pl) & 1u))
+            alive = false;
+    }
+    return v;
+}
+
 }  // namespace brm

@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(256) k_split(CsrDev A, CsrDev B, PlanDev P)
 // ---------------------------------------------------------------------------
 // 3. segment kernel
 // ---------------------------------------------------------------------------
-constexpr int kLongMin = 9;  // columns with this many products are reduced by warps
+constexpr int kLongMin = 17;  // columns with this many products are handed to the column reducers
 constexpr int kLongMax = kSegCap / kLongMin + 1;
 constexpr int kSegPWords = kSegCap / 32;  // words of a bitmap over a segment's products
 static_assert(kSegCap % 32 == 0 && kSegPWords <= 96, "p-bitmap prefix: three words per lane");
@@ -552,16 +552,18 @@ struct SegLayout {
     static_assert(o_bmp + NW * kSegPWords * 6 <= o_lleaf, "the bitmaps fit in the list table");
     static constexpr size_t o_pre = o_lleaf + mid_a16(kSegCap * 2);   // word prefixes, then runs
     static constexpr size_t o_cnt = o_pre + mid_a16(kSegCap * 2);     // products of each column,
-    static constexpr size_t o_list = o_cnt;                           // then lists by position
+    static constexpr size_t o_list = o_cnt;                           // then products by position
     static constexpr size_t o_ucol = o_cnt + mid_a16(kSegCap * 2);
-    // columns of two and of three or four products (from both ends), and of
-    // five to eight and more (the same)
+    // columns of two and of three or four products (from both ends), of five
+    // to eight and of nine to sixteen (the same), and of more
     static constexpr int n_a = kSegCap / 2, n_b = kSegCap / 5 + 2;
     static constexpr size_t o_lista = o_ucol + mid_a16(kSegCap * 4);
     static constexpr size_t o_listb = o_lista + mid_a16(n_a * 2);
-    static constexpr size_t o_llen = o_listb + mid_a16(n_b * 2);  // products of the long ones
+    static constexpr size_t o_listc = o_listb + mid_a16(n_b * 2);
+    static constexpr size_t o_llen = o_listc + mid_a16(kLongMax * 2);  // their products
     static constexpr size_t o_sb = o_llen + mid_a16(kLongMax * 2);
-    static constexpr size_t o_ws = o_sb + mid_a16(kSegPWords * 4);
+    static constexpr size_t o_sbp = o_sb + mid_a16(kSegPWords * 4);  // lists before each word of sb
+    static constexpr size_t o_ws = o_sbp + mid_a16(kSegPWords * 2);
     static constexpr size_t o_misc = o_ws + mid_a16((NW + 1) * 8);
     static constexpr size_t o_run = o_misc + 64;  // the next segment's record
     static constexpr size_t bytes = o_run + sizeof(SegRun);
@@ -628,8 +630,10 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
     int *ucol = (int *)(smem + L::o_ucol);
     unsigned short *lista = (unsigned short *)(smem + L::o_lista);
     unsigned short *listb = (unsigned short *)(smem + L::o_listb);
+    unsigned short *listc = (unsigned short *)(smem + L::o_listc);
     unsigned short *llen = (unsigned short *)(smem + L::o_llen);
     unsigned *sb = (unsigned *)(smem + L::o_sb);
+    unsigned short *sbp = (unsigned short *)(smem + L::o_sbp);
     long long *ws = (long long *)(smem + L::o_ws);
     int *wsi = (int *)(smem + L::o_ws);
     int *misc = (int *)(smem + L::o_misc);
@@ -641,6 +645,10 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
     const int *__restrict__ bcol = B.col;
     const T *__restrict__ bval = (const T *)B.val;
     const T *__restrict__ aval = (const T *)A.val;
+    // leaf of product e (numbered in list order)
+    auto leaf_of = [&](int e) -> int {
+        return lleaf[sbp[e >> 5] + __popc(sb[e >> 5] & ((2u << (e & 31)) - 1u)) - 1];
+    };
     // thread 0 takes the next work item one segment ahead and copies its
     // record into srun (cp.async) while the current segment runs, so a
     // segment starts without a chain of dependent global loads
@@ -657,6 +665,8 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         }
         if (tid < kSegPWords)
             sb[tid] = 0;
+        if (tid < 8)
+            misc[1 + tid] = 0;  // columns of each size, positions, an input error
         __syncthreads();
         const int item = misc[0];
         if (item >= nsegs)
@@ -689,12 +699,14 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 ((uint4 *)cnt2)[i] = make_uint4(0, 0, 0, 0);
         }
         // 1. nonempty sub-lists of the segment, in leaf order (a thread takes
-        //    four consecutive lists per pass: hub rows have thousands of lists
-        //    and few products of each in one segment), and a bit per list
-        //    start in product order
+        //    four consecutive lists per pass), and a bit per list start in
+        //    product order: by the first warp where the row has few lists, by
+        //    the block for hub rows (thousands of lists, few products of each
+        //    in one segment)
         constexpr int LPT = 4;
         int nlists = 0, nprod = 0;
-        for (int lb = 0; lb < k; lb += NT * LPT) {
+        const bool few = k <= 32 * LPT;
+        for (int lb = 0; lb < k && (!few || w == 0); lb += NT * LPT) {
             int st[LPT], len[LPT];
             int ne = 0, psum = 0;
 #pragma unroll
@@ -709,9 +721,15 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 ne += len[q] > 0;
                 psum += len[q];
             }
-            long long tot;
-            const long long ex = block_excl_scan<NT, long long>(
-                ((long long)ne << 32) | (long long)psum, ws, &tot);
+            const long long x = ((long long)ne << 32) | (long long)psum;
+            long long tot, ex;
+            if (few) {
+                ex = warp_incl_scan(x);
+                tot = __shfl_sync(kFull, ex, 31);
+                ex -= x;
+            } else {
+                ex = block_excl_scan<NT, long long>(x, ws, &tot);
+            }
             int li = nlists + (int)(ex >> 32);
             int po = nprod + (int)(ex & 0xffffffffLL);
 #pragma unroll
@@ -729,6 +747,15 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
             nlists += (int)(tot >> 32);
             nprod += (int)(tot & 0xffffffffLL);
         }
+        if (few && tid == 0) {
+            misc[9] = nlists;
+            misc[10] = nprod;
+        }
+        __syncthreads();
+        if (few) {
+            nlists = misc[9];
+            nprod = misc[10];
+        }
         if (nprod > kSegCap || nprod != d.nprod || nsum > kSumWords || span <= 0 || nprod == 0) {
             // (the columns before a chunk's first cut may hold no product)
             if (tid == 0 && !(nprod == 0 && d.nprod == 0 && next_u == d.u_off))
@@ -736,9 +763,6 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
             __syncthreads();
             continue;
         }
-        if (tid < 8)
-            misc[1 + tid] = 0;  // columns of each size, positions, an input error
-        __syncthreads();
         // 2. this warp's words of 32 products, [w0, w0 + nw): columns into
         //    registers, their bits into the bitmap or the summary.  Lanes
         //    beyond the last product take no part from the counting on
@@ -761,6 +785,8 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 const int e = min((w0 + u) * 32 + lane, nprod - 1);
                 const unsigned bits = sb[w0 + u];
                 const int j = jb + __popc(bits & lem);
+                if (lane == 0)
+                    sbp[w0 + u] = (unsigned short)(jb + 1);
                 jb += __popc(bits);
                 pk[u] = (unsigned)j << 17;
                 const int bi = lofs[j] + e;
@@ -786,14 +812,14 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
             }
         }
         if (bad)
-            misc[6] = 1;
+            misc[7] = 1;
         __syncthreads();
         // every thread has read this segment's record: copy the next one
         if (tid == 0 && pf < nsegs) {
             copy_seg_run(srun, P.run + pf);
             pf_copied = true;
         }
-        if (misc[6]) {  // the plan does not match the input
+        if (misc[7]) {  // the plan does not match the input
             if (tid == 0)
                 atomicOr(&P.cnt->err, kErrBadInput);
             __syncthreads();
@@ -849,51 +875,31 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         // 5. columns of several products: positions for the second and further
         //    ones (column u's i-th at run[u] + i, its first at u), lists by size
         if (!nodup) {
-            for (int ib = w * 32; ib < U; ib += NT) {
-                const int u = ib + lane;
-                const int n = u < U ? cnt[u] : 0;
-                const unsigned mb = __ballot_sync(kFull, n > 1);
-                if (!mb)
+            for (int u = tid; u < U; u += NT) {
+                const int n = cnt[u];
+                if (n == 1)
                     continue;
-                const int x = n > 1 ? n - 1 : 0;
-                const int inc = warp_incl_scan(x);
-                int at = 0;
-                if (lane == 31)
-                    at = atomicAdd(&misc[5], inc);
-                at = __shfl_sync(kFull, at, 31) + inc - x;
-                // one list position a column: a warp's columns of one size together
-                const int cls = n == 2 ? 0 : n <= 4 ? 1 : n <= 8 ? 2 : 3;
-                unsigned left = mb;
-                int o = 0;
-                while (left) {
-                    const int k0 = __shfl_sync(kFull, cls, __ffs(left) - 1);
-                    const unsigned same = __ballot_sync(kFull, n > 1 && cls == k0);
-                    int first = 0;
-                    if (lane == 0)
-                        first = atomicAdd(&misc[1 + k0], __popc(same));
-                    first = __shfl_sync(kFull, first, 0);
-                    if (cls == k0)
-                        o = first + __popc(same & ltm);
-                    left &= ~same;
-                }
-                if (n > 1) {
-                    run[u] = (unsigned short)(U - 1 + at);
-                    // (the size beside the column's 12 bits)
-                    if (cls == 0)
-                        lista[o] = (unsigned short)u;
-                    else if (cls == 1)
-                        lista[L::n_a - 1 - o] = (unsigned short)(u | ((n - 3) << 12));
-                    else if (cls == 2)
-                        listb[o] = (unsigned short)(u | ((n - 5) << 12));
-                    else {
-                        listb[L::n_b - 1 - o] = (unsigned short)u;
-                        llen[o] = (unsigned short)n;
-                    }
+                run[u] = (unsigned short)(U - 1 + atomicAdd(&misc[6], n - 1));
+                const int cls = n == 2 ? 0 : n <= 4 ? 1 : n <= 8 ? 2 : n <= 16 ? 3 : 4;
+                const int o = atomicAdd(&misc[1 + cls], 1);
+                // (the size beside the column's 12 bits)
+                if (cls == 0) {
+                    lista[o] = (unsigned short)u;
+                } else if (cls == 1) {
+                    lista[L::n_a - 1 - o] = (unsigned short)(u | ((n - 3) << 12));
+                } else if (cls == 2) {
+                    listb[o] = (unsigned short)(u | ((n - 5) << 12));
+                } else if (cls == 3) {
+                    listb[L::n_b - 1 - o] = (unsigned short)(u | ((n - 9) << 12));
+                } else if (o < kLongMax) {
+                    listc[o] = (unsigned short)u;
+                    llen[o] = (unsigned short)n;
                 }
             }
             __syncthreads();
         }
-        const int n2 = misc[1], n34 = misc[2], n58 = misc[3], nlong = misc[4];
+        const int n2 = misc[1], n34 = misc[2], n58 = misc[3], n16 = misc[4];
+        const int nlong = min(misc[5], kLongMax);
         // 6. values to their positions
         {
             constexpr int VB = 4;  // gathers in flight a lane
@@ -922,7 +928,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                             if (c[u])
                                 p = run[p] + c[u];
                             vals[p] = vmul(av[q], bv[q]);
-                            plist[p] = (unsigned short)(pk[u] >> 12);
+                            plist[p] = (unsigned short)((w0 + u) * 32 + lane);
                         }
                     }
                 }
@@ -930,22 +936,58 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         }
         __syncthreads();
         // 7. columns of several products, each size by its own loop so that
-        //    the lanes of a warp run the same code; the value to position u
+        //    the lanes of a warp run the same code (and starting at another
+        //    warp: most sizes fill a few); the value to position u
         if (!nodup) {
+            const int hl = lane & 15, hb = lane & 16;
+            for (int ib = 2 * w; ib < n16; ib += 2 * NW) {
+                // half a warp each: leaf order by counting, then the trie
+                const int i = ib + (hb >> 4);
+                int u = 0, n = 0, x = 0, l = INT_MAX, r = 0;
+                T v = T(0);
+                if (i < n16) {
+                    const int y = listb[L::n_b - 1 - i];
+                    u = y & 0xfff;
+                    n = 9 + (y >> 12);
+                    x = hl ? run[u] + hl : u;
+                    if (hl < n) {
+                        l = plist[x];
+                        v = vals[x];
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; j++)
+                    r += __shfl_sync(kFull, l, hb | j) < l;
+                __syncwarp();
+                if (hl < n) {
+                    const int y = r ? run[u] + r : u;
+                    plist[y] = (unsigned short)l;
+                    vals[y] = v;
+                }
+                __syncwarp();
+                int lf = 0;
+                if (hl < n) {
+                    lf = leaf_of(plist[x]);
+                    v = vals[x];
+                }
+                v = half_trie<T>(lf, v, n);
+                if (hl == 0 && n)
+                    vals[u] = v;
+            }
             for (int i = tid; i < n2; i += NT) {
                 const int u = lista[i];
                 vals[u] = vadd(vals[u], vals[run[u] + 1]);
             }
-            for (int i = tid; i < n34; i += NT) {
+            for (int i = (NW - 1 - w) * 32 + lane; i < n34; i += NT) {
                 const int x = lista[L::n_a - 1 - i], u = x & 0xfff, p = run[u];
-                // sort the (list, value) pairs in registers, then the closed form
+                // sort the (product, value) pairs in registers, then the closed form
                 int l0 = plist[u], l1 = plist[p + 1], l2 = plist[p + 2];
                 T v0 = vals[u], v1 = vals[p + 1], v2 = vals[p + 2];
                 if (!(x >> 12)) {
                     leaf_cas(l0, v0, l1, v1);
                     leaf_cas(l1, v1, l2, v2);
                     leaf_cas(l0, v0, l1, v1);
-                    vals[u] = trie3<T>(lleaf[l0], lleaf[l1], lleaf[l2], v0, v1, v2);
+                    vals[u] = trie3<T>(leaf_of(l0), leaf_of(l1), leaf_of(l2), v0, v1, v2);
                 } else {
                     int l3 = plist[p + 3];
                     T v3 = vals[p + 3];
@@ -954,10 +996,11 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     leaf_cas(l0, v0, l2, v2);
                     leaf_cas(l1, v1, l3, v3);
                     leaf_cas(l1, v1, l2, v2);
-                    vals[u] = trie4<T>(lleaf[l0], lleaf[l1], lleaf[l2], lleaf[l3], v0, v1, v2, v3);
+                    vals[u] = trie4<T>(leaf_of(l0), leaf_of(l1), leaf_of(l2), leaf_of(l3), v0, v1,
+                                       v2, v3);
                 }
             }
-            for (int i = tid; i < n58; i += NT) {
+            for (int i = ((w + NW / 2) % NW) * 32 + lane; i < n58; i += NT) {
                 const int y = listb[i], u = y & 0xfff, p = run[u], len = 5 + (y >> 12);
                 // sorting network and a register stack
                 int l8[8];
@@ -974,17 +1017,17 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 }
                 leaf_sort8(l8, v8);
                 RegShiftReduce<T, 8> sr;
-                sr.init(lleaf[l8[0]], v8[0]);
+                sr.init(leaf_of(l8[0]), v8[0]);
 #pragma unroll
                 for (int j = 1; j < 8; j++)
                     if (j < len)
-                        sr.push(lleaf[l8[j]], v8[j]);
+                        sr.push(leaf_of(l8[j]), v8[j]);
                 vals[u] = sr.finish();
             }
         }
-        // columns with more than eight products: one warp each puts them in
-        // list order with a bitmap over the lists and hands them to the column
-        // reducer through the long-column scratch; when the scratch is full
+        // columns with more than sixteen products: one warp each puts them in
+        // leaf order (up to 32 by counting, more with a bitmap over the
+        // products) and hands them to the column reducer through the long-column scratch; when the scratch is full
         // it reduces them itself (across its lanes up to 32 products, in its
         // first lane beyond)
         const long long obase = (UPPER ? P.scan_flop[row] : (long long)crpt[row]) + d.u_off;
@@ -992,7 +1035,6 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
             unsigned *bmp = (unsigned *)(smem + L::o_bmp) + w * kSegPWords;
             unsigned short *wpre =
                 (unsigned short *)((unsigned *)(smem + L::o_bmp) + NW * kSegPWords) + w * kSegPWords;
-            const int nwl = (nlists + 31) >> 5;
             T *lval = (T *)P.long_val;
             for (int lb = w; lb < nlong; lb += 32 * NW) {
                 // the warp's next (up to) 32 columns lb + j * NW: one
@@ -1000,7 +1042,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 const int lj = lb + lane * NW;
                 int lu = 0, ln = 0;
                 if (lj < nlong) {
-                    lu = listb[L::n_b - 1 - lj];
+                    lu = listc[lj];
                     ln = llen[lj];
                 }
                 const int ncol = __popc(__ballot_sync(kFull, lj < nlong));
@@ -1020,34 +1062,44 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     const long long leo =
                         (long long)relem + __shfl_sync(kFull, lincl - ln, jc);
                     const bool handoff = lci < P.long_cap_cols && leo + len <= P.long_cap_elems;
-                    for (int x = lane; x < nwl; x += 32)
-                        bmp[x] = 0;
-                    __syncwarp();
-                    for (int i = lane; i < len; i += 32) {
-                        const int l = plist[i ? rp + i : u];
-                        atomicOr(&bmp[l >> 5], 1u << (l & 31));
-                    }
-                    __syncwarp();
-                    {
+                    if (len > 32) {
+                        for (int x = lane; x < nwd; x += 32)
+                            bmp[x] = 0;
+                        __syncwarp();
+                        for (int i = lane; i < len; i += 32) {
+                            const int l = plist[i ? rp + i : u];
+                            atomicOr(&bmp[l >> 5], 1u << (l & 31));
+                        }
+                        __syncwarp();
                         const int x0 = lane * 3;
-                        const int c0 = x0 < nwl ? __popc(bmp[x0]) : 0;
-                        const int c1 = x0 + 1 < nwl ? __popc(bmp[x0 + 1]) : 0;
-                        const int c2 = x0 + 2 < nwl ? __popc(bmp[x0 + 2]) : 0;
+                        const int c0 = x0 < nwd ? __popc(bmp[x0]) : 0;
+                        const int c1 = x0 + 1 < nwd ? __popc(bmp[x0 + 1]) : 0;
+                        const int c2 = x0 + 2 < nwd ? __popc(bmp[x0 + 2]) : 0;
                         const int ex = warp_incl_scan(c0 + c1 + c2) - (c0 + c1 + c2);
-                        if (x0 < nwl)
+                        if (x0 < nwd)
                             wpre[x0] = (unsigned short)ex;
-                        if (x0 + 1 < nwl)
+                        if (x0 + 1 < nwd)
                             wpre[x0 + 1] = (unsigned short)(ex + c0);
-                        if (x0 + 2 < nwl)
+                        if (x0 + 2 < nwd)
                             wpre[x0 + 2] = (unsigned short)(ex + c0 + c1);
+                        __syncwarp();
                     }
-                    __syncwarp();
+                    int turn = 0;  // up to 32 products: those before the lane's
+                    if (len <= 32) {
+                        const int l =
+                            lane < len ? (int)plist[lane ? rp + lane : u] : INT_MAX;
+                        for (int j = 0; j < len; j++)
+                            turn += __shfl_sync(kFull, l, j) < l;
+                    }
                     for (int i = lane; i < len; i += 32) {
                         const int x = i ? rp + i : u;
                         const int l = plist[x];
-                        const int r = wpre[l >> 5] + __popc(bmp[l >> 5] & ((1u << (l & 31)) - 1u));
+                        const int r =
+                            len <= 32 ? turn
+                                      : wpre[l >> 5] +
+                                            __popc(bmp[l >> 5] & ((1u << (l & 31)) - 1u));
                         if (handoff) {
-                            P.long_leaf[leo + r] = lleaf[l];
+                            P.long_leaf[leo + r] = (unsigned short)leaf_of(l);
                             lval[leo + r] = vals[x];
                         } else {
                             ord[r ? rp + r : u] = (unsigned short)x;
@@ -1066,15 +1118,15 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                         continue;
                     if (len <= 32) {
                         const int x = ord[lane > 0 && lane < len ? rp + lane : u];
-                        const T r = warp_trie<T>(lleaf[plist[x]], vals[x], len);
+                        const T r = warp_trie<T>(leaf_of(plist[x]), vals[x], len);
                         __syncwarp();
                         if (lane == 0)
                             vals[u] = r;
                     } else if (lane == 0) {
                         ShiftReduce<T, 17> sr;
-                        sr.init(lleaf[plist[ord[u]]], vals[ord[u]]);
+                        sr.init(leaf_of(plist[ord[u]]), vals[ord[u]]);
                         for (int i = 1; i < len; i++)
-                            sr.push(lleaf[plist[ord[rp + i]]], vals[ord[rp + i]]);
+                            sr.push(leaf_of(plist[ord[rp + i]]), vals[ord[rp + i]]);
                         vals[u] = sr.finish();
                     }
                     __syncwarp();
