@@ -243,32 +243,6 @@ __device__ __forceinline__ void leaf_cas(int &la, T &va, int &lb, T &vb)
     }
 }
 
-// Sorts eight (leaf, value) pairs by leaf in registers (Batcher's odd-even
-// merge network, 19 comparators).
-template <typename T>
-__device__ __forceinline__ void leaf_sort8(int (&l)[8], T (&v)[8])
-{
-    leaf_cas(l[0], v[0], l[1], v[1]);
-    leaf_cas(l[2], v[2], l[3], v[3]);
-    leaf_cas(l[4], v[4], l[5], v[5]);
-    leaf_cas(l[6], v[6], l[7], v[7]);
-    leaf_cas(l[0], v[0], l[2], v[2]);
-    leaf_cas(l[1], v[1], l[3], v[3]);
-    leaf_cas(l[4], v[4], l[6], v[6]);
-    leaf_cas(l[5], v[5], l[7], v[7]);
-    leaf_cas(l[1], v[1], l[2], v[2]);
-    leaf_cas(l[5], v[5], l[6], v[6]);
-    leaf_cas(l[0], v[0], l[4], v[4]);
-    leaf_cas(l[1], v[1], l[5], v[5]);
-    leaf_cas(l[2], v[2], l[6], v[6]);
-    leaf_cas(l[3], v[3], l[7], v[7]);
-    leaf_cas(l[2], v[2], l[4], v[4]);
-    leaf_cas(l[3], v[3], l[5], v[5]);
-    leaf_cas(l[1], v[1], l[2], v[2]);
-    leaf_cas(l[3], v[3], l[4], v[4]);
-    leaf_cas(l[5], v[5], l[6], v[6]);
-}
-
 // ShiftReduce with its stack in registers for at most D leaves: the entry
 // below the top is always st[0], so every access uses a fixed index (a push
 // shifts the stack down, a reduction shifts it up).
@@ -351,26 +325,27 @@ __device__ __forceinline__ T warp_trie(int leaf, T v, int n)
     return v;
 }
 
-// The same for two columns at once, one per half warp (lane 16 h + j < 16 h + n
-// holds the j-th smallest of the n <= 16 leaves of half h's column); results in
-// lanes 0 and 16.  A round joins every adjacent pair whose split level is
+// The same for 32 / W columns at once, W lanes each (lane j < n of a group
+// holds the j-th smallest of the n <= W leaves of its column); results in the
+// groups' first lanes.  A round joins every adjacent pair whose split level is
 // below its neighbours' (such pairs are siblings too), in as many rounds as
 // the tree is deep or fewer.  Adjacent splits differ unless leaves are equal
 // (a list that repeats a column): then the last pair of the equal ones joins,
 // so every round joins some pair.
-template <typename T>
-__device__ __forceinline__ T half_trie(int leaf, T v, int n)
+template <typename T, int W>
+__device__ __forceinline__ T group_trie(int leaf, T v, int n)
 {
-    const int lane = threadIdx.x & 31, hl = lane & 15, hb = lane & 16;
-    bool alive = hl < n;
+    const int lane = threadIdx.x & 31, gl = lane & (W - 1), gb = lane & ~(W - 1);
+    constexpr unsigned gm = W == 32 ? kFull : (1u << (W & 31)) - 1u;
+    bool alive = gl < n;
     for (;;) {
-        const unsigned am = (__ballot_sync(kFull, alive) >> hb) & 0xffffu;
+        const unsigned am = (__ballot_sync(kFull, alive) >> gb) & gm;
         if (!__any_sync(kFull, (am & (am - 1u)) != 0u))
             break;
-        const unsigned after = am & ~((2u << hl) - 1u), before = am & ((1u << hl) - 1u);
+        const unsigned after = am & ~((2u << gl) - 1u), before = am & ((1u << gl) - 1u);
         const bool has = alive && after != 0u;
-        const int nl = has ? __ffs(after) - 1 + hb : lane;
-        const int pl = before ? 31 - __clz(before) + hb : lane;
+        const int nl = has ? __ffs(after) - 1 + gb : lane;
+        const int pl = before ? 31 - __clz(before) + gb : lane;
         const int kn = __shfl_sync(kFull, leaf, nl);
         const T vn = __shfl_sync(kFull, v, nl);
         const int s = has ? split_level(leaf, kn) : 64;

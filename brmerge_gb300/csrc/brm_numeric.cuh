@@ -31,9 +31,8 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
     // The warp and mid rows computed with the plan (one-call Precise) are moved
     // into C by a bandwidth-bound copy.  With heavy-row segments it waits for
     // the segment kernel (which holds every SM's registers) and runs beside
-    // the latency-bound column reducers that follow it (R-MAT n=2^18 one-call
-    // Precise 2.875 -> 2.838 ms; the two reducers on separate streams as
-    // well: 2.917 ms).  A numeric phase run in row parts (the host drop-in
+    // the latency-bound column reducer that follows it (R-MAT n=2^18 one-call
+    // Precise 2.875 -> 2.838 ms when it came in).  A numeric phase run in row parts (the host drop-in
     // copies each part back while the next computes) keeps it first.  Without
     // segments it does the copy rows too, in one launch.
     // (kernels of row classes without rows are not launched)
@@ -104,8 +103,6 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
             count_launch();
             cudaEventRecord(fk.join, fk.aux);
         }
-        k_long_reduce<T><<<num_sms * 4, 128, 0, s>>>(P, ccol, cval);
-        count_launch();
         k_long_warp<T><<<num_sms * 4, 128, 0, s>>>(P, ccol, cval);
         count_launch();
     }

@@ -20,18 +20,27 @@
 //   2. split table (numeric phase): for every segment boundary and every list
 //      of the row, the first list position at or after the boundary column
 //      (one block per boundary, one binary search per list).
-//   3. segment kernel (numeric phase, one CTA pass per segment): stage the
-//      segment's products in list-major order; the rank u of every product's
-//      column among the segment's distinct columns comes from a two-level
-//      bitmap (a summary bit per nonempty 32-column word, then the compressed
-//      words); a counting sort on u groups each column's contributions; one
-//      thread per output column puts up to eight of them in leaf order in
-//      registers and evaluates the merge tree (closed forms for three and
-//      four, a register ShiftReduce up to eight); longer columns are ranked
-//      by leaf by a warp and handed to the column reducer (step 4).  Column u
-//      is stored at position u of the row's segment (coalesced).
-//   4. column reducer: one thread per long column, ShiftReduce with the
-//      stack in registers over the leaf-ordered products.
+//   3. segment kernel (numeric phase, one CTA pass per segment): the
+//      segment's columns into registers in list-major order; the rank u of
+//      every product's column among the segment's distinct columns comes from
+//      a bitmap (of all columns, or a summary bit per nonempty 32-column word
+//      and the compressed words); a shared counter a column gives a product
+//      its turn, its first one position u and the others a run of positions
+//      behind the columns, so columns of one product are done when their
+//      value is placed.  The others are listed by size: two products by a
+//      lane, three or four by a lane in registers (closed forms), up to 8, 16
+//      and 32 by that many lanes (leaf order by counting, then the tree),
+//      more are put in leaf order by a warp and handed to the column reducer
+//      (step 4).  Column u is stored at position u of the row's segment
+//      (coalesced).
+//   4. column reducer: one warp per long column.
+//
+// What bounds the segment kernel: latency and issue (three CTAs of eight warps
+// an SM, about half of the issue slots).  R-MAT n=2^18, 4.1e7 products in
+// 17.9 k segments: 1147 us when every product's column, value, leaf, rank and
+// turn were staged in shared memory (111 KB, two CTAs an SM), 915 with the
+// columns in registers, 746 with columns of up to 32 products reduced in
+// place by groups of lanes.
 #pragma once
 
 #include <climits>
@@ -516,7 +525,7 @@ __global__ void __launch_bounds__(256) k_split(CsrDev A, CsrDev B, PlanDev P)
 // ---------------------------------------------------------------------------
 // 3. segment kernel
 // ---------------------------------------------------------------------------
-constexpr int kLongMin = 17;  // columns with this many products are handed to the column reducers
+constexpr int kLongMin = 33;  // columns with this many products are handed to the column reducer
 constexpr int kLongMax = kSegCap / kLongMin + 1;
 constexpr int kSegPWords = kSegCap / 32;  // words of a bitmap over a segment's products
 static_assert(kSegCap % 32 == 0 && kSegPWords <= 96, "p-bitmap prefix: three words per lane");
@@ -527,6 +536,54 @@ __device__ __forceinline__ void copy_seg_run(SegRun *dst, const SegRun *src)
 #pragma unroll
     for (int q = 0; q < 3; q++)
         cp_async16((unsigned char *)dst + 16 * q, (const unsigned char *)src + 16 * q);
+}
+
+// n columns of at most W products, W lanes each, warp w of the block's; entry(i)
+// is a column (12 bits) and its products less `least`.  Leaf order by counting
+// (products are numbered in list order), then the merge tree; the value to
+// the column's first position.
+template <typename T, int W, typename LeafOf, typename Entry>
+__device__ __forceinline__ void seg_columns(int n, int w, T *vals, unsigned short *plist,
+                                            const unsigned short *run, const LeafOf &leaf_of,
+                                            const Entry &entry, int least)
+{
+    constexpr int PER = 32 / W;
+    const int lane = threadIdx.x & 31, gl = lane & (W - 1), gb = lane & ~(W - 1);
+    for (int ib = PER * w; ib < n; ib += PER * (kSegThreads / 32)) {
+        const int i = ib + gb / W;
+        int u = 0, p = 0, len = 0, x = 0, e = INT_MAX, r = 0;
+        T v = T(0);
+        if (i < n) {
+            const int y = entry(i);
+            u = y & 0xfff;
+            len = least + (y >> 12);
+            p = run[u];
+            x = gl ? p + gl : u;
+            if (gl < len) {
+                e = plist[x];
+                v = vals[x];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < W; j++)
+            r += __shfl_sync(kFull, e, gb | j) < e;
+        __syncwarp();
+        if (gl < len) {
+            const int y = r ? p + r : u;
+            plist[y] = (unsigned short)e;
+            vals[y] = v;
+        }
+        __syncwarp();
+        int lf = 0;
+        if (gl < len) {
+            lf = leaf_of(plist[x]);
+            v = vals[x];
+        }
+        v = group_trie<T, W>(lf, v, len);
+        if (gl == 0 && len)
+            vals[u] = v;
+        __syncwarp();
+    }
 }
 
 constexpr int kSegNP = kSegCap / kSegThreads;  // products a lane
@@ -555,12 +612,12 @@ struct SegLayout {
     static constexpr size_t o_list = o_cnt;                           // then products by position
     static constexpr size_t o_ucol = o_cnt + mid_a16(kSegCap * 2);
     // columns of two and of three or four products (from both ends), of five
-    // to eight and of nine to sixteen (the same), and of more
-    static constexpr int n_a = kSegCap / 2, n_b = kSegCap / 5 + 2;
+    // to eight and of nine to sixteen (the same), of up to 32 and of more
+    static constexpr int n_a = kSegCap / 2, n_b = kSegCap / 5 + 2, n_c = kSegCap / 17 + 2;
     static constexpr size_t o_lista = o_ucol + mid_a16(kSegCap * 4);
     static constexpr size_t o_listb = o_lista + mid_a16(n_a * 2);
     static constexpr size_t o_listc = o_listb + mid_a16(n_b * 2);
-    static constexpr size_t o_llen = o_listc + mid_a16(kLongMax * 2);  // their products
+    static constexpr size_t o_llen = o_listc + mid_a16(n_c * 2);  // products of the long ones
     static constexpr size_t o_sb = o_llen + mid_a16(kLongMax * 2);
     static constexpr size_t o_sbp = o_sb + mid_a16(kSegPWords * 4);  // lists before each word of sb
     static constexpr size_t o_ws = o_sbp + mid_a16(kSegPWords * 2);
@@ -812,14 +869,14 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
             }
         }
         if (bad)
-            misc[7] = 1;
+            misc[8] = 1;
         __syncthreads();
         // every thread has read this segment's record: copy the next one
         if (tid == 0 && pf < nsegs) {
             copy_seg_run(srun, P.run + pf);
             pf_copied = true;
         }
-        if (misc[7]) {  // the plan does not match the input
+        if (misc[8]) {  // the plan does not match the input
             if (tid == 0)
                 atomicOr(&P.cnt->err, kErrBadInput);
             __syncthreads();
@@ -879,8 +936,8 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 const int n = cnt[u];
                 if (n == 1)
                     continue;
-                run[u] = (unsigned short)(U - 1 + atomicAdd(&misc[6], n - 1));
-                const int cls = n == 2 ? 0 : n <= 4 ? 1 : n <= 8 ? 2 : n <= 16 ? 3 : 4;
+                run[u] = (unsigned short)(U - 1 + atomicAdd(&misc[7], n - 1));
+                const int cls = n == 2 ? 0 : n <= 4 ? 1 : n <= 8 ? 2 : n <= 16 ? 3 : n < kLongMin ? 4 : 5;
                 const int o = atomicAdd(&misc[1 + cls], 1);
                 // (the size beside the column's 12 bits)
                 if (cls == 0) {
@@ -891,15 +948,17 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     listb[o] = (unsigned short)(u | ((n - 5) << 12));
                 } else if (cls == 3) {
                     listb[L::n_b - 1 - o] = (unsigned short)(u | ((n - 9) << 12));
+                } else if (cls == 4) {
+                    listc[o] = (unsigned short)(u | ((n - 17) << 12));
                 } else if (o < kLongMax) {
-                    listc[o] = (unsigned short)u;
+                    listc[L::n_c - 1 - o] = (unsigned short)u;
                     llen[o] = (unsigned short)n;
                 }
             }
             __syncthreads();
         }
-        const int n2 = misc[1], n34 = misc[2], n58 = misc[3], n16 = misc[4];
-        const int nlong = min(misc[5], kLongMax);
+        const int n2 = misc[1], n34 = misc[2], n8 = misc[3], n16 = misc[4], n32 = misc[5];
+        const int nlong = min(misc[6], kLongMax);
         // 6. values to their positions
         {
             constexpr int VB = 4;  // gathers in flight a lane
@@ -937,43 +996,105 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         __syncthreads();
         // 7. columns of several products, each size by its own loop so that
         //    the lanes of a warp run the same code (and starting at another
-        //    warp: most sizes fill a few); the value to position u
-        if (!nodup) {
-            const int hl = lane & 15, hb = lane & 16;
-            for (int ib = 2 * w; ib < n16; ib += 2 * NW) {
-                // half a warp each: leaf order by counting, then the trie
-                const int i = ib + (hb >> 4);
-                int u = 0, n = 0, x = 0, l = INT_MAX, r = 0;
-                T v = T(0);
-                if (i < n16) {
-                    const int y = listb[L::n_b - 1 - i];
-                    u = y & 0xfff;
-                    n = 9 + (y >> 12);
-                    x = hl ? run[u] + hl : u;
-                    if (hl < n) {
-                        l = plist[x];
-                        v = vals[x];
+        //    warp: most sizes fill a few); the value to position u.
+        //    Columns with more than 32 products first: one warp each puts them
+        //    in leaf order with a bitmap over the products and hands them to
+        //    the column reducer through the long-column scratch; when the
+        //    scratch is full its first lane reduces them
+        const long long obase = (UPPER ? P.scan_flop[row] : (long long)crpt[row]) + d.u_off;
+        if (nlong > 0) {
+            unsigned *bmp = (unsigned *)(smem + L::o_bmp) + w * kSegPWords;
+            unsigned short *wpre =
+                (unsigned short *)((unsigned *)(smem + L::o_bmp) + NW * kSegPWords) + w * kSegPWords;
+            T *lval = (T *)P.long_val;
+            for (int lb = w; lb < nlong; lb += 32 * NW) {
+                // the warp's next (up to) 32 columns lb + j * NW: one
+                // reservation of long-column scratch covers all of them
+                const int lj = lb + lane * NW;
+                int lu = 0, ln = 0;
+                if (lj < nlong) {
+                    lu = listc[L::n_c - 1 - lj];
+                    ln = llen[lj];
+                }
+                const int ncol = __popc(__ballot_sync(kFull, lj < nlong));
+                const int lincl = warp_incl_scan(ln);
+                unsigned long long rcol = 0, relem = 0;
+                if (lane == 31) {
+                    rcol = atomicAdd(&P.cnt->long_cols, (unsigned long long)ncol);
+                    relem = atomicAdd(&P.cnt->long_elems, (unsigned long long)lincl);
+                }
+                rcol = __shfl_sync(kFull, rcol, 31);
+                relem = __shfl_sync(kFull, relem, 31);
+                for (int jc = 0; jc < ncol; jc++) {
+                    const int u = __shfl_sync(kFull, lu, jc);
+                    const int len = __shfl_sync(kFull, ln, jc);
+                    const int rp = run[u];
+                    const long long lci = (long long)rcol + jc;
+                    const long long leo =
+                        (long long)relem + __shfl_sync(kFull, lincl - ln, jc);
+                    const bool handoff = lci < P.long_cap_cols && leo + len <= P.long_cap_elems;
+                    for (int x = lane; x < nwd; x += 32)
+                        bmp[x] = 0;
+                    __syncwarp();
+                    for (int i = lane; i < len; i += 32) {
+                        const int l = plist[i ? rp + i : u];
+                        atomicOr(&bmp[l >> 5], 1u << (l & 31));
                     }
+                    __syncwarp();
+                    {
+                        const int x0 = lane * 3;
+                        const int c0 = x0 < nwd ? __popc(bmp[x0]) : 0;
+                        const int c1 = x0 + 1 < nwd ? __popc(bmp[x0 + 1]) : 0;
+                        const int c2 = x0 + 2 < nwd ? __popc(bmp[x0 + 2]) : 0;
+                        const int ex = warp_incl_scan(c0 + c1 + c2) - (c0 + c1 + c2);
+                        if (x0 < nwd)
+                            wpre[x0] = (unsigned short)ex;
+                        if (x0 + 1 < nwd)
+                            wpre[x0 + 1] = (unsigned short)(ex + c0);
+                        if (x0 + 2 < nwd)
+                            wpre[x0 + 2] = (unsigned short)(ex + c0 + c1);
+                    }
+                    __syncwarp();
+                    for (int i = lane; i < len; i += 32) {
+                        const int x = i ? rp + i : u;
+                        const int l = plist[x];
+                        const int r = wpre[l >> 5] + __popc(bmp[l >> 5] & ((1u << (l & 31)) - 1u));
+                        if (handoff) {
+                            P.long_leaf[leo + r] = (unsigned short)leaf_of(l);
+                            lval[leo + r] = vals[x];
+                        } else {
+                            ord[r ? rp + r : u] = (unsigned short)x;
+                        }
+                    }
+                    if (lci < P.long_cap_cols && lane == 0) {
+                        LongCol lc;
+                        lc.out = obase + u;
+                        lc.off = leo;
+                        lc.col = d.c_lo + ucol[u];
+                        lc.len = handoff ? len : -1;
+                        P.long_col[lci] = lc;
+                    }
+                    __syncwarp();
+                    if (handoff)
+                        continue;
+                    if (lane == 0) {
+                        ShiftReduce<T, 17> sr;
+                        sr.init(leaf_of(plist[ord[u]]), vals[ord[u]]);
+                        for (int i = 1; i < len; i++)
+                            sr.push(leaf_of(plist[ord[rp + i]]), vals[ord[rp + i]]);
+                        vals[u] = sr.finish();
+                    }
+                    __syncwarp();
                 }
-#pragma unroll
-                for (int j = 0; j < 16; j++)
-                    r += __shfl_sync(kFull, l, hb | j) < l;
-                __syncwarp();
-                if (hl < n) {
-                    const int y = r ? run[u] + r : u;
-                    plist[y] = (unsigned short)l;
-                    vals[y] = v;
-                }
-                __syncwarp();
-                int lf = 0;
-                if (hl < n) {
-                    lf = leaf_of(plist[x]);
-                    v = vals[x];
-                }
-                v = half_trie<T>(lf, v, n);
-                if (hl == 0 && n)
-                    vals[u] = v;
             }
+        }
+        if (!nodup) {
+            seg_columns<T, 32>(n32, w, vals, plist, run, leaf_of,
+                               [&](int i) { return listc[i]; }, 17);
+            seg_columns<T, 16>(n16, (w + 5) % NW, vals, plist, run, leaf_of,
+                               [&](int i) { return listb[L::n_b - 1 - i]; }, 9);
+            seg_columns<T, 8>(n8, (w + 3) % NW, vals, plist, run, leaf_of,
+                              [&](int i) { return listb[i]; }, 5);
             for (int i = tid; i < n2; i += NT) {
                 const int u = lista[i];
                 vals[u] = vadd(vals[u], vals[run[u] + 1]);
@@ -1000,138 +1121,6 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                                        v2, v3);
                 }
             }
-            for (int i = ((w + NW / 2) % NW) * 32 + lane; i < n58; i += NT) {
-                const int y = listb[i], u = y & 0xfff, p = run[u], len = 5 + (y >> 12);
-                // sorting network and a register stack
-                int l8[8];
-                T v8[8];
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    l8[j] = INT_MAX;
-                    v8[j] = T(0);
-                    if (j < len) {
-                        const int x = j ? p + j : u;
-                        l8[j] = plist[x];
-                        v8[j] = vals[x];
-                    }
-                }
-                leaf_sort8(l8, v8);
-                RegShiftReduce<T, 8> sr;
-                sr.init(leaf_of(l8[0]), v8[0]);
-#pragma unroll
-                for (int j = 1; j < 8; j++)
-                    if (j < len)
-                        sr.push(leaf_of(l8[j]), v8[j]);
-                vals[u] = sr.finish();
-            }
-        }
-        // columns with more than sixteen products: one warp each puts them in
-        // leaf order (up to 32 by counting, more with a bitmap over the
-        // products) and hands them to the column reducer through the long-column scratch; when the scratch is full
-        // it reduces them itself (across its lanes up to 32 products, in its
-        // first lane beyond)
-        const long long obase = (UPPER ? P.scan_flop[row] : (long long)crpt[row]) + d.u_off;
-        if (nlong > 0) {
-            unsigned *bmp = (unsigned *)(smem + L::o_bmp) + w * kSegPWords;
-            unsigned short *wpre =
-                (unsigned short *)((unsigned *)(smem + L::o_bmp) + NW * kSegPWords) + w * kSegPWords;
-            T *lval = (T *)P.long_val;
-            for (int lb = w; lb < nlong; lb += 32 * NW) {
-                // the warp's next (up to) 32 columns lb + j * NW: one
-                // reservation of long-column scratch covers all of them
-                const int lj = lb + lane * NW;
-                int lu = 0, ln = 0;
-                if (lj < nlong) {
-                    lu = listc[lj];
-                    ln = llen[lj];
-                }
-                const int ncol = __popc(__ballot_sync(kFull, lj < nlong));
-                const int lincl = warp_incl_scan(ln);
-                unsigned long long rcol = 0, relem = 0;
-                if (lane == 31) {
-                    rcol = atomicAdd(&P.cnt->long_cols, (unsigned long long)ncol);
-                    relem = atomicAdd(&P.cnt->long_elems, (unsigned long long)lincl);
-                }
-                rcol = __shfl_sync(kFull, rcol, 31);
-                relem = __shfl_sync(kFull, relem, 31);
-                for (int jc = 0; jc < ncol; jc++) {
-                    const int u = __shfl_sync(kFull, lu, jc);
-                    const int len = __shfl_sync(kFull, ln, jc);
-                    const int rp = run[u];
-                    const long long lci = (long long)rcol + jc;
-                    const long long leo =
-                        (long long)relem + __shfl_sync(kFull, lincl - ln, jc);
-                    const bool handoff = lci < P.long_cap_cols && leo + len <= P.long_cap_elems;
-                    if (len > 32) {
-                        for (int x = lane; x < nwd; x += 32)
-                            bmp[x] = 0;
-                        __syncwarp();
-                        for (int i = lane; i < len; i += 32) {
-                            const int l = plist[i ? rp + i : u];
-                            atomicOr(&bmp[l >> 5], 1u << (l & 31));
-                        }
-                        __syncwarp();
-                        const int x0 = lane * 3;
-                        const int c0 = x0 < nwd ? __popc(bmp[x0]) : 0;
-                        const int c1 = x0 + 1 < nwd ? __popc(bmp[x0 + 1]) : 0;
-                        const int c2 = x0 + 2 < nwd ? __popc(bmp[x0 + 2]) : 0;
-                        const int ex = warp_incl_scan(c0 + c1 + c2) - (c0 + c1 + c2);
-                        if (x0 < nwd)
-                            wpre[x0] = (unsigned short)ex;
-                        if (x0 + 1 < nwd)
-                            wpre[x0 + 1] = (unsigned short)(ex + c0);
-                        if (x0 + 2 < nwd)
-                            wpre[x0 + 2] = (unsigned short)(ex + c0 + c1);
-                        __syncwarp();
-                    }
-                    int turn = 0;  // up to 32 products: those before the lane's
-                    if (len <= 32) {
-                        const int l =
-                            lane < len ? (int)plist[lane ? rp + lane : u] : INT_MAX;
-                        for (int j = 0; j < len; j++)
-                            turn += __shfl_sync(kFull, l, j) < l;
-                    }
-                    for (int i = lane; i < len; i += 32) {
-                        const int x = i ? rp + i : u;
-                        const int l = plist[x];
-                        const int r =
-                            len <= 32 ? turn
-                                      : wpre[l >> 5] +
-                                            __popc(bmp[l >> 5] & ((1u << (l & 31)) - 1u));
-                        if (handoff) {
-                            P.long_leaf[leo + r] = (unsigned short)leaf_of(l);
-                            lval[leo + r] = vals[x];
-                        } else {
-                            ord[r ? rp + r : u] = (unsigned short)x;
-                        }
-                    }
-                    if (lci < P.long_cap_cols && lane == 0) {
-                        LongCol lc;
-                        lc.out = obase + u;
-                        lc.off = leo;
-                        lc.col = d.c_lo + ucol[u];
-                        lc.len = handoff ? len : -1;
-                        P.long_col[lci] = lc;
-                    }
-                    __syncwarp();
-                    if (handoff)
-                        continue;
-                    if (len <= 32) {
-                        const int x = ord[lane > 0 && lane < len ? rp + lane : u];
-                        const T r = warp_trie<T>(leaf_of(plist[x]), vals[x], len);
-                        __syncwarp();
-                        if (lane == 0)
-                            vals[u] = r;
-                    } else if (lane == 0) {
-                        ShiftReduce<T, 17> sr;
-                        sr.init(leaf_of(plist[ord[u]]), vals[ord[u]]);
-                        for (int i = 1; i < len; i++)
-                            sr.push(leaf_of(plist[ord[rp + i]]), vals[ord[rp + i]]);
-                        vals[u] = sr.finish();
-                    }
-                    __syncwarp();
-                }
-            }
         }
         __syncthreads();
         // 8. the segment's columns (the column reducer overwrites those handed
@@ -1147,10 +1136,8 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
 }
 
 // ---------------------------------------------------------------------------
-// 4. column reducer: one thread per long column handed over by the segment
-//    kernel; its products are in leaf order, so the trie is one ShiftReduce
-//    pass with the stack in registers (leaves below 2^16: at most 16 entries
-//    below the top).
+// 4. column reducer: one warp per long column handed over by the segment
+//    kernel; its products are in leaf order.
 // ---------------------------------------------------------------------------
 // Sequential trie of the elements [b, e) of a long column (leaves in
 // increasing order, below 2^(D-1)); the elements are loaded GB at a time, so
@@ -1178,9 +1165,6 @@ __device__ __forceinline__ T long_run(const unsigned short *__restrict__ lleaf,
     }
     return sr.finish();
 }
-
-constexpr int kLrWarpMin = 32;  // columns with more products are reduced by a whole warp
-                                // (and so are columns with leaves of 4096 or more)
 
 // A long column reduced by a whole warp.  Its leaves (strictly increasing,
 // below 2^bits) are cut into the 32 aligned ranges of 2^s leaves, s = bits - 5:
@@ -1223,46 +1207,6 @@ __device__ __forceinline__ T warp_long_column(const unsigned short *__restrict__
     return __shfl_sync(kFull, warp_trie<T>(li, vi, nh), 0);  // the trie's value is in lane 0
 }
 
-// Columns of at most kLrWarpMin products with leaves below 4096 are reduced
-// one per thread (k_long_reduce), the others by whole warps (k_long_warp):
-// two kernels, so that neither pays the other's registers.
-__device__ __forceinline__ bool long_by_thread(const LongCol &c, int last)
-{
-    return c.len <= kLrWarpMin && last < 4096;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(128) k_long_reduce(PlanDev P, int *ccol, T *cval)
-{
-    if (P.cnt->abort)  // a capacity check of a captured pipeline failed
-        return;
-    const long long n = min((long long)P.cnt->long_cols, P.long_cap_cols);
-    const T *__restrict__ lval = (const T *)P.long_val;
-    const unsigned short *__restrict__ lleaf = P.long_leaf;
-    for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n;
-         i0 += (long long)gridDim.x * blockDim.x) {
-        const long long i = i0 + threadIdx.x;
-        LongCol c;
-        c.len = 0;
-        if (i < n)
-            c = P.long_col[i];
-        if (c.len > 0 && !BRM_IN(P.cnt, c.off + c.len - 1, P.long_cap_elems))
-            c.len = 0;  // checked build: a record outside the scratch is skipped
-        const int last = c.len > 0 ? (int)lleaf[c.off + c.len - 1] : 0;
-        const bool mine = c.len > 0 && long_by_thread(c, last);
-        // the stack depth follows the warp's largest last leaf
-        const int top = __reduce_max_sync(kFull, mine ? last : 0);
-        if (mine) {
-            if (BRM_IN(P.cnt, c.out, P.c_cap) &&
-                BRM_IN(P.cnt, c.off + c.len - 1, P.long_cap_elems)) {
-                ccol[c.out] = c.col;
-                cval[c.out] = top < 256 ? long_run<T, 9>(lleaf, lval, c.off, c.off + c.len)
-                                    : long_run<T, 13, 4>(lleaf, lval, c.off, c.off + c.len);
-            }
-        }
-    }
-}
-
 template <typename T>
 __global__ void __launch_bounds__(128) k_long_warp(PlanDev P, int *ccol, T *cval)
 {
@@ -1274,30 +1218,17 @@ __global__ void __launch_bounds__(128) k_long_warp(PlanDev P, int *ccol, T *cval
     const long long n = min((long long)P.cnt->long_cols, P.long_cap_cols);
     const T *__restrict__ lval = (const T *)P.long_val;
     const unsigned short *__restrict__ lleaf = P.long_leaf;
-    for (long long i0 = (long long)blockIdx.x * blockDim.x; i0 < n;
-         i0 += (long long)gridDim.x * blockDim.x) {
-        const long long i = i0 + threadIdx.x;
-        LongCol c;
-        c.len = 0;
-        if (i < n)
-            c = P.long_col[i];
-        if (c.len > 0 && !BRM_IN(P.cnt, c.off + c.len - 1, P.long_cap_elems))
-            c.len = 0;  // checked build: a record outside the scratch is skipped
-        const int last = c.len > 0 ? (int)lleaf[c.off + c.len - 1] : 0;
-        unsigned lm = __ballot_sync(kFull, c.len > 0 && !long_by_thread(c, last));
-        while (lm) {
-            const int src = __ffs(lm) - 1;
-            lm &= lm - 1u;
-            const long long off = __shfl_sync(kFull, c.off, src);
-            const int len = __shfl_sync(kFull, c.len, src);
-            const T r = warp_long_column<T>(lleaf, lval, off, len, s_cnt[wid], s_val[wid]);
-            if (lane == src) {
-                if (BRM_IN(P.cnt, c.out, P.c_cap) &&
-                    BRM_IN(P.cnt, c.off + c.len - 1, P.long_cap_elems)) {
-                    ccol[c.out] = c.col;
-                    cval[c.out] = r;
-                }
-            }
+    for (long long i = (long long)blockIdx.x * 4 + wid; i < n; i += (long long)gridDim.x * 4) {
+        const LongCol c = P.long_col[i];
+        // (reduced by the segment kernel; checked build: a record outside the
+        // scratch or C is skipped)
+        if (c.len <= 0 || !BRM_IN(P.cnt, c.off + c.len - 1, P.long_cap_elems) ||
+            !BRM_IN(P.cnt, c.out, P.c_cap))
+            continue;
+        const T r = warp_long_column<T>(lleaf, lval, c.off, c.len, s_cnt[wid], s_val[wid]);
+        if (lane == 0) {
+            ccol[c.out] = c.col;
+            cval[c.out] = r;
         }
     }
 }

@@ -131,7 +131,7 @@ typedef struct brm_tuning {
     int seg_cut;
     int mid_flop;
     /* products the long-column scratch holds (columns of heavy-row segments
-     * with more than eight products, reduced by separate kernels); columns
+     * with more than 32 products, reduced by a separate kernel); columns
      * beyond it are reduced inside the segment kernel.  0: 16 Mi, the default;
      * otherwise 1 .. 2^31. */
     long long long_scratch;
