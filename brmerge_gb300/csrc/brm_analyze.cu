@@ -51,7 +51,7 @@ __device__ __forceinline__ T grp_min(T v, unsigned gm)
 
 // Rows of more than kAnaLongK entries are left, by groups of fewer than 32
 // lanes, to the block's whole warps (a second pass in the same launch).
-constexpr int kAnaLongK = 64;
+constexpr int kAnaLongK = 96;
 
 // What a block gathers of its rows before it takes places in the global lists.
 template <int RPB>
@@ -60,18 +60,19 @@ struct AnaBlock {
     int base[kNumBins];
     int bin[RPB];
     int idx[RPB];
-    unsigned long long off[RPB];   // place among the block's scratch entries
-    unsigned long long foff[RPB];  // place among the block's products
+    int flop[RPB];
     int longs[RPB];
     int nlong;
     int max_k;
-    unsigned long long mw, mid, flop, mw_base, flop_base;
+    unsigned long long mid;
+    unsigned long long tot[RPB / 32 + 1][2];  // products and scratch entries of 32 rows, then
+                                              // where they start among all rows'
 };
 
 // One row by a group of TW lanes (lane gl of it, mask gm): its products, list
-// table entries (P.abs, P.alen), class and column range.  LONG: eight entries
-// a lane in flight, and the first and last column of every list (the column
-// range) taken in the same pass, so their long lists are walked once.
+// table entries (P.abs, P.alen), class and column range.  LONG: the first and
+// last column of every list (the column range) are taken in the same pass, so
+// that long rows are walked once.
 template <int TW, bool LONG, int RPB>
 __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, const PlanDev &P,
                                             int row, int slot, int gl, unsigned gm,
@@ -87,7 +88,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
         bad = true;
         a0 = a1 = 0;
     }
-    constexpr int UN = LONG ? 8 : 4;
+    constexpr int UN = 4;
     int mn = INT_MAX, mx = -1;
     for (int jb = a0 + gl; jb < a1; jb += UN * TW) {
         int b[UN], bs[UN], be[UN];
@@ -168,7 +169,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
         bin = kBinHeavy;  // segmented (brm_seg.cuh)
     else
         bin = kBinMid;    // row CTA / spill path
-    if (bin == kBinHeavy || bin >= kBinMidWarp) {
+    if (bin >= kBinWarp && bin != kBinMid) {
         // column range of the row for the segment planning and the mid rows'
         // keys and bitmaps: the first and last column of every nonempty list
         for (int jb = a0 + gl; !LONG && jb < a1; jb += 4 * TW) {
@@ -221,7 +222,8 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
         P.seg_base[row] = atomicAdd(&P.cnt->seg_cap, seg_bound(f, B.N, P.seg_cut));
     const int weight = bin == kBinBatch ? max((int)f, 2 * nl) : 0;  // batch weight
     P.mid_flop[row] = weight;
-    P.spill[row] = 0;
+    if (bin == kBinHeavy || bin == kBinMid)
+        P.spill[row] = 0;
     if (bin == kBinEmpty)
         P.nnz[row] = 0;
     else if (bin == kBinCopy) {
@@ -238,9 +240,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
     }
     S.bin[slot] = bin;
     S.idx[slot] = bin < 0 || bin == kBinEmpty ? 0 : atomicAdd(&S.cnt[bin], 1);
-    S.foff[slot] = atomicAdd(&S.flop, (unsigned long long)f);
-    if (bin == kBinWarp || bin >= kBinMidWarp)
-        S.off[slot] = atomicAdd(&S.mw, (unsigned long long)f);
+    S.flop[slot] = (int)f;
     if (weight)
         atomicAdd(&S.mid, (unsigned long long)weight);
     atomicMax(&S.max_k, a1 - a0);
@@ -249,7 +249,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
 // A group of TW lanes per row (TW = 8 when rows are short, 32 otherwise),
 // kAnaRowsPerGroup rows per group.
 template <int TW>
-__global__ void __launch_bounds__(kAnaThreads) k_analyze(CsrDev A, CsrDev B, PlanDev P)
+__global__ void __launch_bounds__(kAnaThreads, 6) k_analyze(CsrDev A, CsrDev B, PlanDev P)
 {
     constexpr int NW = kAnaThreads / 32;
     constexpr int NGR = kAnaThreads / TW;  // groups per block
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kAnaThreads) k_analyze(CsrDev A, CsrDev B, Pla
         S.cnt[threadIdx.x] = 0;
     if (threadIdx.x == 0) {
         S.nlong = S.max_k = 0;
-        S.mw = S.mid = S.flop = 0;
+        S.mid = 0;
     }
     __syncthreads();
     const int M = A.M;
@@ -272,8 +272,10 @@ __global__ void __launch_bounds__(kAnaThreads) k_analyze(CsrDev A, CsrDev B, Pla
         const int slot = grp * kAnaRowsPerGroup + r;
         const int row = row0 + slot;
         if (row >= M) {
-            if (gl == 0)
+            if (gl == 0) {
                 S.bin[slot] = -1;
+                S.flop[slot] = 0;
+            }
             continue;
         }
         const int a0 = A.rpt[row], a1 = A.rpt[row + 1];
@@ -293,26 +295,50 @@ __global__ void __launch_bounds__(kAnaThreads) k_analyze(CsrDev A, CsrDev B, Pla
     if (threadIdx.x < kNumBins)
         S.base[threadIdx.x] =
             S.cnt[threadIdx.x] ? atomicAdd(&P.cnt->bin_count[threadIdx.x], S.cnt[threadIdx.x]) : 0;
+    // the rows' offsets: prefix over the block's slots (64-bit shared atomics
+    // a row took longer), one device atomic a total
+    const int slot = threadIdx.x;
+    unsigned long long fx = 0, sx = 0, fi = 0, si = 0;
+    if (slot < (RPB + 31) / 32 * 32) {
+        if (slot < RPB) {
+            const int bin = S.bin[slot];
+            fx = (unsigned long long)S.flop[slot];
+            sx = bin == kBinWarp || bin >= kBinMidWarp ? fx : 0ull;
+        }
+        fi = warp_incl_scan(fx);
+        si = warp_incl_scan(sx);
+        if (lane == 31) {
+            S.tot[w][0] = fi;
+            S.tot[w][1] = si;
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        unsigned long long t = 0;
+        for (int i = 0; i < (RPB + 31) / 32; i++)
+            t += S.tot[i][threadIdx.x];
+        unsigned long long b =
+            t ? atomicAdd(threadIdx.x ? &P.cnt->mw_total : &P.cnt->total_flop, t) : 0ull;
+        for (int i = 0; i < (RPB + 31) / 32; i++) {
+            const unsigned long long x = S.tot[i][threadIdx.x];
+            S.tot[i][threadIdx.x] = b;
+            b += x;
+        }
+    }
     if (threadIdx.x == 32) {
-        S.flop_base = S.flop ? atomicAdd(&P.cnt->total_flop, S.flop) : 0ull;
-        S.mw_base = S.mw ? atomicAdd(&P.cnt->mw_total, S.mw) : 0ull;
         if (S.mid)
             atomicAdd(&P.cnt->mid_total, S.mid);
         if (S.max_k > 0)
             atomicMax(&P.cnt->max_k, S.max_k);
     }
     __syncthreads();
-    for (int slot = threadIdx.x; slot < RPB; slot += kAnaThreads) {
+    if (slot < RPB && S.bin[slot] != -1) {
         const int bin = S.bin[slot], row = row0 + slot;
-        if (bin == -1)
-            continue;
         if (P.upper)
-            P.scan_flop[row] = (long long)(S.flop_base + S.foff[slot]);
-        if (bin <= kBinEmpty || bin == kBinBatch)
-            continue;
+            P.scan_flop[row] = (long long)(S.tot[w][0] + fi - fx);
         if (bin == kBinWarp || bin >= kBinMidWarp)
-            P.mw_pre[row] = (long long)(S.mw_base + S.off[slot]);
-        if (BRM_IN(P.cnt, S.base[bin] + S.idx[slot], M))
+            P.mw_pre[row] = (long long)(S.tot[w][1] + si - sx);
+        if (bin > kBinEmpty && bin != kBinBatch && BRM_IN(P.cnt, S.base[bin] + S.idx[slot], M))
             P.rows[(size_t)bin * M + S.base[bin] + S.idx[slot]] = row;
     }
 }
@@ -322,8 +348,10 @@ void launch_analyze(const CsrDev &A, const CsrDev &B, const PlanDev &P, cudaStre
     if (A.M <= 0)
         return;
     constexpr int RPB32 = (kAnaThreads / 32) * kAnaRowsPerGroup;
-    // eight lanes a row when rows average at most 12 entries
-    if ((long long)A.nnz <= 12ll * A.M) {
+    // eight lanes a row when rows average at most 32 entries (four loads a lane
+    // in flight then cover the row; the 27-point stencil on 128^3 by whole
+    // warps: 1.01 ms, by eighths 0.46)
+    if ((long long)A.nnz <= 32ll * A.M) {
         constexpr int RPB = (kAnaThreads / 8) * kAnaRowsPerGroup;
         k_analyze<8><<<(A.M + RPB - 1) / RPB, kAnaThreads, 0, s>>>(A, B, P);
     } else {

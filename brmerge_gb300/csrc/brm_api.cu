@@ -617,9 +617,10 @@ int numeric_launch(brm_context ctx, brm_dtype dtype, bool upper, const brm_csr *
         P.long_cap_elems = elems;
         static_assert(offsetof(brm::Counters, work_num) ==
                               offsetof(brm::Counters, err) + sizeof(int) &&
-                          offsetof(brm::Counters, long_elems) + sizeof(unsigned long long) -
-                                  offsetof(brm::Counters, err) ==
-                              4 * sizeof(int) + 2 * sizeof(unsigned long long),
+                          offsetof(brm::Counters, long_cols) - offsetof(brm::Counters, work_seg) <=
+                              sizeof(unsigned long long) &&
+                          offsetof(brm::Counters, long_elems) ==
+                              offsetof(brm::Counters, long_cols) + sizeof(unsigned long long),
                       "err and the counters of the numeric phase are cleared together");
     }
     brm::CsrDev a = to_dev(A), b = to_dev(B);

@@ -617,13 +617,21 @@ __global__ void __launch_bounds__(256) k_batch_starts(PlanDev P, int M)
 // Moves the rows written to the one-call scratch -- k_mid_numeric<..., SCRATCH>
 // (row at Counters::mw_total + P.mid_pre[row]), the warp, merge and rank
 // kernels (row at P.mw_pre[row]), P.nnz[row] entries each -- to C at crpt[row].
-// One warp per row.  COPY: the copy rows (one nonempty list, C row = a * B
-// row) in the same launch.
+// COPY: the copy rows (one nonempty list, C row = a * B row) in the same
+// launch.
+//
+// Bound by the copy itself (24 bytes an entry in float64) and, for short rows,
+// by the latency of the look-up before it, hence a warp a row and all 64 warps
+// an SM (32 registers).  Looking 32 rows up at once and copying them end to
+// end, or four rows in flight, took 64 registers and was no faster on 512
+// uneven pairs (2.0 M rows of 72 entries) and slower on R-MAT n=2^18 (0.18 ->
+// 0.25 ms).
 template <typename T, bool COPY>
-__global__ void __launch_bounds__(256) k_mid_compact(CsrDev A, CsrDev B, PlanDev P,
-                                                     const int *__restrict__ scol,
-                                                     const T *__restrict__ sval, const int *crpt,
-                                                     int *__restrict__ ccol, T *__restrict__ cval)
+__global__ void __launch_bounds__(256, 8) k_mid_compact(CsrDev A, CsrDev B, PlanDev P,
+                                                        const int *__restrict__ scol,
+                                                        const T *__restrict__ sval,
+                                                        const int *crpt, int *__restrict__ ccol,
+                                                        T *__restrict__ cval)
 {
     // a capacity check of a captured pipeline failed, or the plan did (row
     // lengths may then be missing)
@@ -634,73 +642,66 @@ __global__ void __launch_bounds__(256) k_mid_compact(CsrDev A, CsrDev B, PlanDev
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     const int M = A.M;
     const int r1 = min(M, P.r_hi);
-    // rows from their class lists, then (only when there are batches) the
-    // batched mid rows by a sweep over the rows
-    constexpr int B0 = COPY ? kBinCopy : kBinWarp;
-    auto listed = [](int b) { return b <= kBinWarp || b >= kBinMidWarp; };
-    int nlist = 0;
-#pragma unroll
-    for (int b = B0; b < kNumBins; b++)
-        nlist += listed(b) ? P.cnt->bin_count[b] : 0;
-    const int nsweep = P.cnt->n_batch > 0 ? r1 - P.r_lo : 0;
-    for (int it = gw; it < nlist + nsweep; it += nwarps) {
-        int row;
-        const int *sc = scol;
-        const T *sv = sval;
-        long long src;
-        T a = T(0);
-        bool copy = false;
-        if (it < nlist) {
-            int b = B0, i = it;
-            for (;; b++) {
-                const int c = listed(b) ? P.cnt->bin_count[b] : 0;
-                if (i < c)
-                    break;
-                i -= c;
-            }
-            row = P.rows[(size_t)b * M + i];
-            if (row < P.r_lo || row >= r1)
+    // classes by their lists of rows, then (only when there are batches) the
+    // batched mid rows by a sweep over the rows (class kNumBins here); each
+    // class starts at the warp after the last one's
+    int w0 = gw;
+    for (int b = COPY ? kBinCopy : kBinWarp; b <= kNumBins; b++) {
+        if (b > kBinWarp && b < kBinMidWarp)
+            continue;
+        const bool sweep = b == kNumBins;
+        const bool copy = COPY && b == kBinCopy;
+        const int n = !sweep ? P.cnt->bin_count[b] : P.cnt->n_batch > 0 ? r1 - P.r_lo : 0;
+        if (n == 0)
+            continue;
+        const int *sc = copy ? B.col : scol;
+        const T *sv = copy ? (const T *)B.val : sval;
+        for (int it = w0; it < n; it += nwarps) {
+            const int row = sweep ? P.r_lo + it : P.rows[(size_t)b * M + it];
+            if (row < P.r_lo || row >= r1 || (sweep && P.mid_flop[row] == 0))
                 continue;
-            copy = COPY && b == kBinCopy;
+            long long src;
+            T a = T(0);
             if (copy) {
                 const int j = A.rpt[row] + P.copy_leaf[row];
                 a = ((const T *)A.val)[j];
-                sc = B.col;
-                sv = (const T *)B.val;
                 src = P.abs[j];
             } else {
-                src = P.mw_pre[row];
+                src = sweep ? (long long)P.cnt->mw_total + P.mid_pre[row] : P.mw_pre[row];
             }
-        } else {
-            row = P.r_lo + (it - nlist);
-            if (P.mid_flop[row] == 0)
-                continue;
-            src = (long long)P.cnt->mw_total + P.mid_pre[row];
-        }
-        const long long dst = crpt[row];
-        int n = P.nnz[row];
-        if (n > 0 && !(BRM_IN(P.cnt, dst + n - 1, P.c_cap) && BRM_IN(P.cnt, src + n - 1, copy ? (long long)B.nnz : P.mid_cap)))
-            n = 0;  // checked build: a row outside C, B or the scratch is skipped
-        // four elements per lane in flight before the stores
-        int i = lane;
-        for (; i + 96 < n; i += 128) {
-            int c[4];
-            T v[4];
+            const int dst = crpt[row];
+            int m = P.nnz[row];
+            if (m > 0 && !(BRM_IN(P.cnt, (long long)dst + m - 1, P.c_cap) &&
+                           BRM_IN(P.cnt, src + m - 1, copy ? (long long)B.nnz : P.mid_cap)))
+                m = 0;  // checked build: a row outside C, B or the scratch is skipped
+            const int *rc = sc + src;
+            const T *rv = sv + src;
+            int *oc = ccol + dst;
+            T *ov = cval + dst;
+            // four entries a lane in flight before the stores
+            int i = lane;
+            for (; i + 96 < m; i += 128) {
+                int c[4];
+                T v[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                c[u] = sc[src + i + 32 * u];
-                v[u] = sv[src + i + 32 * u];
-            }
+                for (int u = 0; u < 4; u++) {
+                    c[u] = rc[i + 32 * u];
+                    v[u] = rv[i + 32 * u];
+                }
 #pragma unroll
-            for (int u = 0; u < 4; u++) {
-                ccol[dst + i + 32 * u] = c[u];
-                cval[dst + i + 32 * u] = copy ? vmul(a, v[u]) : v[u];
+                for (int u = 0; u < 4; u++) {
+                    oc[i + 32 * u] = c[u];
+                    ov[i + 32 * u] = copy ? vmul(a, v[u]) : v[u];
+                }
+            }
+            for (; i < m; i += 32) {
+                oc[i] = rc[i];
+                ov[i] = copy ? vmul(a, rv[i]) : rv[i];
             }
         }
-        for (; i < n; i += 32) {
-            ccol[dst + i] = sc[src + i];
-            cval[dst + i] = copy ? vmul(a, sv[src + i]) : sv[src + i];
-        }
+        w0 -= n % nwarps;
+        if (w0 < 0)
+            w0 += nwarps;
     }
 }
 

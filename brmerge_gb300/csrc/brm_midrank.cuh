@@ -673,11 +673,11 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
     }
 }
 
-// The classes (their limits: kRk* in brm_plan.h).  CTAs an SM by shared memory
+// The classes from 1 on (their limits: kRk* in brm_plan.h; class 0:
+// brm_rankpack.cuh).  CTAs an SM by shared memory
 // or by registers, whichever ends first.  Most columns have several products
 // where rows are long and lists many (class 2: stencils, finite elements;
 // class 7), few where lists are long and few (power-law graphs).
-using Rank0 = RankShape<kBinRank0, 4, 1, false, false, 18, 256, 8, 5>;
 using Rank1 = RankShape<kBinRank0 + 1, 12, 1, false, false, 19, 384, 4, 6>;
 using Rank2 = RankShape<kBinRank0 + 2, 6, 4, false, true, 19, 1536, 1, 10>;
 using Rank3 = RankShape<kBinRank0 + 3, 12, 4, false, false, 19, 1536, 1, 7>;
@@ -685,7 +685,7 @@ using Rank4 = RankShape<kBinRank0 + 4, 12, 8, false, false, 19, 3072, 1, 4>;
 using Rank5 = RankShape<kBinRank0 + 5, 12, 16, false, false, 19, 6144, 1, 2>;
 using Rank6 = RankShape<kBinRank0 + 6, 6, 4, true, false, 19, 768, 1, 8>;
 using Rank7 = RankShape<kBinRank0 + 7, 12, 8, true, true, 19, 3072, 1, 3>;
-static_assert(Rank0::F == kRkF0 && Rank1::F == kRkF1 && Rank2::F == kRkF2 && Rank3::F == kRkF3 &&
+static_assert(Rank1::F == kRkF1 && Rank2::F == kRkF2 && Rank3::F == kRkF3 &&
                   Rank4::F == kRkF4 && Rank5::F == kRkF5 && Rank6::F == kRkF2 && Rank7::F == kRkF4,
               "the analysis bins by these");
 
@@ -700,39 +700,6 @@ inline void launch_mid_rank(const CsrDev &A, const CsrDev &B, const PlanDev &P, 
     k_mid_rank<T, MODE, S><<<num_sms * S::CTAS, S::THREADS, S::bytes, s>>>(A, B, P, crpt, ccol,
                                                                             cval);
     count_launch();
-}
-
-// The warp rows, the four-warp group rows and the tile rows of one mode, by
-// rank or by merging.
-// which: kMidGroups (the four-warp groups), kMidWarps (warp and tile rows) or
-// both; classes without rows are not launched.
-template <typename T, int MODE>
-inline void launch_mid_warp(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int *crpt,
-                            int *ccol, T *cval, int num_sms, cudaStream_t s,
-                            int which = kMidGroups | kMidWarps)
-{
-    if (which & kMidGroups) {
-        if (plan_live(P, live_bit(kBinMidGroup2)))
-            launch_mid_group<T, MODE, 5>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(kBinMidGroup)))
-            launch_mid_group<T, MODE, 4>(A, B, P, crpt, ccol, cval, num_sms, s);
-        launch_mid_rank<T, MODE, Rank5>(A, B, P, crpt, ccol, cval, num_sms, s);
-        launch_mid_rank<T, MODE, Rank7>(A, B, P, crpt, ccol, cval, num_sms, s);
-        launch_mid_rank<T, MODE, Rank4>(A, B, P, crpt, ccol, cval, num_sms, s);
-        launch_mid_rank<T, MODE, Rank3>(A, B, P, crpt, ccol, cval, num_sms, s);
-    }
-    if (which & kMidWarps) {
-        launch_mid_rank<T, MODE, Rank6>(A, B, P, crpt, ccol, cval, num_sms, s);
-        launch_mid_rank<T, MODE, Rank2>(A, B, P, crpt, ccol, cval, num_sms, s);
-        launch_mid_rank<T, MODE, Rank1>(A, B, P, crpt, ccol, cval, num_sms, s);
-        launch_mid_rank<T, MODE, Rank0>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(kBinMidWarp)))
-            launch_mid_group<T, MODE, 1>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(kBinMidTile2)))
-            launch_mid_tile<T, MODE, 8>(A, B, P, crpt, ccol, cval, num_sms, s);
-        if (plan_live(P, live_bit(kBinMidTile)))
-            launch_mid_tile<T, MODE, 4>(A, B, P, crpt, ccol, cval, num_sms, s);
-    }
 }
 
 }  // namespace brm

@@ -5,7 +5,7 @@
 
 #include "brm_kernels.h"
 #include "brm_mid.cuh"
-#include "brm_midrank.cuh"
+#include "brm_rankpack.cuh"
 #include "brm_seg.cuh"
 #include "brm_rows.cuh"
 
@@ -63,6 +63,9 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
         }
         launch_mid_warp<T, UPPER ? kMwUpper : kMwPrecise>(A, B, P, crpt, ccol, cval, num_sms,
                                                           s);
+        if (plan_live(P, live_bit(kBinSegRow)))
+            launch_seg_kernel<T, UPPER ? kSegRowUpper : kSegRowPrecise>(A, B, P, crpt, ccol, cval,
+                                                                        num_sms, s);
         if (plan_live(P, live_bit(kBinBatch))) {
             const size_t msm = MidNumLayout<T>::bytes;
             cudaFuncSetAttribute(k_mid_numeric<T, UPPER>,
@@ -78,21 +81,8 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
     if (segs) {
         k_split<0><<<num_sms * 8, 256, 0, s>>>(A, B, P);
         count_launch();
-        const size_t ssm = SegLayout<T>::bytes;
-        cudaFuncSetAttribute(k_seg_numeric<T, UPPER>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ssm);
-        // as many segment CTAs as fit on every SM (shared memory and registers)
-        static int seg_per_sm = 0;
-        if (seg_per_sm <= 0) {
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&seg_per_sm,
-                                                              k_seg_numeric<T, UPPER>,
-                                                              kSegThreads, ssm) != cudaSuccess ||
-                seg_per_sm <= 0)
-                seg_per_sm = 1;
-        }
-        k_seg_numeric<T, UPPER><<<num_sms * seg_per_sm, kSegThreads, ssm, s>>>(A, B, P, crpt,
-                                                                                ccol, cval);
-        count_launch();
+        launch_seg_kernel<T, UPPER ? kSegUpper : kSegPrecise>(A, B, P, crpt, ccol, cval, num_sms,
+                                                              s);
         if (compact_late) {
             // fork again after the segments (the event is re-recorded: the
             // aux stream's first wait has already taken its earlier state)
@@ -157,6 +147,8 @@ void launch_mid_scratch_t(const CsrDev &A, const CsrDev &B, const PlanDev &P, in
                                                                     (T *)mid_val);
         count_launch();
     }
+    if ((which & kMidGroups) && plan_live(P, live_bit(kBinSegRow)))
+        launch_seg_kernel<T, kSegRowScratch>(A, B, P, nullptr, mid_col, (T *)mid_val, num_sms, s);
     launch_mid_warp<T, kMwScratch>(A, B, P, nullptr, mid_col, (T *)mid_val, num_sms, s, which);
 }
 

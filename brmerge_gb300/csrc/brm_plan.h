@@ -41,7 +41,9 @@ constexpr int kMidMaxRows = kMidCap / (kWarpMaxFlop + 1) + 2;
 // kMidMaxK A entries) in their own class.  All take precedence over the
 // batched mid rows and over the segmented heavy rows.  Holding the first two
 // classes to 64 lists keeps their merge-tree stacks at seven levels and
-// their kernels within 80 registers without spills.
+// their kernels within 80 registers without spills.  Longer rows are cut into
+// segments (merged in one piece up to 5888 products they took 178 us of R-MAT
+// n=2^18, the whole call 2.24 -> 2.18 ms without).
 constexpr int kMwF = 768;
 constexpr int kMwMaxK = 64;
 constexpr int kMwRangeBits = 22;
@@ -50,14 +52,13 @@ constexpr int kMt2F = 128;        // second tile class: at most 128 products
 constexpr int kMtRangeBits = 25;
 constexpr int kMgF = 3072;
 constexpr int kMgRangeBits = 20;
-constexpr int kMg2F = 5888;       // second group class: two groups a CTA fit 2 CTAs an SM
+constexpr int kMg2F = 3072;       // second group class: 65 to 255 lists
 constexpr int kMg2RangeBits = 19;
 // Rank rows (brm_midrank.cuh): rows of at most 64 lists whose products are
 // placed by population counts instead of sorted; they take precedence over the
 // tile, warp and group rows above, which keep the rows of 65 to 255 lists and
 // the wide ranges (the bitmap's summary outgrows a row's shared memory there).
-// R-MAT n=2^18: rows of 769..3072 products 0.35 -> 0.28 ms, of 3073..5888 0.40
-// -> 0.37 (the rows of more than 32 lists still merged).
+// R-MAT n=2^18: rows of 769..3072 products 0.35 -> 0.28 ms.
 // The most products of a row of each class:
 constexpr int kRkF0 = 128;
 constexpr int kRkF1 = 384;
@@ -67,20 +68,24 @@ constexpr int kRkF4 = 3072;
 constexpr int kRkF5 = 6144;
 constexpr int kRkNarrowK = 32;      // lists of the rows with one mask word a column
 constexpr int kRkMaxK = 64;
-constexpr int kRkRangeBits0 = 18;   // column range, class 0
+constexpr int kRkF8 = 3072;         // class 8: more lists, by a segment's kernel
+constexpr int kRkSegMaxK = 255;
+constexpr int kRkRangeBits0 = 18;   // column range, classes 0 and 8
 constexpr int kRkRangeBits = 19;    // the others
 // The class of a row of f products, k lists and columns within `range` of the
 // first, -1 where it has none.
 __host__ __device__ inline int rank_class(long long f, int k, long long range)
 {
-    if (f <= 0 || f > kRkF5 || k > kRkMaxK || range < 0 || range >= (1ll << kRkRangeBits))
+    if (f <= 0 || f > kRkF5 || range < 0 || range >= (1ll << kRkRangeBits))
         return -1;
     if (k <= kRkNarrowK) {
         if (f <= kRkF0)
             return range < (1ll << kRkRangeBits0) ? 0 : -1;
         return f <= kRkF1 ? 1 : f <= kRkF2 ? 2 : f <= kRkF3 ? 3 : f <= kRkF4 ? 4 : 5;
     }
-    return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f <= kRkF4 ? 7 : -1;
+    if (k <= kRkMaxK)
+        return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f <= kRkF4 ? 7 : -1;
+    return f > kRkF0 && f <= kRkF8 && k <= kRkSegMaxK && range < (1ll << kRkRangeBits0) ? 8 : -1;
 }
 // Subsets of the mid-row kernels (they can run on different streams).
 constexpr int kMidGroups = 1;     // the batched mid rows and the four-warp group rows
@@ -100,6 +105,7 @@ constexpr int kMidWarps = 2;      // the warp and tile rows
 #endif
 constexpr int kSegThreads = BRM_SEG_THREADS;
 constexpr int kSegCap = BRM_SEG_CAP;
+static_assert(kRkF8 <= kSegCap, "rank rows of class 8 are a segment's size");
 // Target products between cuts (a runtime knob, brm_tuning.seg_cut): the
 // default and the largest accepted.  Segments average about the target, so a
 // larger one means fewer segments (less fixed work per product in the
@@ -143,7 +149,8 @@ enum RowBin : int {
     kBinMidTile2 = 9, // the same with twice the products
     kBinMidGroup2 = 10,  // four warps per row, longer rows (brm_midwarp.cuh)
     kBinRank0 = 11,      // rank rows, classes 0 .. 7 (brm_midrank.cuh)
-    kNumBins = 19,
+    kBinSegRow = 19,     // rank rows of more than 64 lists, class 8 (brm_seg.cuh)
+    kNumBins = 20,
 };
 
 constexpr int kRankClasses = kNumBins - kBinRank0;
@@ -329,7 +336,7 @@ constexpr unsigned kLiveMidRows = live_bit(kBinWarp) | live_bit(kBinBatch) | liv
 constexpr unsigned kLiveGroups = live_bit(kBinBatch) | live_bit(kBinMidGroup) |
                                  live_bit(kBinMidGroup2) | live_bit(kBinRank0 + 3) |
                                  live_bit(kBinRank0 + 4) | live_bit(kBinRank0 + 5) |
-                                 live_bit(kBinRank0 + 7);  // kMidGroups
+                                 live_bit(kBinRank0 + 7) | live_bit(kBinSegRow);  // kMidGroups
 inline bool plan_live(const PlanDev &P, unsigned bits) { return (P.live & bits) != 0; }
 
 // Capacities of a captured batch pipeline: every buffer sized by a count the

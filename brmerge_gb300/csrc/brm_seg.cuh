@@ -662,13 +662,94 @@ __device__ __forceinline__ int seg_word_prefix(const unsigned *words, int n, uns
     return tot;
 }
 
-template <typename T, bool UPPER>
+// Sequential trie of the elements [b, e) of a long column (leaves in
+// increasing order, below 2^(D-1)); the elements are loaded GB at a time, so
+// a long column does not wait for one load per element.
+template <typename T, int D, int GB, typename GetLeaf, typename GetVal>
+__device__ __forceinline__ T long_run(const GetLeaf &leaf, const GetVal &val, int b, int e)
+{
+    RegShiftReduce<T, D> sr;
+    sr.init(leaf(b), val(b));
+    for (int j0 = b + 1; j0 < e; j0 += GB) {
+        int lf[GB];
+        T lv[GB];
+#pragma unroll
+        for (int q = 0; q < GB; q++) {
+            if (j0 + q < e) {
+                lf[q] = leaf(j0 + q);
+                lv[q] = val(j0 + q);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < GB; q++)
+            if (j0 + q < e)
+                sr.push(lf[q], lv[q]);
+    }
+    return sr.finish();
+}
+
+// A long column (len products in leaf order) reduced by a whole warp.  Its
+// leaves (increasing, below 2^bits) are cut into the 32 aligned ranges of 2^s
+// leaves, s = bits - 5: every range is one subtree of the merge tree at level
+// s, so lane j reduces the products of range j on its own (at most s split
+// levels: 12 stack entries suffice for 16-bit leaves), and the subtree values
+// are then joined by the trie over their range indices (warp_trie); every
+// lane returns the value.  cnt and sv are the warp's 32-entry shared scratch.
+template <typename T, typename GetLeaf, typename GetVal>
+__device__ __forceinline__ T warp_long_column(const GetLeaf &leaf, const GetVal &val, int len,
+                                              int *cnt, T *sv)
+{
+    const int lane = threadIdx.x & 31;
+    const int bits = 32 - __clz(leaf(len - 1) | 1);
+    const int s = bits > 5 ? bits - 5 : 0;
+    __syncwarp();
+    cnt[lane] = 0;
+    __syncwarp();
+    for (int p = lane; p < len; p += 32)
+        atomicAdd(&cnt[leaf(p) >> s], 1);
+    __syncwarp();
+    const int mc = cnt[lane];
+    const int lo = warp_incl_scan(mc) - mc;
+    T v = T(0);
+    if (mc > 0)
+        v = long_run<T, 12, 4>(leaf, val, lo, lo + mc);
+    // the nonempty ranges in order, one per lane
+    const unsigned hm = __ballot_sync(kFull, mc > 0);
+    const int r = __popc(hm & ((1u << lane) - 1u));
+    __syncwarp();
+    if (mc > 0) {
+        sv[r] = v;
+        cnt[r] = lane;
+    }
+    __syncwarp();
+    const int nh = __popc(hm);
+    const int li = lane < nh ? cnt[lane] : 0;
+    const T vi = lane < nh ? sv[lane] : T(0);
+    __syncwarp();
+    return __shfl_sync(kFull, warp_trie<T>(li, vi, nh), 0);  // the trie's value is in lane 0
+}
+
+// What the kernel works on and where it writes: heavy-row segments into C
+// (kSegPrecise) or C_bar (kSegUpper); or whole rows of at most kSegCap products
+// and 65 to 255 lists (rank class 8), counted (kSegRowSymbolic) or written
+// at crpt, at the row's offset in C_bar or in the one-call scratch.
+enum SegMode : int {
+    kSegPrecise = 0,
+    kSegUpper = 1,
+    kSegRowSymbolic = 2,
+    kSegRowPrecise = 3,
+    kSegRowUpper = 4,
+    kSegRowScratch = 5,
+};
+
+template <typename T, int MODE>
 __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
     k_seg_numeric(CsrDev A, CsrDev B, PlanDev P, const int *crpt, int *ccol, T *cval)
 {
     if (P.cnt->abort)  // a capacity check of a captured pipeline failed
         return;
     constexpr int NT = kSegThreads, NP = kSegNP;
+    constexpr bool ROWS = MODE >= kSegRowSymbolic;
     using L = SegLayout<T>;
     constexpr int NW = L::NW;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -697,8 +778,12 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
     SegRun *srun = (SegRun *)(smem + L::o_run);
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const unsigned ltm = lanemask_lt(), lem = ltm | (1u << lane);
-    const int i0 = P.seg_range ? P.seg_range[0] : 0;
-    const int nsegs = P.seg_range ? P.seg_range[1] : P.cnt->n_seg;
+    const int i0 = !ROWS && P.seg_range ? P.seg_range[0] : 0;
+    const int nsegs = ROWS            ? P.cnt->bin_count[kBinSegRow]
+                      : P.seg_range ? P.seg_range[1]
+                                    : P.cnt->n_seg;
+    const int *rows = P.rows + (size_t)kBinSegRow * A.M;
+    int *work = ROWS ? &P.cnt->work_mw[kMwRankCounter + kBinSegRow - kBinRank0] : &P.cnt->work_seg;
     const int *__restrict__ bcol = B.col;
     const T *__restrict__ bval = (const T *)B.val;
     const T *__restrict__ aval = (const T *)A.val;
@@ -712,12 +797,14 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
     int pf = 0;
     bool pf_copied = false;
     if (tid == 0)
-        pf = i0 + atomicAdd(&P.cnt->work_seg, 1);
+        pf = i0 + atomicAdd(work, 1);
     for (;;) {
         if (tid == 0) {
-            if (!pf_copied && pf < nsegs)
-                copy_seg_run(srun, P.run + pf);
-            cp_async_wait_all();
+            if (!ROWS) {
+                if (!pf_copied && pf < nsegs)
+                    copy_seg_run(srun, P.run + pf);
+                cp_async_wait_all();
+            }
             misc[0] = pf;
         }
         if (tid < kSegPWords)
@@ -728,20 +815,35 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         const int item = misc[0];
         if (item >= nsegs)
             break;
-        const SegRun d = *srun;
+        SegRun d;
+        if (ROWS) {
+            d.row = rows[item];
+            const int2 cr = P.crange[d.row];
+            d.c_lo = cr.x;
+            d.c_hi = cr.y + 1;
+            d.u_off = 0;
+            d.nprod = P.flop[d.row];
+            d.a0 = A.rpt[d.row];
+            d.k = A.rpt[d.row + 1] - d.a0;
+        } else {
+            d = *srun;
+        }
         if (tid == 0) {
-            pf = i0 + atomicAdd(&P.cnt->work_seg, 1);  // consumed after the columns are read
+            pf = i0 + atomicAdd(work, 1);  // consumed after the columns are read
             pf_copied = false;
+        }
+        if (ROWS && (d.row < P.r_lo || d.row >= P.r_hi)) {
+            __syncthreads();
+            continue;
         }
         const int row = d.row;
         const int a0 = d.a0;
         const int k = d.k;
         const int span = d.c_hi - d.c_lo;
-        // distinct columns of the row up to the next segment (checked below)
-        const int next_u = d.next_u;
         const int nsum = (span + 1023) >> 10;
-        const int *sp0 = P.split + d.sp;
-        const int *sp1 = sp0 + k;
+        // where each list starts, and ends (rows: how long it is)
+        const int *sp0 = ROWS ? P.abs + a0 : P.split + d.sp;
+        const int *sp1 = ROWS ? P.alen + a0 : sp0 + k;
         // a segment spanning at most 32 * kSegCap columns ranks its columns
         // with one flat bitmap; wider ones with a summary bit per nonempty
         // word and compressed words
@@ -773,7 +875,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 len[q] = 0;
                 if (l < k) {
                     st[q] = sp0[l];
-                    len[q] = sp1[l] - st[q];
+                    len[q] = ROWS ? sp1[l] : sp1[l] - st[q];
                 }
                 ne += len[q] > 0;
                 psum += len[q];
@@ -815,7 +917,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         }
         if (nprod > kSegCap || nprod != d.nprod || nsum > kSumWords || span <= 0 || nprod == 0) {
             // (the columns before a chunk's first cut may hold no product)
-            if (tid == 0 && !(nprod == 0 && d.nprod == 0 && next_u == d.u_off))
+            if (tid == 0 && (ROWS || nprod != 0 || d.nprod != 0 || d.next_u != d.u_off))
                 atomicOr(&P.cnt->err, kErrWindowOverflow);
             __syncthreads();
             continue;
@@ -872,7 +974,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
             misc[8] = 1;
         __syncthreads();
         // every thread has read this segment's record: copy the next one
-        if (tid == 0 && pf < nsegs) {
+        if (!ROWS && tid == 0 && pf < nsegs) {
             copy_seg_run(srun, P.run + pf);
             pf_copied = true;
         }
@@ -905,12 +1007,26 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         // 3. distinct columns, and those before each word
         const int U = seg_word_prefix<NT>(cw, ncw, pre, wsi);
         const bool nodup = U == nprod;
-        if (U != next_u - d.u_off) {  // must produce exactly its share of the row's columns
+        if (MODE == kSegRowSymbolic) {
+            if (tid == 0)
+                P.nnz[row] = U;
+            __syncthreads();
+            continue;
+        }
+        // must produce exactly the row's columns, or its share of them
+        const long long rbase = MODE == kSegPrecise || MODE == kSegRowPrecise ? (long long)crpt[row]
+                                : MODE == kSegRowScratch ? P.mw_pre[row]
+                                                         : P.scan_flop[row];
+        if ((!ROWS && U != d.next_u - d.u_off) ||
+            (MODE == kSegRowPrecise && U != crpt[row + 1] - (int)rbase)) {
             if (tid == 0)
                 atomicOr(&P.cnt->err, kErrNnzMismatch);
             __syncthreads();
             continue;
         }
+        if ((MODE == kSegRowUpper || MODE == kSegRowScratch) && tid == 0)
+            P.nnz[row] = U;
+        const long long obase = rbase + d.u_off;
         __syncthreads();
         // 4. column rank of each product and its turn among the column's (in
         //    arbitrary order)
@@ -999,9 +1115,9 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         //    warp: most sizes fill a few); the value to position u.
         //    Columns with more than 32 products first: one warp each puts them
         //    in leaf order with a bitmap over the products and hands them to
-        //    the column reducer through the long-column scratch; when the
-        //    scratch is full its first lane reduces them
-        const long long obase = (UPPER ? P.scan_flop[row] : (long long)crpt[row]) + d.u_off;
+        //    the column reducer through the long-column scratch; of whole rows
+        //    (at most 255 lists), and when the scratch is full, its first lane
+        //    reduces them
         if (nlong > 0) {
             unsigned *bmp = (unsigned *)(smem + L::o_bmp) + w * kSegPWords;
             unsigned short *wpre =
@@ -1019,7 +1135,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 const int ncol = __popc(__ballot_sync(kFull, lj < nlong));
                 const int lincl = warp_incl_scan(ln);
                 unsigned long long rcol = 0, relem = 0;
-                if (lane == 31) {
+                if (!ROWS && lane == 31) {
                     rcol = atomicAdd(&P.cnt->long_cols, (unsigned long long)ncol);
                     relem = atomicAdd(&P.cnt->long_elems, (unsigned long long)lincl);
                 }
@@ -1032,7 +1148,8 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     const long long lci = (long long)rcol + jc;
                     const long long leo =
                         (long long)relem + __shfl_sync(kFull, lincl - ln, jc);
-                    const bool handoff = lci < P.long_cap_cols && leo + len <= P.long_cap_elems;
+                    const bool handoff =
+                        !ROWS && lci < P.long_cap_cols && leo + len <= P.long_cap_elems;
                     for (int x = lane; x < nwd; x += 32)
                         bmp[x] = 0;
                     __syncwarp();
@@ -1066,7 +1183,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                             ord[r ? rp + r : u] = (unsigned short)x;
                         }
                     }
-                    if (lci < P.long_cap_cols && lane == 0) {
+                    if (!ROWS && lci < P.long_cap_cols && lane == 0) {
                         LongCol lc;
                         lc.out = obase + u;
                         lc.off = leo;
@@ -1077,7 +1194,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     __syncwarp();
                     if (handoff)
                         continue;
-                    if (lane == 0) {
+                    if (lane == 0) {  // (a stack in local memory: registers are short)
                         ShiftReduce<T, 17> sr;
                         sr.init(leaf_of(plist[ord[u]]), vals[ord[u]]);
                         for (int i = 1; i < len; i++)
@@ -1126,87 +1243,41 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
         // 8. the segment's columns (the column reducer overwrites those handed
         //    to it)
         for (int u = tid; u < U; u += NT) {
-            if (BRM_IN(P.cnt, obase + u, P.c_cap)) {
+            if (BRM_IN(P.cnt, obase + u, MODE == kSegRowScratch ? P.mid_cap : P.c_cap)) {
                 ccol[obase + u] = d.c_lo + ucol[u];
                 cval[obase + u] = vals[u];
             }
         }
         __syncthreads();
     }
+    // whole rows: the last block clears the counter for the next launch
+    if (ROWS && tid == 0) {
+        int *done = &P.cnt->done_mw[kMwRankCounter + kBinSegRow - kBinRank0];
+        __threadfence();
+        if (atomicAdd(done, 1) == (int)gridDim.x - 1) {
+            atomicExch(work, 0);
+            atomicExch(done, 0);
+        }
+    }
+}
+
+template <typename T, int MODE>
+inline void launch_seg_kernel(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int *crpt,
+                              int *ccol, T *cval, int num_sms, cudaStream_t s)
+{
+    const size_t ssm = SegLayout<T>::bytes;
+    cudaFuncSetAttribute(k_seg_numeric<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)ssm);
+    // as many CTAs as fit on every SM (shared memory and registers)
+    k_seg_numeric<T, MODE><<<num_sms * (3 * 256 / kSegThreads), kSegThreads, ssm, s>>>(
+        A, B, P, crpt, ccol, cval);
+    count_launch();
 }
 
 // ---------------------------------------------------------------------------
 // 4. column reducer: one warp per long column handed over by the segment
 //    kernel; its products are in leaf order.
 // ---------------------------------------------------------------------------
-// Sequential trie of the elements [b, e) of a long column (leaves in
-// increasing order, below 2^(D-1)); the elements are loaded GB at a time, so
-// a long column does not wait for one load per element.
-template <typename T, int D, int GB = kGatherBatch>
-__device__ __forceinline__ T long_run(const unsigned short *__restrict__ lleaf,
-                                      const T *__restrict__ lval, long long b, long long e)
-{
-    RegShiftReduce<T, D> sr;
-    sr.init(lleaf[b], lval[b]);
-    for (long long j0 = b + 1; j0 < e; j0 += GB) {
-        int lf[GB];
-        T lv[GB];
-#pragma unroll
-        for (int q = 0; q < GB; q++) {
-            if (j0 + q < e) {
-                lf[q] = lleaf[j0 + q];
-                lv[q] = lval[j0 + q];
-            }
-        }
-#pragma unroll
-        for (int q = 0; q < GB; q++)
-            if (j0 + q < e)
-                sr.push(lf[q], lv[q]);
-    }
-    return sr.finish();
-}
-
-// A long column reduced by a whole warp.  Its leaves (strictly increasing,
-// below 2^bits) are cut into the 32 aligned ranges of 2^s leaves, s = bits - 5:
-// every range is one subtree of the merge tree at level s, so lane j reduces
-// the products of range j on its own (at most s split levels: 12 stack
-// entries suffice for 16-bit leaves), and the subtree values are then joined
-// by the trie over their range indices (warp_trie); every lane returns the
-// value.  cnt and sv are the warp's 32-entry shared scratch.
-template <typename T>
-__device__ __forceinline__ T warp_long_column(const unsigned short *__restrict__ lleaf,
-                                              const T *__restrict__ lval, long long b, int len,
-                                              int *cnt, T *sv)
-{
-    const int lane = threadIdx.x & 31;
-    const int bits = 32 - __clz((int)lleaf[b + len - 1] | 1);
-    const int s = bits > 5 ? bits - 5 : 0;
-    cnt[lane] = 0;
-    __syncwarp();
-    for (int p = lane; p < len; p += 32)
-        atomicAdd(&cnt[lleaf[b + p] >> s], 1);
-    __syncwarp();
-    const int mc = cnt[lane];
-    const int lo = warp_incl_scan(mc) - mc;
-    T v = T(0);
-    if (mc > 0)
-        v = long_run<T, 12, 4>(lleaf, lval, b + lo, b + lo + mc);
-    // the nonempty ranges in order, one per lane
-    const unsigned hm = __ballot_sync(kFull, mc > 0);
-    const int r = __popc(hm & ((1u << lane) - 1u));
-    __syncwarp();
-    if (mc > 0) {
-        sv[r] = v;
-        cnt[r] = lane;
-    }
-    __syncwarp();
-    const int nh = __popc(hm);
-    const int li = lane < nh ? cnt[lane] : 0;
-    const T vi = lane < nh ? sv[lane] : T(0);
-    __syncwarp();
-    return __shfl_sync(kFull, warp_trie<T>(li, vi, nh), 0);  // the trie's value is in lane 0
-}
-
 template <typename T>
 __global__ void __launch_bounds__(128) k_long_warp(PlanDev P, int *ccol, T *cval)
 {
@@ -1225,7 +1296,11 @@ __global__ void __launch_bounds__(128) k_long_warp(PlanDev P, int *ccol, T *cval
         if (c.len <= 0 || !BRM_IN(P.cnt, c.off + c.len - 1, P.long_cap_elems) ||
             !BRM_IN(P.cnt, c.out, P.c_cap))
             continue;
-        const T r = warp_long_column<T>(lleaf, lval, c.off, c.len, s_cnt[wid], s_val[wid]);
+        const unsigned short *lf = lleaf + c.off;
+        const T *lv = lval + c.off;
+        const T r = warp_long_column<T>([&](int j) { return (int)lf[j]; },
+                                        [&](int j) { return lv[j]; }, c.len, s_cnt[wid],
+                                        s_val[wid]);
         if (lane == 0) {
             ccol[c.out] = c.col;
             cval[c.out] = r;

@@ -1,7 +1,7 @@
 // brm_symbolic.cu -- symbolic phase launchers (exact row nnz, spill routing).
 #include "brm_kernels.h"
 #include "brm_mid.cuh"
-#include "brm_midrank.cuh"
+#include "brm_rankpack.cuh"
 #include "brm_rows.cuh"
 #include "brm_seg.cuh"
 
@@ -35,6 +35,9 @@ void launch_symbolic(const CsrDev &A, const CsrDev &B, const PlanDev &P, int num
                 count_launch();
             }
             launch_mid_warp<double, kMwSymbolic>(A, B, P, nullptr, nullptr, nullptr, num_sms, s);
+            if (plan_live(P, live_bit(kBinSegRow)))
+                launch_seg_kernel<float, kSegRowSymbolic>(A, B, P, nullptr, nullptr, nullptr,
+                                                          num_sms, s);
         }
     }
     // heavy rows: exact nnz and segment plan (both Precise and Upper)

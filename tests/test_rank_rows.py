@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 EDGES = [(33, 2, 0), (64, 3, 1), (127, 32, 0), (128, 5, 3), (129, 32, 0), (383, 31, 1), (384, 7, 0),
          (385, 20, 12), (767, 32, 0), (768, 32, 0), (769, 9, 0), (1536, 32, 0), (1537, 17, 2),
          (3072, 32, 0), (3073, 30, 2), (6144, 32, 0), (6145, 32, 0), (5888, 21, 0),
-         (128, 33, 0), (129, 33, 0), (500, 40, 24), (768, 64, 0), (769, 64, 0), (2000, 48, 16),
+         (128, 33, 0), (129, 33, 0), (500, 40, 24), (129, 65, 0), (700, 300, 9), (3072, 70, 0), (3000, 2000, 5), (768, 64, 0), (769, 64, 0), (2000, 48, 16),
          (3072, 64, 0), (3073, 64, 0), (600, 65, 0)]
 
 
