@@ -621,13 +621,16 @@ __global__ void __launch_bounds__(256) k_batch_starts(PlanDev P, int M)
 // launch.
 //
 // Bound by the copy itself (24 bytes an entry in float64) and, for short rows,
-// by the latency of the look-up before it, hence a warp a row and all 64 warps
-// an SM (32 registers).  Looking 32 rows up at once and copying them end to
-// end, or four rows in flight, took 64 registers and was no faster on 512
-// uneven pairs (2.0 M rows of 72 entries) and slower on R-MAT n=2^18 (0.18 ->
-// 0.25 ms).
+// by the latency of the look-ups before it, hence a warp a row, four entries a
+// lane in flight whatever the row's length, and the next row looked up while
+// one is copied (40 registers, 48 warps an SM).  4096 uneven pairs in float64,
+// 1.15 G entries: 6.5 -> 5.4 ms (5.1 TB/s); R-MAT n=2^16 in float32 0.10 -> 0.086 ms, n=2^18 in
+// float64 0.16 ms as before.  Without the look ahead and with 64 warps an SM
+// 5.7 ms; half warps or quarters a row, which suit rows of at most 64 entries,
+// 6.4 and 8.8 ms; 32 rows looked up at once and copied end to end, 64
+// registers, was slower still.
 template <typename T, bool COPY>
-__global__ void __launch_bounds__(256, 8) k_mid_compact(CsrDev A, CsrDev B, PlanDev P,
+__global__ void __launch_bounds__(256, 6) k_mid_compact(CsrDev A, CsrDev B, PlanDev P,
                                                         const int *__restrict__ scol,
                                                         const T *__restrict__ sval,
                                                         const int *crpt, int *__restrict__ ccol,
@@ -656,21 +659,37 @@ __global__ void __launch_bounds__(256, 8) k_mid_compact(CsrDev A, CsrDev B, Plan
             continue;
         const int *sc = copy ? B.col : scol;
         const T *sv = copy ? (const T *)B.val : sval;
-        for (int it = w0; it < n; it += nwarps) {
-            const int row = sweep ? P.r_lo + it : P.rows[(size_t)b * M + it];
+        // the next row's place, and the number of the one after it, are fetched
+        // while a row is copied
+        auto row_at = [&](long long i) {
+            return i >= n ? -1 : sweep ? P.r_lo + (int)i : P.rows[(size_t)b * M + i];
+        };
+        long long src_n = 0;
+        int dst_n = 0, m_n = 0;
+        T a_n = T(0);
+        auto look_up = [&](int row) {
+            m_n = 0;
             if (row < P.r_lo || row >= r1 || (sweep && P.mid_flop[row] == 0))
-                continue;
-            long long src;
-            T a = T(0);
+                return;
             if (copy) {
                 const int j = A.rpt[row] + P.copy_leaf[row];
-                a = ((const T *)A.val)[j];
-                src = P.abs[j];
+                a_n = ((const T *)A.val)[j];
+                src_n = P.abs[j];
             } else {
-                src = sweep ? (long long)P.cnt->mw_total + P.mid_pre[row] : P.mw_pre[row];
+                src_n = sweep ? (long long)P.cnt->mw_total + P.mid_pre[row] : P.mw_pre[row];
             }
-            const int dst = crpt[row];
-            int m = P.nnz[row];
+            dst_n = crpt[row];
+            m_n = P.nnz[row];
+        };
+        look_up(row_at(w0));
+        int row2 = row_at((long long)w0 + nwarps);
+        for (long long it = w0; it < n; it += nwarps) {
+            const long long src = src_n;
+            const int dst = dst_n;
+            const T a = a_n;
+            int m = m_n;
+            look_up(row2);
+            row2 = row_at(it + 2 * nwarps);
             if (m > 0 && !(BRM_IN(P.cnt, (long long)dst + m - 1, P.c_cap) &&
                            BRM_IN(P.cnt, src + m - 1, copy ? (long long)B.nnz : P.mid_cap)))
                 m = 0;  // checked build: a row outside C, B or the scratch is skipped
@@ -679,24 +698,23 @@ __global__ void __launch_bounds__(256, 8) k_mid_compact(CsrDev A, CsrDev B, Plan
             int *oc = ccol + dst;
             T *ov = cval + dst;
             // four entries a lane in flight before the stores
-            int i = lane;
-            for (; i + 96 < m; i += 128) {
+            for (int i = lane; i < m; i += 128) {
                 int c[4];
                 T v[4];
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    c[u] = rc[i + 32 * u];
-                    v[u] = rv[i + 32 * u];
+                    if (i + 32 * u < m) {
+                        c[u] = rc[i + 32 * u];
+                        v[u] = rv[i + 32 * u];
+                    }
                 }
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    oc[i + 32 * u] = c[u];
-                    ov[i + 32 * u] = copy ? vmul(a, v[u]) : v[u];
+                    if (i + 32 * u < m) {
+                        oc[i + 32 * u] = c[u];
+                        ov[i + 32 * u] = copy ? vmul(a, v[u]) : v[u];
+                    }
                 }
-            }
-            for (; i < m; i += 32) {
-                oc[i] = rc[i];
-                ov[i] = copy ? vmul(a, rv[i]) : rv[i];
             }
         }
         w0 -= n % nwarps;

@@ -40,7 +40,7 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
     const bool compact_late = compact && fork && !P.seg_range;
     const bool copies = plan_live(P, live_bit(kBinCopy));
     if (compact && !segs && copies) {
-        k_mid_compact<T, true><<<num_sms * 8, 256, 0, s>>>(A, B, P, mid_col, (const T *)mid_val,
+        k_mid_compact<T, true><<<num_sms * 6, 256, 0, s>>>(A, B, P, mid_col, (const T *)mid_val,
                                                            crpt, ccol, cval);
         count_launch();
     } else {
@@ -49,7 +49,7 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
             count_launch();
         }
         if (compact && !compact_late) {
-            k_mid_compact<T, false><<<num_sms * 8, 256, 0, s>>>(A, B, P, mid_col,
+            k_mid_compact<T, false><<<num_sms * 6, 256, 0, s>>>(A, B, P, mid_col,
                                                                 (const T *)mid_val, crpt, ccol,
                                                                 cval);
             count_launch();
@@ -88,7 +88,7 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
             // aux stream's first wait has already taken its earlier state)
             cudaEventRecord(fk.fork, s0);
             cudaStreamWaitEvent(fk.aux, fk.fork, 0);
-            k_mid_compact<T, false><<<num_sms * 8, 256, 0, fk.aux>>>(
+            k_mid_compact<T, false><<<num_sms * 6, 256, 0, fk.aux>>>(
                 A, B, P, mid_col, (const T *)mid_val, crpt, ccol, cval);
             count_launch();
             cudaEventRecord(fk.join, fk.aux);
