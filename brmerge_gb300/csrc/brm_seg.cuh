@@ -39,8 +39,11 @@
 // an SM, about half of the issue slots).  R-MAT n=2^18, 4.1e7 products in
 // 17.9 k segments: 1147 us when every product's column, value, leaf, rank and
 // turn were staged in shared memory (111 KB, two CTAs an SM), 915 with the
-// columns in registers, 746 with columns of up to 32 products reduced in
-// place by groups of lanes.
+// columns in registers, 747 with columns of up to 32 products reduced in
+// place by groups of lanes (825 since rows of 3073 to 5888 products are cut
+// into segments too, 178 us less elsewhere).  A lane a column instead of a group
+// took 979 us with 12 % fewer instructions, the size lists claimed once a warp by
+// ballots 883, the next segment's split entries prefetched 831.
 #pragma once
 
 #include <climits>
@@ -60,8 +63,11 @@ constexpr int kPlanThreads = 512;
 constexpr int kPlanGroupLog2 = 7;
 constexpr int kPlanGroupBits = 1 << kPlanGroupLog2;      // 128 columns
 constexpr int kPlanGroupWords = kPlanGroupBits / 32;     // 4 bitmap words
+static_assert(kPlanGroupWords == 4, "one 16-byte access a group");
 constexpr int kPlanGroups = kPlanBits / kPlanGroupBits;  // 2048 per chunk
 constexpr int kDenseGroups = 128;  // 16-bit column counts: a count is at most k <= 65535
+
+static_assert(2 * kPlanThreads * 8 / 32 <= kPlanThreads, "the bits of two windows");
 
 struct PlanLayout {
     static constexpr size_t o_bm = 0;
@@ -70,26 +76,28 @@ struct PlanLayout {
     static constexpr size_t o_dix = o_gpop + kPlanGroups * 2;
     static constexpr size_t o_ccnt = o_dix + kPlanGroups * 2;
     static constexpr size_t o_lst = o_ccnt + kDenseGroups * kPlanGroupBits * 2;
-    static constexpr size_t o_loffs = o_lst + (kPlanThreads + 1) * 4;
-    static constexpr size_t o_ws = o_loffs + (kPlanThreads + 1) * 4 + 8;
+    static constexpr size_t o_starts = o_lst + kPlanThreads * 4;  // two windows of starts
+    static constexpr size_t o_ws = o_starts + kPlanThreads * 4;
     static constexpr size_t o_misc = o_ws + (kPlanThreads / 32 + 1) * 8;
     static constexpr size_t bytes = o_misc + 64;
 };
 
 // Calls f(rc) for every product of the row, rc = column - base; with clip,
 // only for the products whose column lies in [lo, chi) (each list is cut by
-// binary search).  The products are split evenly over the block: the lists
-// are taken NT at a time, their lengths scanned, and every thread walks a
-// contiguous share of the chunk's products (a single very long list of a
-// power-law row is shared by all threads instead of one group).  A thread
-// sees its products in list order, column-sorted within each list.
-// lst/loffs are NT+1 ints of shared scratch.
+// binary search).  The lists are taken NT at a time and their products in
+// windows of NT * kPlanPer: a bit per list start in product order (starts)
+// tells a product its list by a population count, and a warp's loads are
+// consecutive within a list.  lst (NT ints, a list's place in B less its first
+// product) and starts (two windows of bits) are shared scratch.
+constexpr int kPlanPer = 8;
 template <int NT, typename Fn>
 __device__ __forceinline__ void plan_products(const PlanDev &P, const int *__restrict__ bcol,
                                               int a0, int k, bool clip, int lo, int chi, int base,
-                                              int *lst, int *loffs, long long *ws, Fn f)
+                                              int *lst, unsigned *starts, long long *ws, Fn f)
 {
-    const int tid = threadIdx.x;
+    constexpr int W = NT * kPlanPer, NWD = W / 32;  // products and words of a window
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const unsigned lem = lanemask_lt() | (1u << lane);
     for (int lb = 0; lb < k; lb += NT) {
         const int l = lb + tid;
         int s = 0, len = 0;
@@ -103,51 +111,69 @@ __device__ __forceinline__ void plan_products(const PlanDev &P, const int *__res
                 len = e - s;
             }
         }
+        if (tid < 2 * NWD)
+            starts[tid] = 0;
         long long tot;
-        const int off = (int)block_excl_scan<NT, long long>(len, ws, &tot);
-        lst[tid] = s;
-        loffs[tid] = off;
-        if (tid == 0)
-            loffs[NT] = (int)tot;
+        const long long ex = block_excl_scan<NT, long long>(
+            ((long long)(len > 0) << 32) | (long long)len, ws, &tot);
+        const int off = (int)(ex & 0xffffffffLL);
+        const int n = (int)(tot & 0xffffffffLL);
+        if (len > 0)
+            lst[(int)(ex >> 32)] = s - off;
         __syncthreads();
-        const int n = (int)tot;
-        const int ipt = (n + NT - 1) / NT;
-        const int p0 = min(tid * ipt, n), p1 = min(p0 + ipt, n);
-        if (p0 < p1) {
-            int j = last_le(loffs, NT, p0);
-            int lbeg = loffs[j], lend = loffs[j + 1], bsj = lst[j];
-            for (int p = p0; p < p1; p += kGatherBatch) {
-                const int m = min(kGatherBatch, p1 - p);
-                int addr[kGatherBatch], c[kGatherBatch];
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; i++) {
-                    if (i < m) {
-                        while (p + i >= lend) {
-                            j++;
-                            lbeg = lend;
-                            lend = loffs[j + 1];
-                            bsj = lst[j];
-                        }
-                        addr[i] = bsj + (p + i - lbeg);
-                    }
-                }
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; i++)
-                    c[i] = i < m ? bcol[addr[i]] : 0;
-#pragma unroll
-                for (int i = 0; i < kGatherBatch; i++)
-                    if (i < m)
-                        f(c[i] - base);
+        int seen = -1;  // lists that start before the window, less one
+        for (long long win = 0; win < n; win += W) {
+            unsigned *cur = starts + ((win / W) & 1 ? NWD : 0);
+            unsigned *next = starts + ((win / W) & 1 ? 0 : NWD);
+            if (len > 0 && off >= win && off < win + W)
+                atomicOr(&cur[(off - (int)win) >> 5], 1u << (off & 31));
+            __syncthreads();
+            int before = 0, all = 0;
+            for (int i = lane; i < NWD; i += 32) {
+                const int c = __popc(cur[i]);
+                all += c;
+                before += i < w * kPlanPer ? c : 0;
             }
+            int j = seen + __reduce_add_sync(kFull, before);
+            seen += __reduce_add_sync(kFull, all);
+            const long long e0 = win + w * (32 * kPlanPer);
+            int c[kPlanPer];
+#pragma unroll
+            for (int u = 0; u < kPlanPer; u++) {
+                const unsigned bits = cur[w * kPlanPer + u];
+                const long long e = e0 + 32 * u + lane;
+                c[u] = e < n ? bcol[lst[j + __popc(bits & lem)] + (int)e] : 0;
+                j += __popc(bits);
+            }
+#pragma unroll
+            for (int u = 0; u < kPlanPer; u++)
+                if (e0 + 32 * u + lane < n)
+                    f(c[u] - base);
+            if (tid < NWD)
+                next[tid] = 0;
+            __syncthreads();
         }
-        __syncthreads();
     }
+}
+
+// Adds h products to a running count kept modulo cut (rem); true when a
+// multiple of cut was crossed (a division a group took a third of the planning).
+__device__ __forceinline__ bool plan_cross(unsigned &rem, unsigned h, unsigned cut)
+{
+    rem += h;
+    if (rem < cut)
+        return false;
+    rem -= cut;
+    if (rem >= cut)
+        rem %= cut;
+    return true;
 }
 
 // Walks the segment starts of planning group g (chunk-relative) in column
 // order and calls f(column_in_group, product_prefix, distinct_prefix) for
-// each.  `run` packs (products << 32 | distinct columns) before group g and
-// ph is the product count of group g-1.  A dense group (more than
+// each.  `run` packs (products << 32 | distinct columns) before group g, ph is
+// the product count of group g-1 and cross tells whether the running count
+// crossed a multiple of `cut` in that group (plan_cross).  A dense group (more than
 // dense = kSegCap - cut products) is always cut before and after; it is one
 // segment when it holds at most kSegCap products, and inside a larger one a
 // new segment starts at a column when the running product count would exceed
@@ -158,7 +184,7 @@ template <typename Fn>
 __device__ __forceinline__ void plan_group_starts(int g, unsigned h, unsigned ph,
                                                   unsigned long long run,
                                                   const unsigned short *ccnt, unsigned cut,
-                                                  unsigned dense, Fn f)
+                                                  unsigned dense, bool cross, Fn f)
 {
     const unsigned pe = (unsigned)(run >> 32);
     const unsigned ue = (unsigned)(run & 0xffffffffu);
@@ -183,16 +209,22 @@ __device__ __forceinline__ void plan_group_starts(int g, unsigned h, unsigned ph
         }
         return;
     }
-    const bool start = (g == 0) || ph > dense || (pe / cut) != ((pe - ph) / cut);
-    if (start)
+    if (g == 0 || ph > dense || cross)
         f(0, pe, ue);
 }
 
 // ---------------------------------------------------------------------------
 // 1. planning
+//
+// Bound by issue (58 % of the slots at two CTAs an SM, which shared memory
+// allows).  R-MAT n=2^18: 293 us with a contiguous share of the products a
+// thread and its columns' runs gathered in registers, 226 with windows of
+// products a lane apart, 16-byte accesses to the bitmap and no division a
+// group; float32 R-MAT n=2^16 420 -> 358.  Four products a lane: 234 and 371;
+// 40 registers (three CTAs, were there the shared memory): 246 and 328.
 // ---------------------------------------------------------------------------
 template <int UNUSED = 0>
-__global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B, PlanDev P)
+__global__ void __launch_bounds__(kPlanThreads, 2) k_heavy_plan(CsrDev A, CsrDev B, PlanDev P)
 {
     if (P.cnt->abort)  // a capacity check of a captured pipeline failed
         return;
@@ -207,7 +239,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
     unsigned *ccnt2 = (unsigned *)(smem + PlanLayout::o_ccnt);
     const unsigned short *ccnt = (const unsigned short *)(smem + PlanLayout::o_ccnt);
     int *lst = (int *)(smem + PlanLayout::o_lst);
-    int *loffs = (int *)(smem + PlanLayout::o_loffs);
+    unsigned *starts = (unsigned *)(smem + PlanLayout::o_starts);
     long long *ws = (long long *)(smem + PlanLayout::o_ws);
     int *misc = (int *)(smem + PlanLayout::o_misc);
     const int tid = threadIdx.x;
@@ -219,10 +251,13 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
     const int *__restrict__ bcol = B.col;
     const unsigned cut = (unsigned)P.seg_cut;                // <= kSegMaxCut
     const unsigned dense = (unsigned)(kSegCap - P.seg_cut);  // >= kSegCap / 4
-    for (int i = tid; i < kPlanWords; i += NT)
-        bm[i] = 0;
-    for (int i = tid; i < kPlanGroups; i += NT)
-        hist[i] = 0;
+    auto clear_groups = [&](int n) {
+        for (int g = tid; g < n; g += NT) {
+            hist[g] = 0;
+            ((uint4 *)bm)[g] = make_uint4(0, 0, 0, 0);
+        }
+    };
+    clear_groups(kPlanGroups);
     for (;;) {
         if (tid == 0)
             misc[0] = atomicAdd(&P.cnt->work_plan, 1);
@@ -264,59 +299,41 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
             }
             __syncthreads();
             // pass over the chunk's products: column bitmap and products per
-            // group.  A thread's products are column-sorted within each list,
-            // so runs in one word (group) are gathered in registers and
-            // flushed once.
+            // group
             bool bad = false;
-            unsigned run_w = 0xffffffffu, run_b = 0, run_g = 0xffffffffu, run_n = 0;
-            plan_products<NT>(P, bcol, a0, k, multi, lo, chi, lo, lst, loffs, ws, [&](int rc) {
+            plan_products<NT>(P, bcol, a0, k, multi, lo, chi, lo, lst, starts, ws, [&](int rc) {
                 if ((unsigned)rc >= (unsigned)span) {
                     bad = true;
                     return;
                 }
-                const unsigned w = (unsigned)rc >> 5;
-                if (w != run_w) {
-                    if (run_b)
-                        atomicOr(&bm[run_w], run_b);
-                    run_w = w;
-                    run_b = 0;
-                }
-                run_b |= 1u << (rc & 31);
-                const unsigned g = (unsigned)rc >> kPlanGroupLog2;
-                if (g != run_g) {
-                    if (run_n)
-                        atomicAdd(&hist[run_g], run_n);
-                    run_g = g;
-                    run_n = 0;
-                }
-                run_n++;
+                const unsigned w = (unsigned)rc >> 5, b = 1u << (rc & 31);
+                if (!(bm[w] & b))
+                    atomicOr(&bm[w], b);
+                atomicAdd(&hist[rc >> kPlanGroupLog2], 1u);
             });
-            if (run_b)
-                atomicOr(&bm[run_w], run_b);
-            if (run_n)
-                atomicAdd(&hist[run_g], run_n);
             if (bad)
                 atomicOr(&P.cnt->err, kErrBadInput);
             __syncthreads();
+            // distinct columns per group, a group a thread (16 bytes apart: a
+            // thread's own consecutive groups would meet in two banks)
+            for (int g = tid; g < ng; g += NT) {
+                const uint4 b = ((const uint4 *)bm)[g];
+                gpop[g] = (unsigned short)(__popc(b.x) + __popc(b.y) + __popc(b.z) + __popc(b.w));
+            }
+            __syncthreads();
             const int gpt = (ng + NT - 1) / NT;
             const int g0 = min(tid * gpt, ng), g1 = min(g0 + gpt, ng);
-            // distinct columns per group; groups above kSegCap products get
-            // per-column counts
+            // groups above kSegCap products get per-column counts
             int nd_local = 0, dlo = INT_MAX, dhi = -1;
             unsigned long long sp = 0;
             for (int g = g0; g < g1; g++) {
                 const unsigned h = hist[g];
-                int pc = 0;
-#pragma unroll
-                for (int q = 0; q < kPlanGroupWords; q++)
-                    pc += __popc(bm[g * kPlanGroupWords + q]);
-                gpop[g] = (unsigned short)pc;
                 if (h > (unsigned)kSegCap) {
                     nd_local++;
                     dlo = min(dlo, g);
                     dhi = g;
                 }
-                sp += ((unsigned long long)h << 32) | (unsigned)pc;
+                sp += ((unsigned long long)h << 32) | (unsigned)gpop[g];
             }
             if (nd_local) {
                 atomicMin(&misc[4], dlo);
@@ -338,7 +355,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
                 const int dlo_c = lo + kPlanGroupBits * misc[4];
                 const int dhi_c = (int)min((long long)chi,
                                            (long long)lo + (long long)kPlanGroupBits * (misc[5] + 1));
-                plan_products<NT>(P, bcol, a0, k, true, dlo_c, dhi_c, lo, lst, loffs, ws, [&](int rc) {
+                plan_products<NT>(P, bcol, a0, k, true, dlo_c, dhi_c, lo, lst, starts, ws, [&](int rc) {
                     if ((unsigned)rc < (unsigned)span) {
                         const int g = rc >> kPlanGroupLog2;
                         if (hist[g] > (unsigned)kSegCap) {
@@ -360,11 +377,13 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
             if (!fail) {
                 unsigned long long run = ex;
                 unsigned ph = (g0 > 0 && g0 < ng) ? hist[g0 - 1] : 0u;
+                unsigned rem = ((unsigned)(run >> 32) - ph) % cut;
                 for (int g = g0; g < g1; g++) {
                     const unsigned h = hist[g];
                     plan_group_starts(g, h, ph, run,
                                       h > (unsigned)kSegCap ? ccnt + dix[g] * kPlanGroupBits : ccnt, cut,
-                                      dense, [&](int, unsigned, unsigned) { nstart++; });
+                                      dense, plan_cross(rem, ph, cut),
+                                      [&](int, unsigned, unsigned) { nstart++; });
                     run += ((unsigned long long)h << 32) | (unsigned)gpop[g];
                     ph = h;
                 }
@@ -377,12 +396,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
             u_run += (long long)((unsigned long long)tot & 0xffffffffull);
             if (fail) {
                 __syncthreads();
-                for (int g = g0; g < g1; g++) {
-                    hist[g] = 0;
-#pragma unroll
-                    for (int q = 0; q < kPlanGroupWords; q++)
-                        bm[g * kPlanGroupWords + q] = 0;
-                }
+                clear_groups(ng);
                 __syncthreads();
                 continue;  // keep counting distinct columns; the row takes the spill path
             }
@@ -390,12 +404,14 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
             {
                 unsigned long long run = ex;
                 unsigned ph = (g0 > 0 && g0 < ng) ? hist[g0 - 1] : 0u;
+                unsigned rem = ((unsigned)(run >> 32) - ph) % cut;
                 int r = sx;
                 for (int g = g0; g < g1; g++) {
                     const unsigned h = hist[g];
                     plan_group_starts(g, h, ph, run,
                                       h > (unsigned)kSegCap ? ccnt + dix[g] * kPlanGroupBits : ccnt, cut,
-                                      dense, [&](int c, unsigned pe, unsigned ue) {
+                                      dense, plan_cross(rem, ph, cut),
+                                      [&](int c, unsigned pe, unsigned ue) {
                                           if (BRM_IN(P.cnt, base + nseg + r, P.cnt->seg_cap)) {
                                               SegDesc &d = P.seg[base + nseg + r];
                                               d.row = row;
@@ -411,12 +427,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_heavy_plan(CsrDev A, CsrDev B,
                 }
             }
             __syncthreads();  // descriptors of this chunk visible to the block
-            for (int g = g0; g < g1; g++) {
-                hist[g] = 0;
-#pragma unroll
-                for (int q = 0; q < kPlanGroupWords; q++)
-                    bm[g * kPlanGroupWords + q] = 0;
-            }
+            clear_groups(ng);
             // c_hi and product count of each segment: read every neighbour
             // first, then write (rounds of NT segments)
             const int ctot_prod = (int)((unsigned long long)tot >> 32);
