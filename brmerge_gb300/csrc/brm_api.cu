@@ -374,7 +374,8 @@ constexpr unsigned long long kDeferProducts = 2ull << 20;
 // another class a little more than in theirs).
 void plan_rank_spans(brm::PlanDev &P, const brm::Counters &c, int num_sms)
 {
-    // rows of each narrow class on one SM at a time (brm_midrank.cuh)
+    // rows of each narrow class on one SM at a time (brm_midrank.cuh; class 0 on
+    // its own has no smaller one to take)
     constexpr int kRows[6] = {40, 24, 10, 7, 4, 2};
     std::memset(P.rank_span, 0, sizeof(P.rank_span));
     P.rank_taken = 0;

@@ -624,11 +624,11 @@ __global__ void __launch_bounds__(256) k_batch_starts(PlanDev P, int M)
 // by the latency of the look-ups before it, hence a warp a row, four entries a
 // lane in flight whatever the row's length, and the next row looked up while
 // one is copied (40 registers, 48 warps an SM).  4096 uneven pairs in float64,
-// 1.15 G entries: 6.5 -> 5.4 ms (5.1 TB/s); R-MAT n=2^16 in float32 0.10 -> 0.086 ms, n=2^18 in
-// float64 0.16 ms as before.  Without the look ahead and with 64 warps an SM
-// 5.7 ms; half warps or quarters a row, which suit rows of at most 64 entries,
-// 6.4 and 8.8 ms; 32 rows looked up at once and copied end to end, 64
-// registers, was slower still.
+// 1.15 G entries: 6.5 -> 5.4 ms (5.1 TB/s); R-MAT n=2^16 in float32 0.10 ->
+// 0.086 ms, n=2^18 in float64 0.16 ms as before.  Without the look ahead and
+// with 64 warps an SM 5.7 ms; half or quarter warps a row 6.4 and 8.8 ms; 32
+// rows looked up at once and copied end to end (64 registers) took R-MAT
+// n=2^18 from 0.18 to 0.25 ms.
 template <typename T, bool COPY>
 __global__ void __launch_bounds__(256, 6) k_mid_compact(CsrDev A, CsrDev B, PlanDev P,
                                                         const int *__restrict__ scol,

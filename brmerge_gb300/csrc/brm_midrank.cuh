@@ -1,6 +1,7 @@
 // brm_midrank.cuh -- mid rows by ranking: a product's place is computed, not sorted.
 //
-// A row of at most 64 lists (A entries) is done by a group of G warps.  Where
+// A row of at most 64 lists (A entries) is done by a group of G warps (short
+// rows: several by one warp, brm_rankpack.cuh).  Where
 // the merge kernels (brm_midwarp.cuh) sort every product's key, here the
 // distinct columns are ranked with a bitmap and a product finds its place
 // with population counts:

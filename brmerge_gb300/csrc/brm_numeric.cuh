@@ -32,7 +32,8 @@ void numeric_phase(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int
     // into C by a bandwidth-bound copy.  With heavy-row segments it waits for
     // the segment kernel (which holds every SM's registers) and runs beside
     // the latency-bound column reducer that follows it (R-MAT n=2^18 one-call
-    // Precise 2.875 -> 2.838 ms when it came in).  A numeric phase run in row parts (the host drop-in
+    // Precise 2.875 -> 2.838 ms when it came in).  A numeric phase run in row
+    // parts (the host drop-in
     // copies each part back while the next computes) keeps it first.  Without
     // segments it does the copy rows too, in one launch.
     // (kernels of row classes without rows are not launched)

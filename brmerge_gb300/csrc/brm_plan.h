@@ -56,8 +56,9 @@ constexpr int kMg2F = 3072;       // second group class: 65 to 255 lists
 constexpr int kMg2RangeBits = 19;
 // Rank rows (brm_midrank.cuh): rows of at most 64 lists whose products are
 // placed by population counts instead of sorted; they take precedence over the
-// tile, warp and group rows above, which keep the rows of 65 to 255 lists and
-// the wide ranges (the bitmap's summary outgrows a row's shared memory there).
+// tile, warp and group rows above, which keep the wide ranges (the bitmap's
+// summary outgrows a row's shared memory there).  Class 8 takes the rows of 65
+// to 255 lists through the segment kernel, a row a segment.
 // R-MAT n=2^18: rows of 769..3072 products 0.35 -> 0.28 ms.
 // The most products of a row of each class:
 constexpr int kRkF0 = 128;
@@ -111,8 +112,9 @@ static_assert(kRkF8 <= kSegCap, "rank rows of class 8 are a segment's size");
 // larger one means fewer segments (less fixed work per product in the
 // segment kernel, a smaller split table) but more dense planning groups
 // (above kSegCap - target products), whose columns are counted one by one.
-// R-MAT n=2^18 C = A*A one-call Precise: 1536 -> 3.10 ms, 2048 -> 3.02,
-// 2304 -> 2.94, 2560 -> 3.11, 2688 -> 3.11 (same output).
+// R-MAT n=2^18 C = A*A one-call Precise: 1536 -> 2.33 ms, 2048 -> 2.21,
+// 2304 -> 2.16, 2560 -> 2.18, 2688 -> 2.24; float32 R-MAT n=2^16: 3.31, 3.08,
+// 3.24, 3.30, 3.65 (same output).
 constexpr int kSegCut = kSegCap * 3 / 4;
 constexpr int kSegMaxCut = kSegCap * 7 / 8;
 constexpr int kSegMaxK = 65535;           // leaf index stored in 16 bits
