@@ -224,12 +224,11 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
     P.mid_flop[row] = weight;
     if (bin == kBinHeavy || bin == kBinMid)
         P.spill[row] = 0;
-    if (bin == kBinEmpty)
-        P.nnz[row] = 0;
-    else if (bin == kBinCopy) {
-        P.nnz[row] = (int)f;
+    // (0 until a kernel has counted the row: one that stops at an error leaves
+    // no length of an earlier call behind)
+    P.nnz[row] = bin == kBinCopy ? (int)f : 0;
+    if (bin == kBinCopy)
         P.copy_leaf[row] = leaf;
-    }
     if (bin == kBinHeavy && f > kHugeFlop) {
         // the planning takes these first, so the longest rows do not
         // start last and finish after every other block

@@ -593,9 +593,10 @@ int numeric_launch(brm_context ctx, brm_dtype dtype, bool upper, const brm_csr *
         P.seg_list = (int *)part.seg_list;
     // the phase's counters and (unless the errors of earlier parts must
     // survive) err, unless the plan has just cleared them (the batched mid rows
-    // of a one-call plan use work_bnum)
+    // of a one-call plan use work_bnum).  The err of a fresh plan stays: a plan
+    // that did not wait (ctx->deferred) has errors that nobody has read yet
     if (!ctx->fresh || sizes || brm::plan_live(P, brm::live_bit(brm::kBinBatch))) {
-        char *from = (char *)(clear_err ? &P.cnt->err : &P.cnt->work_num);
+        char *from = (char *)(clear_err && !ctx->fresh ? &P.cnt->err : &P.cnt->work_num);
         BRM_CK(cudaMemsetAsync(from, 0, (char *)(&P.cnt->long_elems + 1) - from, s));
     }
     ctx->fresh = false;
