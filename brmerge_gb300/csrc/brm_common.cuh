@@ -197,6 +197,18 @@ struct ShiftReduce {
         n++;
         last = leaf;
     }
+    // The same where leaves may repeat (a B row that repeats a column): equal
+    // leaves are joined last of all, so their number is not bounded by the tree's
+    // levels; a full stack joins its two top entries first, and no product is
+    // lost or written past the stack.
+    __device__ __forceinline__ void push_bounded(int leaf, T v)
+    {
+        if (n == DEPTH) {
+            val[n - 2] = vadd(val[n - 2], val[n - 1]);
+            n--;
+        }
+        push(leaf, v);
+    }
     __device__ __forceinline__ T finish()
     {
         while (n >= 2) {

@@ -225,8 +225,8 @@ __device__ __noinline__ void rank_row_repeats(const CsrDev B, const int *abs, co
                 const T v = vmul(arow[j], bval[i]);
                 if (sr.n == 0)
                     sr.init(j, v);
-                else if (sr.n < 64)
-                    sr.push(j, v);
+                else
+                    sr.push_bounded(j, v);
             }
         }
         ccol[u] = c;

@@ -1205,11 +1205,13 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     __syncwarp();
                     if (handoff)
                         continue;
-                    if (lane == 0) {  // (a stack in local memory: registers are short)
+                    // (a stack in local memory: registers are short; bounded: a B row
+                    // may repeat the column)
+                    if (lane == 0) {
                         ShiftReduce<T, 17> sr;
                         sr.init(leaf_of(plist[ord[u]]), vals[ord[u]]);
                         for (int i = 1; i < len; i++)
-                            sr.push(leaf_of(plist[ord[rp + i]]), vals[ord[rp + i]]);
+                            sr.push_bounded(leaf_of(plist[ord[rp + i]]), vals[ord[rp + i]]);
                         vals[u] = sr.finish();
                     }
                     __syncwarp();
