@@ -172,7 +172,9 @@ __device__ __forceinline__ int split_level(int a, int b) { return 31 - __clz(a ^
 // ShiftReduce evaluates that trie for leaves presented in increasing order:
 // consecutive leaves a < b are joined at split_level(a, b), and a lower split
 // binds tighter (operator-precedence parsing).  The stack holds at most one
-// entry per tree level.
+// entry per tree level, and so never fills; equal leaves (a B row that repeats
+// a column) are joined last of all and would outgrow it, so a full stack joins
+// its two top entries first.
 template <typename T, int DEPTH = 33>
 struct ShiftReduce {
     T val[DEPTH];
@@ -188,7 +190,7 @@ struct ShiftReduce {
     __device__ __forceinline__ void push(int leaf, T v)
     {
         int s = split_level(last, leaf);
-        while (n >= 2 && op[n - 2] < s) {
+        while (n >= 2 && (op[n - 2] < s || n == DEPTH)) {
             val[n - 2] = vadd(val[n - 2], val[n - 1]);
             n--;
         }
@@ -196,18 +198,6 @@ struct ShiftReduce {
         val[n] = v;
         n++;
         last = leaf;
-    }
-    // The same where leaves may repeat (a B row that repeats a column): equal
-    // leaves are joined last of all, so their number is not bounded by the tree's
-    // levels; a full stack joins its two top entries first, and no product is
-    // lost or written past the stack.
-    __device__ __forceinline__ void push_bounded(int leaf, T v)
-    {
-        if (n == DEPTH) {
-            val[n - 2] = vadd(val[n - 2], val[n - 1]);
-            n--;
-        }
-        push(leaf, v);
     }
     __device__ __forceinline__ T finish()
     {

@@ -226,7 +226,7 @@ __device__ __noinline__ void rank_row_repeats(const CsrDev B, const int *abs, co
                 if (sr.n == 0)
                     sr.init(j, v);
                 else
-                    sr.push_bounded(j, v);
+                    sr.push(j, v);
             }
         }
         ccol[u] = c;

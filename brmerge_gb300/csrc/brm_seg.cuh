@@ -1205,13 +1205,11 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     __syncwarp();
                     if (handoff)
                         continue;
-                    // (a stack in local memory: registers are short; bounded: a B row
-                    // may repeat the column)
-                    if (lane == 0) {
+                    if (lane == 0) {  // (a stack in local memory: registers are short)
                         ShiftReduce<T, 17> sr;
                         sr.init(leaf_of(plist[ord[u]]), vals[ord[u]]);
                         for (int i = 1; i < len; i++)
-                            sr.push_bounded(leaf_of(plist[ord[rp + i]]), vals[ord[rp + i]]);
+                            sr.push(leaf_of(plist[ord[rp + i]]), vals[ord[rp + i]]);
                         vals[u] = sr.finish();
                     }
                     __syncwarp();
