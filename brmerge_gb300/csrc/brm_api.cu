@@ -110,7 +110,6 @@ struct brm_context_s {
     // ordered by part (device), and a second stream that copies finished
     // parts of C back while the next part computes
     DevBuf partbuf;
-    DevBuf batchbuf;  // table and stacked operands of the last batch
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t part_ev[brm::kMaxParts] = {};
     // a second compute stream: the mid rows run on it beside the heavy-row
@@ -957,13 +956,6 @@ int host_call(bool upper, const int *arpt, const int *acol, const T *aval, const
 
 cudaStream_t brm::context_stream(brm_context ctx) { return ctx->stream; }
 
-int brm::batch_scratch(brm_context ctx, size_t bytes, void **p)
-{
-    BRM_TRY(grow(ctx, ctx->batchbuf, bytes));
-    *p = ctx->batchbuf.p;
-    return BRM_SUCCESS;
-}
-
 int brm::context_num_sms(brm_context ctx) { return ctx->num_sms; }
 
 int brm::numeric_async(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
@@ -1227,7 +1219,6 @@ int brm_destroy(brm_context ctx)
     if (ctx->fork.join)
         cudaEventDestroy(ctx->fork.join);
     release(ctx->partbuf);
-    release(ctx->batchbuf);
     delete ctx;
     return BRM_SUCCESS;
 }

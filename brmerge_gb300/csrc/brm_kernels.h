@@ -14,9 +14,6 @@ namespace brm {
 // The stream and SM count of a context (brm_api.cu).
 cudaStream_t context_stream(brm_context ctx);
 int context_num_sms(brm_context ctx);
-// The context's buffer for a batch's table and stacked operands, at least
-// `bytes`.
-int batch_scratch(brm_context ctx, size_t bytes, void **p);
 
 // brm_numeric without its closing synchronisation (it only enqueues work on
 // the context stream, so it can be captured into a CUDA graph once every
