@@ -200,7 +200,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
             P.crange[row] = make_int2(mn, mx);
         // rows placed by rank, where their lists and column range allow
         const int rc = rank_class(f, a1 - a0, (long long)mx - mn);
-        if (rc >= 0)
+        if (rc > 0 || (rc == 0 && !P.any_order))
             bin = kBinRank0 + rc;
         if ((bin == kBinMidWarp && (long long)mx - mn >= (1ll << kMwRangeBits)) ||
             (bin == kBinMidGroup && (long long)mx - mn >= (1ll << kMgRangeBits)) ||

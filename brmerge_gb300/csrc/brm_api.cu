@@ -293,7 +293,7 @@ int device_err_status(int err)
         return BRM_SUCCESS;
     if (err & brm::kErrOverflow)
         return BRM_ERR_OVERFLOW;
-    if (err & brm::kErrBadInput)
+    if (err & (brm::kErrBadInput | brm::kErrUnsorted))
         return BRM_ERR_INVALID_CSR;
     if (err & brm::kErrCapacity)
         return BRM_ERR_CAPACITY;
@@ -399,6 +399,14 @@ void plan_rank_spans(brm::PlanDev &P, const brm::Counters &c, int num_sms)
     }
 }
 
+// True when a call failed for nothing but short rows of unsorted B rows (not
+// valid CSR, seen where inputs are not checked): made again with any_order, its
+// plan gives them to the kernels that sort.
+bool needs_any_order(brm_context ctx, int status)
+{
+    return status != BRM_SUCCESS && ctx->last_err == brm::kErrUnsorted;
+}
+
 // Analysis + symbolic (+ crpt scan for Precise).  Leaves ctx->h_cnt filled.
 // Timed: events kEvStart, kEvAna, kEvPre, kEvSized, kEvSym, kEvScan.
 // fused_dtype >= 0 (one-call Precise only): the warp and mid rows are computed
@@ -406,10 +414,13 @@ void plan_rank_spans(brm::PlanDev &P, const brm::Counters &c, int num_sms)
 // them.  may_defer: a small call without heavy rows does not wait for nnz(C)
 // and the plan's errors (ctx->deferred; the caller reads the counters at the
 // end, and the numeric phase does nothing when the plan has failed).
+// any_order: see needs_any_order.
 int plan_phase(brm_context ctx, const brm_csr *A, const brm_csr *B, int *crpt, bool upper,
-               bool timed, int fused_dtype = -1, bool may_defer = false)
+               bool timed, int fused_dtype = -1, bool may_defer = false, bool any_order = false)
 {
     const bool fused = fused_dtype >= 0 && !upper;
+    ctx->last_err = 0;
+    ctx->plan.any_order = any_order;
     ctx->mid_ready = false;
     ctx->deferred = false;
     BRM_TRY(ensure_workspace(ctx, A->M));
@@ -975,6 +986,8 @@ int brm::read_device_error(brm_context ctx) { return read_err(ctx); }
 
 int brm::device_status(int err) { return device_err_status(err); }
 
+bool brm::only_unsorted(int err) { return err == brm::kErrUnsorted; }
+
 const brm::Counters *brm::context_counters(brm_context ctx) { return ctx->plan.cnt; }
 
 int brm::set_context_sms(brm_context ctx, int sms)
@@ -1036,7 +1049,7 @@ int brm::reserve_pipe(brm_context ctx, brm_dtype dtype, const brm::PipeCaps &c)
 }
 
 int brm::precise_pipe(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
-                      int *crpt, int *ccol, void *cval, const brm::PipeCaps &caps)
+                      int *crpt, int *ccol, void *cval, const brm::PipeCaps &caps, bool any_order)
 {
     BRM_TRY(check_dtype(dtype));
     BRM_TRY(check_pair(A, B));
@@ -1050,6 +1063,7 @@ int brm::precise_pipe(brm_context ctx, brm_dtype dtype, const brm_csr *A, const 
     ctx->plan.seg_range = nullptr;
     ctx->plan.live = brm::kLiveAll;  // the counts are on the device only
     ctx->plan.upper = 0;
+    ctx->plan.any_order = any_order;
     std::memset(ctx->plan.rank_span, 0, sizeof(ctx->plan.rank_span));
     ctx->plan.rank_taken = 0;
     ctx->fresh = false;
@@ -1346,7 +1360,10 @@ int brm_symbolic(brm_context ctx, const brm_csr *A, const brm_csr *B, int *crpt,
         return BRM_ERR_INVALID_VALUE;
     BRM_TRY(check_pair(A, B));
     ctx->planned = false;
-    BRM_TRY(plan_phase(ctx, A, B, crpt, false, false));
+    int st = plan_phase(ctx, A, B, crpt, false, false);
+    if (needs_any_order(ctx, st))
+        st = plan_phase(ctx, A, B, crpt, false, false, -1, false, true);
+    BRM_TRY(st);
     *cnnz = (int)ctx->h_cnt->cnnz;
     return BRM_SUCCESS;
 }
@@ -1368,21 +1385,17 @@ int brm_numeric(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_cs
     return read_err(ctx);
 }
 
-int brm_precise_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
-                       int **crpt_, int **ccol_, void **cval_, int *cnnz_,
-                       brm_precise_timing *timing)
+static int precise_device_once(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
+                               int **crpt_, int **ccol_, void **cval_, int *cnnz_,
+                               brm_precise_timing *timing, bool any_order)
 {
-    if (!ctx || !crpt_ || !ccol_ || !cval_ || !cnnz_)
-        return BRM_ERR_INVALID_VALUE;
-    BRM_TRY(check_dtype(dtype));
-    BRM_TRY(check_pair(A, B));
     const bool timed = timing != nullptr;
     double t0 = now_sec();
     int *crpt = nullptr;
     BRM_CK(cudaMallocAsync((void **)&crpt, 4 * ((size_t)A->M + 1), ctx->stream));
     double t1 = now_sec();
     ctx->planned = false;
-    int st = plan_phase(ctx, A, B, crpt, false, timed, dtype, true);
+    int st = plan_phase(ctx, A, B, crpt, false, timed, dtype, true, any_order);
     if (st != BRM_SUCCESS) {
         cudaFreeAsync(crpt, ctx->stream);
         return st;
@@ -1435,17 +1448,27 @@ int brm_precise_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const
     return BRM_SUCCESS;
 }
 
-int brm_upper_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
-                     int **crpt_, int **ccol_, void **cval_, int *cnnz_, brm_upper_timing *timing)
+int brm_precise_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
+                       int **crpt, int **ccol, void **cval, int *cnnz, brm_precise_timing *timing)
 {
-    if (!ctx || !crpt_ || !ccol_ || !cval_ || !cnnz_)
+    if (!ctx || !crpt || !ccol || !cval || !cnnz)
         return BRM_ERR_INVALID_VALUE;
     BRM_TRY(check_dtype(dtype));
     BRM_TRY(check_pair(A, B));
+    int st = precise_device_once(ctx, dtype, A, B, crpt, ccol, cval, cnnz, timing, false);
+    if (needs_any_order(ctx, st))
+        st = precise_device_once(ctx, dtype, A, B, crpt, ccol, cval, cnnz, timing, true);
+    return st;
+}
+
+static int upper_device_once(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
+                             int **crpt_, int **ccol_, void **cval_, int *cnnz_,
+                             brm_upper_timing *timing, bool any_order)
+{
     const bool timed = timing != nullptr;
     double t0 = now_sec();
     ctx->planned = false;
-    BRM_TRY(plan_phase(ctx, A, B, nullptr, true, timed));
+    BRM_TRY(plan_phase(ctx, A, B, nullptr, true, timed, -1, false, any_order));
     double t1 = now_sec();
     BRM_TRY(grow(ctx, ctx->bar_col, (size_t)ctx->h_cnt->total_flop * 4));
     BRM_TRY(grow(ctx, ctx->bar_val, (size_t)ctx->h_cnt->total_flop * vsize(dtype)));
@@ -1514,6 +1537,19 @@ int brm_upper_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const b
         timing->total = t5 - t0;
     }
     return BRM_SUCCESS;
+}
+
+int brm_upper_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
+                     int **crpt, int **ccol, void **cval, int *cnnz, brm_upper_timing *timing)
+{
+    if (!ctx || !crpt || !ccol || !cval || !cnnz)
+        return BRM_ERR_INVALID_VALUE;
+    BRM_TRY(check_dtype(dtype));
+    BRM_TRY(check_pair(A, B));
+    int st = upper_device_once(ctx, dtype, A, B, crpt, ccol, cval, cnnz, timing, false);
+    if (needs_any_order(ctx, st))
+        st = upper_device_once(ctx, dtype, A, B, crpt, ccol, cval, cnnz, timing, true);
+    return st;
 }
 
 int brm_device_free(brm_context ctx, void *p)

@@ -707,10 +707,68 @@ struct brm_batch_pipe_s {
     int *crpt = nullptr, *ccol = nullptr, *lrpt = nullptr;
     void *cval = nullptr;
     long long *row_off = nullptr, *nnz_off = nullptr;  // host, pairs + 1
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    long long kernels = 0;
+    // captured at creation; the second one when a batch first has short rows of
+    // unsorted B rows (not valid CSR), planned for the kernels that sort
+    struct Captured {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        long long kernels = 0;
+    } main, any_order;
 };
+
+namespace {
+
+// Captures one run: upload the table, stack, Precise, per-pair offsets, results
+// back.
+int pipe_capture(brm_batch_pipe p, bool any_order)
+{
+    brm_batch_pipe_s::Captured &g = any_order ? p->any_order : p->main;
+    cudaStream_t s = p->stream;
+    const int grid = std::max(brm::context_num_sms(p->ctx), 1) * 16;
+    int st = BRM_SUCCESS;
+    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return BRM_ERR_CUDA;
+    }
+    const long long k0 = brm::launches_so_far();
+    cudaError_t e = cudaMemcpyAsync(p->t.dims, p->ht.dims, p->t.upload, cudaMemcpyHostToDevice, s);
+    if (e == cudaSuccess) {
+        launch_stack(p->dtype, p->t, p->caps.rows, p->caps.b_rows, p->Abd, p->Bbd, grid, s, true);
+        st = brm::precise_pipe(p->ctx, p->dtype, &p->Abd, &p->Bbd, p->crpt, p->ccol, p->cval, p->pc,
+                               any_order);
+    }
+    if (e == cudaSuccess && st == BRM_SUCCESS) {
+        launch_finish(p->t, p->crpt, p->lrpt, grid, s);
+        e = cudaMemcpyAsync(p->hcnt, brm::context_counters(p->ctx), sizeof(brm::Counters),
+                            cudaMemcpyDeviceToHost, s);
+    }
+    if (e == cudaSuccess && st == BRM_SUCCESS)
+        e = cudaMemcpyAsync(p->hfirst, p->t.first, sizeof(long long) * (size_t)p->t.stride,
+                            cudaMemcpyDeviceToHost, s);
+    g.kernels = brm::launches_so_far() - k0;
+    brm::count_launches(-g.kernels);  // captured, not launched
+    const cudaError_t e2 = cudaStreamEndCapture(s, &g.graph);
+    if (st == BRM_SUCCESS && (e != cudaSuccess || e2 != cudaSuccess))
+        st = BRM_ERR_CUDA;
+    if (st == BRM_SUCCESS && cudaGraphInstantiate(&g.exec, g.graph, 0) != cudaSuccess)
+        st = BRM_ERR_CUDA;
+    if (st != BRM_SUCCESS)
+        (void)cudaGetLastError();
+    return st;
+}
+
+// Runs a captured graph and waits for it.
+int pipe_launch(const brm_batch_pipe_s::Captured &g, cudaStream_t s)
+{
+    if (cudaGraphLaunch(g.exec, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return BRM_ERR_CUDA;
+    }
+    brm::count_launches(g.kernels);
+    return BRM_SUCCESS;
+}
+
+}  // namespace
 
 extern "C" {
 
@@ -751,10 +809,12 @@ int brm_batch_pipe_destroy(brm_batch_pipe p)
         return BRM_SUCCESS;
     if (p->stream)
         cudaStreamSynchronize(p->stream);
-    if (p->exec)
-        cudaGraphExecDestroy(p->exec);
-    if (p->graph)
-        cudaGraphDestroy(p->graph);
+    for (brm_batch_pipe_s::Captured *g : {&p->main, &p->any_order}) {
+        if (g->exec)
+            cudaGraphExecDestroy(g->exec);
+        if (g->graph)
+            cudaGraphDestroy(g->graph);
+    }
     if (p->mem)
         cudaFree(p->mem);
     if (p->host)
@@ -849,37 +909,8 @@ int brm_batch_pipe_create(brm_context ctx, brm_dtype dtype, const brm_batch_caps
     p->hcnt = (brm::Counters *)((char *)p->host + b_tab);
     p->hfirst = (long long *)((char *)p->host + b_tab + h_cnt);
     std::memset(p->host, 0, b_tab + h_cnt + h_first);
-    // capture: upload the table, stack, Precise, per-pair offsets, results back
-    cudaStream_t s = p->stream;
-    const int grid = std::max(brm::context_num_sms(p->ctx), 1) * 16;
-    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
-        (void)cudaGetLastError();
-        brm_batch_pipe_destroy(p);
-        return BRM_ERR_CUDA;
-    }
-    const long long k0 = brm::launches_so_far();
-    cudaError_t e = cudaMemcpyAsync(p->t.dims, p->ht.dims, p->t.upload, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) {
-        launch_stack(dtype, p->t, c.rows, c.b_rows, p->Abd, p->Bbd, grid, s, true);
-        st = brm::precise_pipe(p->ctx, dtype, &p->Abd, &p->Bbd, p->crpt, p->ccol, p->cval, p->pc);
-    }
-    if (e == cudaSuccess && st == BRM_SUCCESS) {
-        launch_finish(p->t, p->crpt, p->lrpt, grid, s);
-        e = cudaMemcpyAsync(p->hcnt, brm::context_counters(p->ctx), sizeof(brm::Counters),
-                            cudaMemcpyDeviceToHost, s);
-    }
-    if (e == cudaSuccess && st == BRM_SUCCESS)
-        e = cudaMemcpyAsync(p->hfirst, p->t.first, sizeof(long long) * (size_t)p->t.stride,
-                            cudaMemcpyDeviceToHost, s);
-    p->kernels = brm::launches_so_far() - k0;
-    brm::count_launches(-p->kernels);  // captured, not launched
-    const cudaError_t e2 = cudaStreamEndCapture(s, &p->graph);
-    if (st == BRM_SUCCESS && (e != cudaSuccess || e2 != cudaSuccess))
-        st = BRM_ERR_CUDA;
-    if (st == BRM_SUCCESS && cudaGraphInstantiate(&p->exec, p->graph, 0) != cudaSuccess)
-        st = BRM_ERR_CUDA;
+    st = pipe_capture(p, false);
     if (st != BRM_SUCCESS) {
-        (void)cudaGetLastError();
         brm_batch_pipe_destroy(p);
         return st;
     }
@@ -912,11 +943,12 @@ int brm_batch_pipe_run(brm_batch_pipe p, int n, const brm_csr *A, const brm_csr 
     if (d.rows_a > p->caps.rows || d.nnz_a > p->caps.nnz_a || d.rows_b > p->caps.b_rows ||
         d.nnz_b > p->caps.nnz_b || cb > p->caps.cols)
         return BRM_ERR_CAPACITY;
-    if (cudaGraphLaunch(p->exec, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return BRM_ERR_CUDA;
+    BRM_STATUS_TRY(pipe_launch(p->main, s));
+    if (!p->hcnt->abort && brm::only_unsorted(p->hcnt->err)) {
+        if (!p->any_order.exec)
+            BRM_STATUS_TRY(pipe_capture(p, true));
+        BRM_STATUS_TRY(pipe_launch(p->any_order, s));
     }
-    brm::count_launches(p->kernels);
     if (p->hcnt->abort)
         return BRM_ERR_CAPACITY;
     BRM_STATUS_TRY(brm::device_status(p->hcnt->err));

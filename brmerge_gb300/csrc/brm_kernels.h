@@ -34,10 +34,11 @@ int shared_context(brm_context *out);
 // synchronisation and no allocation (capturable), the counts of each input
 // checked against the capacities on the device.  The mid rows are computed
 // with the plan.  Errors and nnz(C) stay in the device counters
-// (context_counters) for the caller to read after the stream.
+// (context_counters) for the caller to read after the stream; any_order: for
+// short rows of unsorted B rows too (only_unsorted errors).
 int reserve_pipe(brm_context ctx, brm_dtype dtype, const PipeCaps &caps);
 int precise_pipe(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B, int *crpt,
-                 int *ccol, void *cval, const PipeCaps &caps);
+                 int *ccol, void *cval, const PipeCaps &caps, bool any_order);
 const Counters *context_counters(brm_context ctx);
 // The counters the last planning left on the host (after a synchronised call).
 Counters last_plan_counters(brm_context ctx);
@@ -54,6 +55,7 @@ long long upper_bound_bytes(brm_dtype dtype, int M, long long products);
 // analysis and the mid-row prefix sums, stage 1 after the symbolic phase.
 void launch_pipe_admit(const PlanDev &P, int M, const PipeCaps &caps, int stage, cudaStream_t s);
 int device_status(int err);
+bool only_unsorted(int err);
 
 // Counts one kernel launch of this library (brm_kernel_launches reports the
 // process-wide total); every launch site calls it right after <<<...>>>.

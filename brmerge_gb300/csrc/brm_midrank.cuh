@@ -205,16 +205,36 @@ __device__ __forceinline__ unsigned quads_to_join(unsigned m)
     return (((s & 0x33333333u) + ((s >> 2) & 0x33333333u)) + 0x66666666u) & 0x88888888u;
 }
 
+// What a rank row of f products reports when its B rows are not sorted (not
+// valid CSR).  Rows of class 0's length were multiplied in any order before
+// there were rank rows: the host then plans them again for the kernels that
+// sort (PlanDev::any_order).  Longer ones are refused.
+__device__ __forceinline__ int rank_unsorted(int f)
+{
+    return f <= kRkF0 ? kErrUnsorted : kErrBadInput;
+}
+
 // A row whose B rows repeat a column (not valid CSR, but summed all the same
 // by the merge kernels: equal leaves meet first): every column by one
 // thread, list by list.
 template <typename T>
-__device__ __noinline__ void rank_row_repeats(const CsrDev B, const int *abs, const int *alen,
-                                              const T *arow, int k, const int *ucol, int U,
-                                              int cmin, int t, int nt, int *ccol, T *cval)
+__device__ __noinline__ void rank_row_repeats(const CsrDev B, Counters *cnt, const int *abs,
+                                              const int *alen, const T *arow, int k,
+                                              const int *ucol, int U, int cmin, int t, int nt,
+                                              int *ccol, T *cval)
 {
     const int *bcol = B.col;
     const T *bval = (const T *)B.val;
+    // (the search below needs sorted lists)
+    bool sorted = true;
+    int f = 0;
+    for (int j = 0; j < k; j++) {
+        f += alen[j];
+        for (int i = abs[j] + t; i < abs[j] + alen[j] - 1; i += nt)
+            sorted &= bcol[i] <= bcol[i + 1];
+    }
+    if (!sorted)
+        atomicOr(&cnt->err, rank_unsorted(f));
     for (int u = t; u < U; u += nt) {
         const int c = cmin + ucol[u];
         ShiftReduce<T, 64> sr;
@@ -422,7 +442,7 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
             }
         }
         if (bad)
-            atomicOr(&P.cnt->err, kErrBadInput);
+            atomicOr(&P.cnt->err, rank_unsorted(F));
         grp_sync<G>(gid);
         int ncw = nwords;
         if (!flat) {
@@ -573,8 +593,8 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
                 run = (unsigned)gm[3];
             nq = (int)(run >> 16);
             if ((int)(run & 0xffffu) != (S::DENSE ? F : F - U)) {  // a column repeated within a list
-                rank_row_repeats<T>(B, P.abs + a0, P.alen + a0, aval + a0, k, ucol, U, cmin, t, NT,
-                                    ccol + base, cval + base);
+                rank_row_repeats<T>(B, P.cnt, P.abs + a0, P.alen + a0, aval + a0, k, ucol, U, cmin,
+                                    t, NT, ccol + base, cval + base);
                 grp_sync<G>(gid);
                 continue;
             }

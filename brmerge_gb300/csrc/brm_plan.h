@@ -135,6 +135,7 @@ enum DevErr : int {
     kErrBadInput = 16,       // an index out of range seen by a kernel
     kErrCapacity = 32,       // a batch exceeded a captured pipeline's capacities
     kErrChecked = 64,        // a bounds check of the checked build failed (brm_check.cuh)
+    kErrUnsorted = 128,      // a short row of unsorted B rows, for the kernels that sort
 };
 
 // Row classes assigned by the analysis kernel.
@@ -308,6 +309,7 @@ struct PlanDev {
     int seg_cut;
     int mid_limit;
     int upper;  // the analysis writes scan_flop
+    int any_order;  // no rows of rank class 0 (a plan made again after kErrUnsorted)
     // entries of the arrays the numeric kernels write (C, or C_bar for
     // Upper) and of the one-call mid-row scratch; the bounds of the checked
     // build

@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(32 * PackShape::WARPS, PackShape::CTAS)
                 }
             }
             if (bad)
-                atomicOr(&P.cnt->err, kErrBadInput);
+                atomicOr(&P.cnt->err, kErrUnsorted);
             __syncwarp();
             // 3. slots of the nonempty words, their bits, columns before each
             const int ncw = pack_words(summ, nsum, srank);
@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(32 * PackShape::WARPS, PackShape::CTAS)
                     const int rsub = __shfl_sync(kFull, csub, r);
                     const long long rb = __shfl_sync(kFull, base, r) + rub;
                     if (rrow >= 0 && (outm >> r & 1u))
-                        rank_row_repeats<T>(B, P.abs + ra0, P.alen + ra0, aval + ra0, rk,
+                        rank_row_repeats<T>(B, P.cnt, P.abs + ra0, P.alen + ra0, aval + ra0, rk,
                                             ucol + rub, rue - rub, -rsub, lane, 32, ccol + rb,
                                             cval + rb);
                 }

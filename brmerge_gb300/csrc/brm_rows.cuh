@@ -760,7 +760,8 @@ __global__ void __launch_bounds__(256) k_warp_numeric(CsrDev A, CsrDev B, PlanDe
         int node = (int)(key & 0xffffffffu);
         bool active = valid;
         // level-synchronous trie reduction
-        for (int lvl = 0; lvl < 31; lvl++) {
+        int lvl = 0;
+        for (; lvl < 31; lvl++) {
             const unsigned act = __ballot_sync(kFull, active);
             const unsigned higher = lane == 31 ? 0u : (act & (0xffffffffu << (lane + 1)));
             const int nxt = higher ? __ffs(higher) - 1 : lane;
@@ -793,6 +794,10 @@ __global__ void __launch_bounds__(256) k_warp_numeric(CsrDev A, CsrDev B, PlanDe
             }
         }
         if (lane == 0) {
+            // (equal leaves never meet: a B row that repeats a column, refused as
+            // it is where the row has been counted before)
+            if (MODE == kWarpScratch && lvl == 31)
+                atomicOr(&P.cnt->err, kErrNnzMismatch);
             if (MODE != kWarpPrecise)
                 P.nnz[row] = __popc(outm);
             else if (__popc(outm) != crpt[row + 1] - crpt[row])
