@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
                     const unsigned b = 1u << (c[u] & 31);
                     const int ci = srank[sw] + __popc(summ[sw] & ((1u << ((c[u] >> 5) & 31)) - 1u));
                     pk[u] = (pk[u] & 0xfff0001fu) | ((unsigned)ci << 5);
-                    if (!(cw[ci] & b))
+                    if (BRM_IN(P.cnt, ci, S::F) && !(cw[ci] & b))
                         atomicOr(&cw[ci], b);
                 }
             }
@@ -502,6 +502,8 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
                 const int l = (int)(pk[u] >> 20);
                 const int r = pre[ci] + __popc(cw[ci] & ((1u << (pk[u] & 31u)) - 1u));
                 pk[u] = ((unsigned)l << 20) | (unsigned)r;
+                if (!BRM_IN(P.cnt, r, S::F))
+                    continue;
                 ucol[r] = c[u];
                 if (!nodup)
                     atomicOr(&mask[S::WIDE ? 2 * r + (l >> 5) : r], 1u << (l & 31));
@@ -534,7 +536,7 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
                     } else {
                         nm += __popc(mb);
                     }
-                    if (multi)
+                    if (multi && BRM_IN(P.cnt, U + o + __popc(mb & ltm), S::F))
                         mlist[o + __popc(mb & ltm)] = (unsigned short)i;
                 }
                 grp_sync<G>(gid);
@@ -578,13 +580,15 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
                     for (; g0; g0 &= g0 - 1u) {
                         const int b = (__ffs(g0) - 1) & ~3;
                         const int r = __popc(m0 & ((1u << b) - 1u));
-                        quads[o++] = S::quad(sp, r, i, (m0 >> b) & 15u);
+                        if (BRM_IN(P.cnt, o, S::F))
+                            quads[o++] = S::quad(sp, r, i, (m0 >> b) & 15u);
                     }
                     if (S::WIDE)
                         for (; g1; g1 &= g1 - 1u) {
                             const int b = (__ffs(g1) - 1) & ~3;
                             const int r = __popc(m0) + __popc(m1 & ((1u << b) - 1u));
-                            quads[o++] = S::quad(sp, r, i, (m1 >> b) & 15u);
+                            if (BRM_IN(P.cnt, o, S::F))
+                                quads[o++] = S::quad(sp, r, i, (m1 >> b) & 15u);
                         }
                 }
             }
@@ -625,7 +629,8 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
                     if (S::DENSE || i)
                         p = pre[p] + i;
                 }
-                vals[p] = vmul(av[l], v[u]);
+                if (BRM_IN(P.cnt, p, S::F))
+                    vals[p] = vmul(av[l], v[u]);
             }
         }
         grp_sync<G>(gid);

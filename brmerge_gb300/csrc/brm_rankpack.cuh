@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(32 * PackShape::WARPS, PackShape::CTAS)
                     const unsigned b = 1u << (c[u] & 31);
                     const int ci = srank[w] + __popc(summ[w] & ((1u << ((c[u] >> 5) & 31)) - 1u));
                     pk[u] |= ((unsigned)ci << 5) | (unsigned)(c[u] & 31);
-                    if (!(cw[ci] & b))
+                    if (BRM_IN(P.cnt, ci, S::F) && !(cw[ci] & b))
                         atomicOr(&cw[ci], b);
                 }
             }
@@ -301,6 +301,8 @@ __global__ void __launch_bounds__(32 * PackShape::WARPS, PackShape::CTAS)
                     const int ci = (int)((pk[u] >> 5) & 0x7fffu);
                     const int r = pre[ci] + __popc(cw[ci] & ((1u << (pk[u] & 31u)) - 1u));
                     pk[u] = (pk[u] & 0xfff00000u) | (unsigned)r;
+                    if (!BRM_IN(P.cnt, r, S::F))
+                        continue;
                     ucol[r] = c[u];
                     if (!nodup)
                         atomicOr(&mask[r], 1u << (pk[u] >> 26));
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(32 * PackShape::WARPS, PackShape::CTAS)
                     const unsigned m = i < U ? mask[i] : 0u;
                     const bool multi = (m & (m - 1u)) != 0u;
                     const unsigned mb = __ballot_sync(kFull, multi);
-                    if (multi)
+                    if (multi && BRM_IN(P.cnt, U + nm + __popc(mb & ltm), S::F))
                         mlist[nm + __popc(mb & ltm)] = (unsigned short)i;
                     nm += __popc(mb);
                 }
@@ -342,8 +344,9 @@ __global__ void __launch_bounds__(32 * PackShape::WARPS, PackShape::CTAS)
                         pre[i] = (unsigned short)sp;
                         for (; g; g &= g - 1u) {
                             const int b = (__ffs(g) - 1) & ~3;
-                            quads[o++] = Rank1::quad(sp, __popc(m & ((1u << b) - 1u)), i,
-                                                     (m >> b) & 15u);
+                            if (BRM_IN(P.cnt, o, S::F))
+                                quads[o++] = Rank1::quad(sp, __popc(m & ((1u << b) - 1u)), i,
+                                                         (m >> b) & 15u);
                         }
                     }
                 }
@@ -384,7 +387,8 @@ __global__ void __launch_bounds__(32 * PackShape::WARPS, PackShape::CTAS)
                         if (i)
                             p = pre[p] + i;
                     }
-                    vals[p] = vmul(av[(pk[u] >> 20) & 63u], v[u]);
+                    if (BRM_IN(P.cnt, p, S::F))
+                        vals[p] = vmul(av[(pk[u] >> 20) & 63u], v[u]);
                 }
             }
             __syncwarp();

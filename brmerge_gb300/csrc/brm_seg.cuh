@@ -1009,7 +1009,7 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                     const unsigned b = 1u << (c[u] & 31);
                     const int ci = srank[sw] + __popc(summ[sw] & ((1u << ((c[u] >> 5) & 31)) - 1u));
                     pk[u] |= ((unsigned)ci << 5) | (unsigned)(c[u] & 31);
-                    if (!(cw[ci] & b))
+                    if (BRM_IN(P.cnt, ci, kSegCap) && !(cw[ci] & b))
                         atomicOr(&cw[ci], b);
                 }
             }
@@ -1047,6 +1047,8 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 const int ci = (int)((pk[u] >> 5) & 0xfffu);
                 const int r = pre[ci] + __popc(cw[ci] & ((1u << (pk[u] & 31u)) - 1u));
                 pk[u] = ((pk[u] >> 17) << 12) | (unsigned)r;
+                if (!BRM_IN(P.cnt, r, kSegCap))
+                    continue;
                 ucol[r] = c[u];
                 c[u] = 0;
                 if (!nodup && (w0 + u) * 32 + lane < nprod) {
@@ -1067,7 +1069,9 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                 const int cls = n == 2 ? 0 : n <= 4 ? 1 : n <= 8 ? 2 : n <= 16 ? 3 : n < kLongMin ? 4 : 5;
                 const int o = atomicAdd(&misc[1 + cls], 1);
                 // (the size beside the column's 12 bits)
-                if (cls == 0) {
+                if (!BRM_IN(P.cnt, o, cls <= 1 ? L::n_a : cls <= 3 ? L::n_b : L::n_c)) {
+                    continue;
+                } else if (cls == 0) {
                     lista[o] = (unsigned short)u;
                 } else if (cls == 1) {
                     lista[L::n_a - 1 - o] = (unsigned short)(u | ((n - 3) << 12));
@@ -1113,6 +1117,8 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                             int p = (int)(pk[u] & 0xfffu);
                             if (c[u])
                                 p = run[p] + c[u];
+                            if (!BRM_IN(P.cnt, p, kSegCap))
+                                continue;
                             vals[p] = vmul(av[q], bv[q]);
                             plist[p] = (unsigned short)((w0 + u) * 32 + lane);
                         }
@@ -1187,7 +1193,9 @@ __global__ void __launch_bounds__(kSegThreads, 3 * 256 / kSegThreads)
                         const int x = i ? rp + i : u;
                         const int l = plist[x];
                         const int r = wpre[l >> 5] + __popc(bmp[l >> 5] & ((1u << (l & 31)) - 1u));
-                        if (handoff) {
+                        if (!BRM_IN(P.cnt, r, len)) {
+                            continue;
+                        } else if (handoff) {
                             P.long_leaf[leo + r] = (unsigned short)leaf_of(l);
                             lval[leo + r] = vals[x];
                         } else {
