@@ -362,10 +362,14 @@ void plan_times_upper(brm_context ctx, brm_upper_timing *t)
 }
 
 // Products up to which a one-call Precise allocates C for every product (24
-// MB in float64) instead of waiting for nnz(C): one host round trip less where
-// a whole call takes about 100 us (the ER product of 2^20 products 0.205 ->
-// 0.114 ms with it and the launches saved).
+// MB in float64) instead of waiting for nnz(C): one host round trip less.  ER,
+// 64 products a row, waiting against not: 2^12 products 124 -> 105 us, 2^17 124 ->
+// 108, 2^20 146 -> 121, 2^21 160 -> 146, 2^22 199 -> 182, 2^24 588 -> 564.  It
+// saves 15 to 25 us at every size; the line is for the memory.
 constexpr unsigned long long kDeferProducts = 2ull << 20;
+// Such a C is handed over as it is while at most half of it, or less than
+// this many bytes, is room to spare; else it is copied to arrays of its size.
+constexpr size_t kDeferSpare = 1 << 20;
 
 // Few rows: the smaller rank classes go along in the launch of the largest
 // that has rows, as long as its groups of warps hold all rows at once (a
@@ -673,6 +677,36 @@ int read_counters(brm_context ctx)
     BRM_CK(cudaStreamSynchronize(ctx->stream));
     ctx->last_err = ctx->h_cnt->err;
     return device_err_status(ctx->h_cnt->err);
+}
+
+// C of a call that did not wait has room for `room` entries: exchanged for
+// arrays of its size where too much of it is to spare (kDeferSpare).  Without
+// memory for those it stays as it is.
+int fit_results(brm_context ctx, brm_dtype dtype, int room, int cnnz, int **ccol, void **cval)
+{
+    const size_t n = (size_t)std::max(cnnz, 1), v = vsize(dtype);
+    if (room <= 2ll * cnnz || (size_t)(room - cnnz) * (4 + v) < kDeferSpare)
+        return BRM_SUCCESS;
+    int *col = nullptr;
+    void *val = nullptr;
+    cudaError_t e = cudaMallocAsync((void **)&col, 4 * n, ctx->stream);
+    if (e == cudaSuccess)
+        e = cudaMallocAsync(&val, v * n, ctx->stream);
+    if (e == cudaSuccess && cnnz > 0)
+        e = cudaMemcpyAsync(col, *ccol, 4 * n, cudaMemcpyDeviceToDevice, ctx->stream);
+    if (e == cudaSuccess && cnnz > 0)
+        e = cudaMemcpyAsync(val, *cval, v * n, cudaMemcpyDeviceToDevice, ctx->stream);
+    if (e == cudaSuccess) {
+        std::swap(col, *ccol);
+        std::swap(val, *cval);
+    }
+    (void)cudaGetLastError();
+    if (col)
+        cudaFreeAsync(col, ctx->stream);
+    if (val)
+        cudaFreeAsync(val, ctx->stream);
+    BRM_CK(cudaStreamSynchronize(ctx->stream));
+    return BRM_SUCCESS;
 }
 
 int check_dtype(brm_dtype d) { return (d == BRM_F64 || d == BRM_F32) ? BRM_SUCCESS : BRM_ERR_INVALID_VALUE; }
@@ -1424,6 +1458,8 @@ static int precise_device_once(brm_context ctx, brm_dtype dtype, const brm_csr *
     ev_record(ctx, timed, kEvNum1);
     if (st == BRM_SUCCESS)
         st = deferred ? read_counters(ctx) : read_err(ctx);
+    if (st == BRM_SUCCESS && deferred)
+        st = fit_results(ctx, dtype, cnnz, (int)ctx->h_cnt->cnnz, &ccol, &cval);
     if (st != BRM_SUCCESS) {
         ctx->planned = ctx->planned && !deferred;
         cudaFreeAsync(crpt, ctx->stream);

@@ -1,5 +1,6 @@
 """What a call leaves allocated in the device's memory pool once its results are
-released: a batch's stacked operands go back with the call, when it fails too."""
+released: a batch's stacked operands go back with the call, when it fails too;
+and what a small result keeps: at most twice its size, or a megabyte more."""
 import ctypes as C
 import gc
 
@@ -44,4 +45,21 @@ def test_stacked_operands_go_back():
     with pytest.raises(brm.BrmError):
         ctx.batch_precise([(dA, B), (dbad, B)])
     assert pool_used() - before < 64 << 20
+    ctx.close()
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n", [4, 12, 14])  # 27-point stencil: up to 729 products for 125 entries
+def test_room_of_a_small_result(oracle_mod, n, dtype):
+    A = brm.gen_stencil27(n).astype(dtype)
+    R = oracle_mod.precise(A, A)
+    ctx = brm.Context()
+    dA = brm.DeviceCSR.from_host(A)
+    C_ = ctx.precise_device(dA, dA)  # (the context's own buffers)
+    del C_
+    before = pool_used()
+    C_ = ctx.precise_device(dA, dA)
+    size = len(R.col) * (4 + R.val.itemsize)
+    assert pool_used() - before <= 4 * (A.M + 1) + max(2 * size, size + (1 << 20)) + 4096
+    assert np.array_equal(C_.to_host().val, R.val) and np.array_equal(C_.to_host().col, R.col)
     ctx.close()
