@@ -206,7 +206,8 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
             (bin == kBinMidGroup && (long long)mx - mn >= (1ll << kMgRangeBits)) ||
             ((bin == kBinMidTile || bin == kBinMidTile2) &&
              (long long)mx - mn >= (1ll << kMtRangeBits)) ||
-            (bin == kBinMidGroup2 && (long long)mx - mn >= (1ll << kMg2RangeBits)))
+            (bin == kBinMidGroup2 && ((long long)mx - mn >= (1ll << kMg2RangeBits) ||
+                                      !merge_group2(f, (long long)mx - mn))))
             bin = (f <= P.mid_limit && 2 * nl <= P.mid_limit) ? kBinBatch : kBinHeavy;
         if (bin == kBinHeavy && a1 - a0 > kSegMaxK)
             bin = kBinMid;

@@ -52,7 +52,7 @@ constexpr int kMt2F = 128;        // second tile class: at most 128 products
 constexpr int kMtRangeBits = 25;
 constexpr int kMgF = 3072;
 constexpr int kMgRangeBits = 20;
-constexpr int kMg2F = 3072;       // second group class: 65 to 255 lists
+constexpr int kMg2F = 5888;       // second group class (two groups a CTA fit 2 CTAs an SM)
 constexpr int kMg2RangeBits = 19;
 // Rank rows (brm_midrank.cuh): rows of at most 64 lists whose products are
 // placed by population counts instead of sorted; they take precedence over the
@@ -87,6 +87,21 @@ __host__ __device__ inline int rank_class(long long f, int k, long long range)
     if (k <= kRkMaxK)
         return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f <= kRkF4 ? 7 : -1;
     return f > kRkF0 && f <= kRkF8 && k <= kRkSegMaxK && range < (1ll << kRkRangeBits0) ? 8 : -1;
+}
+// Rows of more than kMgF and at most kMg2F products that no rank class takes
+// (33 to 255 lists): merged by a group where columns are shared by several
+// products, else cut into segments, which pay by the column of several
+// products.  The column range tells them apart: A * A, matrices of k entries a
+// row spread over a band, one call, merged against segments:
+//   57 x 57 products  range 457: 1.13 ms, 1.52   1141: 1.10, 1.07   3421: 1.11, 0.88
+//   76 x 76           range 913: 1.09, 1.34      1521: 1.08, 1.26   2433: 1.07, 0.95
+//   100 x 35          range 401: 1.11, 1.50      1201: 1.09, 1.05
+// But a group's thread merges ceil(f / 128) products, and where that is 32 its
+// reads meet in one bank (57 % slower): those are cut whatever their range.
+constexpr int kMg2Share = 3;
+__host__ __device__ inline bool merge_group2(long long f, long long range)
+{
+    return f <= kMgF || (f >= kMg2Share * (range + 1) && (f + 127) / 128 != 32);
 }
 // Subsets of the mid-row kernels (they can run on different streams).
 constexpr int kMidGroups = 1;     // the batched mid rows and the four-warp group rows
