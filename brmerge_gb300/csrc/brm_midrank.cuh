@@ -702,8 +702,12 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
 // The classes from 1 on (their limits: kRk* in brm_plan.h; class 0:
 // brm_rankpack.cuh).  CTAs an SM by shared memory
 // or by registers, whichever ends first.  Most columns have several products
-// where rows are long and lists many (class 2: stencils, finite elements;
-// class 7), few where lists are long and few (power-law graphs).
+// where rows are long and lists many (class 2: stencils, finite elements), few
+// where lists are long and few (power-law graphs).  Rows of 33 to 64 lists are
+// both: class 7 holds those of more products than columns in their range, class
+// 9 the others.  Numeric phase, as class 7 and as class 9: 64 lists of 20 products
+// over 2^17 columns 0.82 and 0.67 ms (merged, before the rank rows: 0.71), 48 of 48
+// over 1537 columns 0.54 and 0.54, over 289 columns 0.38 and 0.41.
 using Rank1 = RankShape<kBinRank0 + 1, 12, 1, false, false, 19, 384, 4, 6>;
 using Rank2 = RankShape<kBinRank0 + 2, 6, 4, false, true, 19, 1536, 1, 10>;
 using Rank3 = RankShape<kBinRank0 + 3, 12, 4, false, false, 19, 1536, 1, 7>;
@@ -711,8 +715,10 @@ using Rank4 = RankShape<kBinRank0 + 4, 12, 8, false, false, 19, 3072, 1, 4>;
 using Rank5 = RankShape<kBinRank0 + 5, 12, 16, false, false, 19, 6144, 1, 2>;
 using Rank6 = RankShape<kBinRank0 + 6, 6, 4, true, false, 19, 768, 1, 8>;
 using Rank7 = RankShape<kBinRank0 + 7, 12, 8, true, true, 19, 3072, 1, 3>;
+using Rank9 = RankShape<kBinRank9, 12, 8, true, false, 19, 3072, 1, 3>;
 static_assert(Rank1::F == kRkF1 && Rank2::F == kRkF2 && Rank3::F == kRkF3 &&
-                  Rank4::F == kRkF4 && Rank5::F == kRkF5 && Rank6::F == kRkF2 && Rank7::F == kRkF4,
+                  Rank4::F == kRkF4 && Rank5::F == kRkF5 && Rank6::F == kRkF2 && Rank7::F == kRkF4 &&
+                  Rank9::F == kRkF4,
               "the analysis bins by these");
 
 template <typename T, int MODE, class S>

@@ -85,7 +85,7 @@ __host__ __device__ inline int rank_class(long long f, int k, long long range)
         return f <= kRkF1 ? 1 : f <= kRkF2 ? 2 : f <= kRkF3 ? 3 : f <= kRkF4 ? 4 : 5;
     }
     if (k <= kRkMaxK)
-        return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f <= kRkF4 ? 7 : -1;
+        return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f > kRkF4 ? -1 : f <= range ? 9 : 7;
     return f > kRkF0 && f <= kRkF8 && k <= kRkSegMaxK && range < (1ll << kRkRangeBits0) ? 8 : -1;
 }
 // Rows of more than kMgF and at most kMg2F products that no rank class takes
@@ -168,7 +168,8 @@ enum RowBin : int {
     kBinMidGroup2 = 10,  // four warps per row, longer rows (brm_midwarp.cuh)
     kBinRank0 = 11,      // rank rows, classes 0 .. 7 (brm_midrank.cuh)
     kBinSegRow = 19,     // rank rows of more than 64 lists, class 8 (brm_seg.cuh)
-    kNumBins = 20,
+    kBinRank9 = 20,      // rank rows, class 9 (brm_midrank.cuh)
+    kNumBins = 21,
 };
 
 constexpr int kRankClasses = kNumBins - kBinRank0;
@@ -355,7 +356,8 @@ constexpr unsigned kLiveMidRows = live_bit(kBinWarp) | live_bit(kBinBatch) | liv
 constexpr unsigned kLiveGroups = live_bit(kBinBatch) | live_bit(kBinMidGroup) |
                                  live_bit(kBinMidGroup2) | live_bit(kBinRank0 + 3) |
                                  live_bit(kBinRank0 + 4) | live_bit(kBinRank0 + 5) |
-                                 live_bit(kBinRank0 + 7) | live_bit(kBinSegRow);  // kMidGroups
+                                 live_bit(kBinRank0 + 7) | live_bit(kBinSegRow) |
+                                 live_bit(kBinRank9);  // kMidGroups
 inline bool plan_live(const PlanDev &P, unsigned bits) { return (P.live & bits) != 0; }
 
 // Capacities of a captured batch pipeline: every buffer sized by a count the

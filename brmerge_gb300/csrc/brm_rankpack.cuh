@@ -471,6 +471,7 @@ inline void launch_mid_warp(const CsrDev &A, const CsrDev &B, const PlanDev &P, 
             launch_mid_group<T, MODE, 4>(A, B, P, crpt, ccol, cval, num_sms, s);
         launch_mid_rank<T, MODE, Rank5>(A, B, P, crpt, ccol, cval, num_sms, s);
         launch_mid_rank<T, MODE, Rank7>(A, B, P, crpt, ccol, cval, num_sms, s);
+        launch_mid_rank<T, MODE, Rank9>(A, B, P, crpt, ccol, cval, num_sms, s);
         launch_mid_rank<T, MODE, Rank4>(A, B, P, crpt, ccol, cval, num_sms, s);
         launch_mid_rank<T, MODE, Rank3>(A, B, P, crpt, ccol, cval, num_sms, s);
     }
