@@ -71,8 +71,20 @@ constexpr int kRkNarrowK = 32;      // lists of the rows with one mask word a co
 constexpr int kRkMaxK = 64;
 constexpr int kRkF8 = 3072;         // class 8: more lists, by a segment's kernel
 constexpr int kRkSegMaxK = 255;
-constexpr int kRkRangeBits0 = 18;   // column range, classes 0 and 8
+constexpr int kRkRangeBits0 = 18;   // column range, class 0
+constexpr int kRkPackBits = 17;     // two rows of class 0 share a pack below
+constexpr int kRkRangeBits8 = 18;   // class 8
 constexpr int kRkRangeBits = 19;    // the others
+// A row of class 0 with a pack to itself pays all of the pack's fixed cost.
+// Numeric phase, 2^18 columns, 30 M products, packed and by the kernels that
+// sort: rows of 2 x 8 products 2.14 and 1.30 ms, 4 x 12 0.84 and 0.61, 8 x 8 0.64
+// and 0.50; 4 x 24 0.50 and 0.60, 16 x 7 0.51 and 0.63, 30 x 1 1.29 and 2.40, 16 x 2
+// 1.15 and 1.27.  So it takes more than kMtF products or, of at most 32 (a warp that
+// walks the lists one by one otherwise), 16 lists.
+__host__ __device__ inline bool rank_alone(long long f, int k)
+{
+    return f > kMtF || (f <= 32 && k >= 16);
+}
 // The class of a row of f products, k lists and columns within `range` of the
 // first, -1 where it has none.
 __host__ __device__ inline int rank_class(long long f, int k, long long range)
@@ -81,12 +93,12 @@ __host__ __device__ inline int rank_class(long long f, int k, long long range)
         return -1;
     if (k <= kRkNarrowK) {
         if (f <= kRkF0)
-            return range < (1ll << kRkRangeBits0) ? 0 : -1;
+            return range < (1ll << (rank_alone(f, k) ? kRkRangeBits0 : kRkPackBits)) ? 0 : -1;
         return f <= kRkF1 ? 1 : f <= kRkF2 ? 2 : f <= kRkF3 ? 3 : f <= kRkF4 ? 4 : 5;
     }
     if (k <= kRkMaxK)
         return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f > kRkF4 ? -1 : f <= range ? 9 : 7;
-    return f > kRkF0 && f <= kRkF8 && k <= kRkSegMaxK && range < (1ll << kRkRangeBits0) ? 8 : -1;
+    return f > kRkF0 && f <= kRkF8 && k <= kRkSegMaxK && range < (1ll << kRkRangeBits8) ? 8 : -1;
 }
 // Rows of more than kMgF and at most kMg2F products that no rank class takes
 // (33 to 255 lists): merged by a group where columns are shared by several

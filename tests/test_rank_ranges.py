@@ -1,6 +1,7 @@
-"""Rank rows at the lines that the column range draws: rows of 33 to 64 lists
-whose columns are as many as their products, one fewer and one more.  Against
-the oracle, bit for bit."""
+"""Rank rows at the lines that the column range draws: short rows on both sides
+of the range at which they have a pack to themselves (many and few of them, few
+and many lists), rows of 33 to 64 lists whose columns are as many as their
+products, one fewer and one more.  Against the oracle, bit for bit."""
 import numpy as np
 import pytest
 
@@ -30,6 +31,22 @@ def spread(ncols, n, rng):
     """n sorted distinct columns, the first and the last one among them."""
     inner = rng.choice(ncols - 2, n - 2, replace=False) + 1 if n > 2 else []
     return np.sort(np.r_[0, inner, ncols - 1][:n]).astype(np.int64)
+
+
+@pytest.mark.parametrize("rows", [3, 9000])
+@pytest.mark.parametrize("ncols", [1 << 16, (1 << 16) + 1025, 1 << 17, (1 << 17) + 1, 1 << 18,
+                                   (1 << 18) + 1])
+def test_short_rows(oracle_mod, ncols, rows):
+    """2 to 128 products of 2 to 32 lists, every row over all of the range."""
+    rng = np.random.default_rng(ncols)
+    lens = [2, 3, 4, 8, 16, 30, 31, 32]
+    B = csr(256, ncols, [spread(ncols, lens[i % 8], rng) for i in range(256)], rng, np.float64)
+    picks = [[0, 8], [5, 7], [7, 15], [0, 8, 16, 24, 32, 40, 48, 56], [1, 9, 17, 25, 33, 41, 49, 57, 65],
+             [6, 14], [7, 15, 23, 31], [4, 12, 20, 28, 36], list(range(0, 128, 8)),
+             list(range(0, 256, 8)), [3, 11, 19, 27], [7, 14]]
+    picks = [sorted(picks[i % len(picks)]) for i in range(rows)]
+    A = csr(rows, 256, [np.array(p) for p in picks], rng, np.float64)
+    check(oracle_mod, A, B)
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
