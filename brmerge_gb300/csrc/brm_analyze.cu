@@ -70,10 +70,12 @@ struct AnaBlock {
 };
 
 // One row by a group of TW lanes (lane gl of it, mask gm): its products, list
-// table entries (P.abs, P.alen), class and column range.  LONG: the first and
-// last column of every list (the column range) are taken in the same pass, so
-// that long rows are walked once.
-template <int TW, bool LONG, int RPB>
+// table entries (P.abs, P.alen), class and column range: the first and the
+// last column of every list, taken in the same pass (fetched afterwards, by way
+// of P.abs and P.alen, they added a round trip to memory: the symbolic phase of
+// 3.75 M rows of two lists 1.35 -> 1.17 ms without it and with the block's device
+// atomics in one phase; one call on 4096 uneven pairs 32.5 -> 31.4 ms)
+template <int TW, int RPB>
 __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, const PlanDev &P,
                                             int row, int slot, int gl, unsigned gm,
                                             AnaBlock<RPB> &S)
@@ -110,22 +112,20 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
                 }
             }
         }
-        if (LONG) {
-            int c0[UN], c1[UN];
+        int c0[UN], c1[UN];
 #pragma unroll
-            for (int u = 0; u < UN; u++) {
-                c0[u] = INT_MAX;
-                c1[u] = -1;
-                if (be[u] > bs[u]) {
-                    c0[u] = B.col[bs[u]];
-                    c1[u] = B.col[be[u] - 1];
-                }
+        for (int u = 0; u < UN; u++) {
+            c0[u] = INT_MAX;
+            c1[u] = -1;
+            if (be[u] > bs[u]) {
+                c0[u] = B.col[bs[u]];
+                c1[u] = B.col[be[u] - 1];
             }
+        }
 #pragma unroll
-            for (int u = 0; u < UN; u++) {
-                mn = min(mn, c0[u]);
-                mx = max(mx, c1[u]);
-            }
+        for (int u = 0; u < UN; u++) {
+            mn = min(mn, c0[u]);
+            mx = max(mx, c1[u]);
         }
 #pragma unroll
         for (int u = 0; u < UN; u++) {
@@ -171,29 +171,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
         bin = kBinMid;    // row CTA / spill path
     if (bin >= kBinWarp && bin != kBinMid) {
         // column range of the row for the segment planning and the mid rows'
-        // keys and bitmaps: the first and last column of every nonempty list
-        for (int jb = a0 + gl; !LONG && jb < a1; jb += 4 * TW) {
-            int c0[4], c1[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const int j = jb + u * TW;
-                c0[u] = INT_MAX;
-                c1[u] = -1;
-                if (j < a1) {
-                    const int len = P.alen[j];
-                    if (len > 0) {
-                        const int bs = P.abs[j];
-                        c0[u] = B.col[bs];
-                        c1[u] = B.col[bs + len - 1];
-                    }
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                mn = min(mn, c0[u]);
-                mx = max(mx, c1[u]);
-            }
-        }
+        // keys and bitmaps
         mn = grp_min<TW>(mn, gm);
         mx = grp_max<TW>(mx, gm);
         if (gl == 0)
@@ -284,19 +262,16 @@ __global__ void __launch_bounds__(kAnaThreads, 6) k_analyze(CsrDev A, CsrDev B, 
                 S.longs[atomicAdd(&S.nlong, 1)] = slot;
             continue;
         }
-        analyze_row<TW, false, RPB>(A, B, P, row, slot, gl, gm, S);
+        analyze_row<TW, RPB>(A, B, P, row, slot, gl, gm, S);
     }
     __syncthreads();
     if (TW < 32 && S.nlong) {
         for (int i = w; i < S.nlong; i += NW)
-            analyze_row<32, true, RPB>(A, B, P, row0 + S.longs[i], S.longs[i], lane, kFull, S);
+            analyze_row<32, RPB>(A, B, P, row0 + S.longs[i], S.longs[i], lane, kFull, S);
         __syncthreads();
     }
-    if (threadIdx.x < kNumBins)
-        S.base[threadIdx.x] =
-            S.cnt[threadIdx.x] ? atomicAdd(&P.cnt->bin_count[threadIdx.x], S.cnt[threadIdx.x]) : 0;
     // the rows' offsets: prefix over the block's slots (64-bit shared atomics
-    // a row took longer), one device atomic a total
+    // a row took longer), then one device atomic a total, and one a bin
     const int slot = threadIdx.x;
     unsigned long long fx = 0, sx = 0, fi = 0, si = 0;
     if (slot < (RPB + 31) / 32 * 32) {
@@ -313,19 +288,21 @@ __global__ void __launch_bounds__(kAnaThreads, 6) k_analyze(CsrDev A, CsrDev B, 
         }
     }
     __syncthreads();
-    if (threadIdx.x < 2) {
+    if (threadIdx.x < kNumBins)
+        S.base[threadIdx.x] =
+            S.cnt[threadIdx.x] ? atomicAdd(&P.cnt->bin_count[threadIdx.x], S.cnt[threadIdx.x]) : 0;
+    if (w == 1 && lane < 2) {
         unsigned long long t = 0;
         for (int i = 0; i < (RPB + 31) / 32; i++)
-            t += S.tot[i][threadIdx.x];
-        unsigned long long b =
-            t ? atomicAdd(threadIdx.x ? &P.cnt->mw_total : &P.cnt->total_flop, t) : 0ull;
+            t += S.tot[i][lane];
+        unsigned long long b = t ? atomicAdd(lane ? &P.cnt->mw_total : &P.cnt->total_flop, t) : 0ull;
         for (int i = 0; i < (RPB + 31) / 32; i++) {
-            const unsigned long long x = S.tot[i][threadIdx.x];
-            S.tot[i][threadIdx.x] = b;
+            const unsigned long long x = S.tot[i][lane];
+            S.tot[i][lane] = b;
             b += x;
         }
     }
-    if (threadIdx.x == 32) {
+    if (threadIdx.x == 64) {
         if (S.mid)
             atomicAdd(&P.cnt->mid_total, S.mid);
         if (S.max_k > 0)
