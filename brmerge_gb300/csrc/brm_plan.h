@@ -110,10 +110,16 @@ __host__ __device__ inline int rank_class(long long f, int k, long long range)
 //   100 x 35          range 401: 1.11, 1.50      1201: 1.09, 1.05
 // But a group's thread merges ceil(f / 128) products, and where that is 32 its
 // reads meet in one bank (57 % slower): those are cut whatever their range.
+// Rows that reach into a second planning chunk pay for the planning of both, which
+// up to kMg2WideF products costs more than it saves where it is not reused: 40 x 90
+// products over 2^19 columns, merged against segments: symbolic 0.48, 0.62, one call
+// 1.05, 1.13, Upper 1.10, 1.34 (numeric phase alone 0.83, 0.49).
 constexpr int kMg2Share = 3;
+constexpr int kMg2WideF = 31 * 128;
 __host__ __device__ inline bool merge_group2(long long f, long long range)
 {
-    return f <= kMgF || (f >= kMg2Share * (range + 1) && (f + 127) / 128 != 32);
+    return f <= kMgF || (f >= kMg2Share * (range + 1) && (f + 127) / 128 != 32) ||
+           (f <= kMg2WideF && range >= (1ll << kRkRangeBits8));
 }
 // Subsets of the mid-row kernels (they can run on different streams).
 constexpr int kMidGroups = 1;     // the batched mid rows and the four-warp group rows

@@ -1,7 +1,8 @@
 """Rank rows at the lines that the column range draws: short rows on both sides
 of the range at which they have a pack to themselves (many and few of them, few
 and many lists), rows of 33 to 64 lists whose columns are as many as their
-products, one fewer and one more.  Against the oracle, bit for bit."""
+products, one fewer and one more, rows of 3073 to 3969 products that reach into a
+second planning chunk.  Against the oracle, bit for bit."""
 import numpy as np
 import pytest
 
@@ -58,3 +59,12 @@ def test_columns_as_many_as_products(oracle_mod, lists, products, dtype):
         B = csr(lists, ncols, [spread(ncols, n, rng) for n in lens], rng, dtype)
         A = csr(1, lists, [np.arange(lists)], rng, dtype)
         check(oracle_mod, A, B)
+
+
+@pytest.mark.parametrize("products", [3073, 3968, 3969])
+@pytest.mark.parametrize("ncols", [1 << 18, (1 << 18) + 1, 1 << 19])
+def test_second_planning_chunk(oracle_mod, ncols, products):
+    rng = np.random.default_rng(products)
+    lens = np.full(40, products // 40) + (np.arange(40) < products % 40)
+    B = csr(40, ncols, [spread(ncols, n, rng) for n in lens], rng, np.float64)
+    check(oracle_mod, csr(1, 40, [np.arange(40)], rng, np.float64), B)
