@@ -561,10 +561,13 @@ struct RowPart {
     const int *seg_list = nullptr;
 };
 
-// Bytes of the long-column scratch for `elems` products.
+// Columns of the long-column scratch for `elems` products (a column has at least
+// kLongMin), and its bytes.
+long long long_cols(long long elems) { return elems / brm::kLongMin + 1024; }
+
 size_t long_bytes(long long elems, brm_dtype dtype)
 {
-    const long long cols = elems / 8 + 1024;
+    const long long cols = long_cols(elems);
     return a256(sizeof(brm::LongCol) * (size_t)cols) + a256(2 * (size_t)elems + 2) +
            vsize(dtype) * (size_t)elems + 8;
 }
@@ -621,7 +624,7 @@ int numeric_launch(brm_context ctx, brm_dtype dtype, bool upper, const brm_csr *
         // long-column scratch: at most kLongElems products (columns beyond it
         // are reduced inside the segment kernel)
         const long long elems = std::min<long long>((long long)sz.total_flop, ctx->long_scratch);
-        const long long cols = elems / 8 + 1024;
+        const long long cols = long_cols(elems);
         const size_t b_col = a256(sizeof(brm::LongCol) * (size_t)cols);
         const size_t b_leaf = a256(2 * (size_t)elems + 2);
         BRM_TRY(grow(ctx, ctx->longbuf, long_bytes(elems, dtype)));

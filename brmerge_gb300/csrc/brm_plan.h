@@ -151,6 +151,7 @@ static_assert(kRkF8 <= kSegCap, "rank rows of class 8 are a segment's size");
 constexpr int kSegCut = kSegCap * 3 / 4;
 constexpr int kSegMaxCut = kSegCap * 7 / 8;
 constexpr int kSegMaxK = 65535;           // leaf index stored in 16 bits
+constexpr int kLongMin = 33;              // products of a column handed to the column reducer
 constexpr int kHugeFlop = 16 * kSegCap;   // heavy rows planned first (longest first)
 constexpr int kMaxParts = 16;             // row parts of a numeric phase run part by part
 constexpr int kPlanWordsLog2 = 13;
@@ -387,7 +388,7 @@ struct PipeCaps {
     long long b_rows;       // rows of the stacked B
     long long nnz_b;        // entries of the stacked B
     long long cols;         // columns of the stacked B
-    long long products;     // intermediate products (bounds nnz(C) and the mid-row scratch)
+    long long products;     // intermediate products (bounds nnz(C); with nnz_a the mid-row scratch)
     long long seg_slots;    // heavy-row segment descriptors
     long long table;        // split-table entries
     long long spill_bytes;  // spill scratch

@@ -536,7 +536,6 @@ __global__ void __launch_bounds__(256) k_split(CsrDev A, CsrDev B, PlanDev P)
 // ---------------------------------------------------------------------------
 // 3. segment kernel
 // ---------------------------------------------------------------------------
-constexpr int kLongMin = 33;  // columns with this many products are handed to the column reducer
 constexpr int kLongMax = kSegCap / kLongMin + 1;
 constexpr int kSegPWords = kSegCap / 32;  // words of a bitmap over a segment's products
 static_assert(kSegCap % 32 == 0 && kSegPWords <= 96, "p-bitmap prefix: three words per lane");
