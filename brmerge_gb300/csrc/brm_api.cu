@@ -377,9 +377,6 @@ constexpr size_t kDeferSpare = 1 << 20;
 // another class a little more than in theirs).
 void plan_rank_spans(brm::PlanDev &P, const brm::Counters &c, int num_sms)
 {
-    // rows of each narrow class on one SM at a time (brm_midrank.cuh; class 0 on
-    // its own has no smaller one to take)
-    constexpr int kRows[6] = {40, 24, 10, 7, 4, 2};
     std::memset(P.rank_span, 0, sizeof(P.rank_span));
     P.rank_taken = 0;
     auto take = [&](int lo, int hi) {  // classes lo .. hi: true when one takes them all
@@ -390,7 +387,7 @@ void plan_rank_spans(brm::PlanDev &P, const brm::Counters &c, int num_sms)
             if (c.bin_count[brm::kBinRank0 + k])
                 top = k;
         }
-        if (top < 0 || rows > (long long)num_sms * kRows[top])
+        if (top < 0 || rows > (long long)num_sms * brm::kRkRows[top])
             return top < 0;
         P.rank_span[top] = top - lo;
         for (int k = lo; k < top; k++)

@@ -72,7 +72,8 @@ struct RankShape {
     static constexpr int NT = 32 * G;
     static constexpr int THREADS = NT * GROUPS;
     static constexpr int F = 32 * G * NP;
-    static constexpr int CLAIM = F <= kRkF0 ? 8 : F <= kRkF1 ? 4 : F <= kRkF2 ? 2 : 1;
+    static constexpr int CLAIM = F <= kRkF1 ? 4 : F <= kRkF2 ? 2 : 1;
+    static constexpr int SM_ROWS = GROUPS * CTAS;  // rows of an SM at a time
     static constexpr int KM = WIDE ? 64 : 32;
     static constexpr int MW = WIDE ? 2 : 1;          // mask words a column
     static constexpr int NSUM = 1 << (RANGE - 10);   // summary words of the widest row
@@ -720,6 +721,10 @@ static_assert(Rank1::F == kRkF1 && Rank2::F == kRkF2 && Rank3::F == kRkF3 &&
                   Rank4::F == kRkF4 && Rank5::F == kRkF5 && Rank6::F == kRkF2 && Rank7::F == kRkF4 &&
                   Rank9::F == kRkF4,
               "the analysis bins by these");
+static_assert(Rank1::SM_ROWS == kRkRows[1] && Rank2::SM_ROWS == kRkRows[2] &&
+                  Rank3::SM_ROWS == kRkRows[3] && Rank4::SM_ROWS == kRkRows[4] &&
+                  Rank5::SM_ROWS == kRkRows[5],
+              "plan_rank_spans counts by these");
 
 template <typename T, int MODE, class S>
 inline void launch_mid_rank(const CsrDev &A, const CsrDev &B, const PlanDev &P, const int *crpt,

@@ -75,6 +75,8 @@ constexpr int kRkRangeBits0 = 18;   // column range, class 0
 constexpr int kRkPackBits = 17;     // two rows of class 0 share a pack below
 constexpr int kRkRangeBits8 = 18;   // class 8
 constexpr int kRkRangeBits = 19;    // the others
+// Rows of each narrow class that one SM works on at a time (class 0: eight a warp).
+constexpr int kRkRows[6] = {256, 24, 10, 7, 4, 2};
 // A row of class 0 with a pack to itself pays all of the pack's fixed cost.
 // Numeric phase, 2^18 columns, 30 M products, packed and by the kernels that
 // sort: rows of 2 x 8 products 2.14 and 1.30 ms, 4 x 12 0.84 and 0.61, 8 x 8 0.64

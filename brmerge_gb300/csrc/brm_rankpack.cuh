@@ -43,6 +43,7 @@ struct PackShape {
     static constexpr size_t bytes = per_warp * WARPS;
     static_assert(o_mask % 16 == 0 && o_tab % 16 == 0, "16-byte accesses");
     static_assert(kRkF0 <= F && kRkNarrowK <= KM, "one row fits");
+    static_assert(ROWS * WARPS * CTAS == kRkRows[0], "plan_rank_spans counts by this");
     static_assert(ROWS * kRkF0 < 2048 && ROWS * kRkNarrowK < 512 && ROWS * NSUM < 4096,
                   "packed sums");
 };

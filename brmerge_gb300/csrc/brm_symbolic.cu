@@ -45,7 +45,8 @@ void launch_symbolic(const CsrDev &A, const CsrDev &B, const PlanDev &P, int num
         const size_t psm = PlanLayout::bytes;
         cudaFuncSetAttribute(k_heavy_plan<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)psm);
-        k_heavy_plan<0><<<num_sms * 3, kPlanThreads, psm, s>>>(A, B, P);
+        // (as many CTAs an SM as its shared memory holds)
+        k_heavy_plan<0><<<num_sms * 2, kPlanThreads, psm, s>>>(A, B, P);
         count_launch();
     }
     if (!plan_live(P, live_bit(kBinMid)))

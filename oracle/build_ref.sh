@@ -1,13 +1,13 @@
 #!/bin/bash
 # Builds the reference's BRMerge path unmodified from its own sources into
-# oracle/_ref/libbrm_ref.so (git-ignored).  Needs the reference tree; the
-# default location is /root/reference (override with BRM_REFERENCE_DIR).
+# oracle/_ref/libbrm_ref.so (git-ignored).  Needs the reference tree, at
+# BRM_REFERENCE_DIR or beside this repository.
 # Only spgemm.h (header-only kernels), src/Timings.cpp and src/CSR.cpp (the
 # MatrixMarket reader) are compiled; two
 # small shims in oracle/ref_shim replace TBB malloc and the x86 TSC timer.
 set -euo pipefail
 HERE="$(cd "$(dirname "$0")" && pwd)"
-REF="${BRM_REFERENCE_DIR:-/root/reference}/BRMerge-SpGEMM"
+REF="${BRM_REFERENCE_DIR:-$HERE/../../reference}/BRMerge-SpGEMM"
 if [ ! -f "$REF/inc/spgemm.h" ]; then
   echo "reference sources not found at $REF; skipping" >&2
   exit 3
