@@ -1,6 +1,6 @@
 """What a call leaves allocated in the device's memory pool once its results are
 released: a batch's stacked operands go back with the call, when it fails too;
-and what a small result keeps: at most twice its size, or a megabyte more."""
+and what a small result keeps: at most twice its size, or 8 MiB more."""
 import ctypes as C
 import gc
 
@@ -60,6 +60,6 @@ def test_room_of_a_small_result(oracle_mod, n, dtype):
     before = pool_used()
     C_ = ctx.precise_device(dA, dA)
     size = len(R.col) * (4 + R.val.itemsize)
-    assert pool_used() - before <= 4 * (A.M + 1) + max(2 * size, size + (1 << 20)) + 4096
+    assert pool_used() - before <= 4 * (A.M + 1) + max(2 * size, size + (8 << 20)) + 4096
     assert np.array_equal(C_.to_host().val, R.val) and np.array_equal(C_.to_host().col, R.col)
     ctx.close()
