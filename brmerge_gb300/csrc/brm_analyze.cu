@@ -177,7 +177,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
         if (gl == 0)
             P.crange[row] = make_int2(mn, mx);
         // rows placed by rank, where their lists and column range allow
-        const int rc = rank_class(f, a1 - a0, (long long)mx - mn);
+        const int rc = rank_class(f, a1 - a0, (long long)mx - mn, M);
         if (rc > 0 || (rc == 0 && !P.any_order))
             bin = kBinRank0 + rc;
         if ((bin == kBinMidWarp && (long long)mx - mn >= (1ll << kMwRangeBits)) ||
@@ -185,7 +185,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
             ((bin == kBinMidTile || bin == kBinMidTile2) &&
              (long long)mx - mn >= (1ll << kMtRangeBits)) ||
             (bin == kBinMidGroup2 && ((long long)mx - mn >= (1ll << kMg2RangeBits) ||
-                                      !merge_group2(f, (long long)mx - mn))))
+                                      !merge_group2(f, (long long)mx - mn, M))))
             bin = (f <= P.mid_limit && 2 * nl <= P.mid_limit) ? kBinBatch : kBinHeavy;
         if (bin == kBinHeavy && a1 - a0 > kSegMaxK)
             bin = kBinMid;

@@ -82,24 +82,32 @@ constexpr int kRkRows[6] = {256, 24, 10, 7, 4, 2};
 // sort: rows of 2 x 8 products 2.14 and 1.30 ms, 4 x 12 0.84 and 0.61, 8 x 8 0.64
 // and 0.50; 4 x 24 0.50 and 0.60, 16 x 7 0.51 and 0.63, 30 x 1 1.29 and 2.40, 16 x 2
 // 1.15 and 1.27.  So it takes more than kMtF products or, of at most 32 (a warp that
-// walks the lists one by one otherwise), 16 lists.
-__host__ __device__ inline bool rank_alone(long long f, int k)
+// walks the lists one by one otherwise), 16 lists.  A matrix of few rows keeps
+// them all in the pack: launches of two more classes cost more than it does
+// (numeric phase, 5000 rows of up to 10 entries over 150,000 columns 60 us packed
+// and 72 split up, 40,000 of up to 12 127 and 105).
+constexpr int kRkAloneRows = 16384;
+__host__ __device__ inline bool rank_alone(long long f, int k, int rows)
 {
-    return f > kMtF || (f <= 32 && k >= 16);
+    return f > kMtF || (f <= 32 && k >= 16) || rows < kRkAloneRows;
 }
+// Classes 7 and 9 are told apart where there are rows enough for both (1000 rows of
+// up to 46 entries over 1000 columns: numeric phase 94 us in one class, 112 in two;
+// 5000 of up to 58 over 5000: 209 and 193).
+constexpr int kRkSplitRows = 4096;
 // The class of a row of f products, k lists and columns within `range` of the
-// first, -1 where it has none.
-__host__ __device__ inline int rank_class(long long f, int k, long long range)
+// first, in a matrix of `rows` rows; -1 where it has none.
+__host__ __device__ inline int rank_class(long long f, int k, long long range, int rows)
 {
     if (f <= 0 || f > kRkF5 || range < 0 || range >= (1ll << kRkRangeBits))
         return -1;
     if (k <= kRkNarrowK) {
         if (f <= kRkF0)
-            return range < (1ll << (rank_alone(f, k) ? kRkRangeBits0 : kRkPackBits)) ? 0 : -1;
+            return range < (1ll << (rank_alone(f, k, rows) ? kRkRangeBits0 : kRkPackBits)) ? 0 : -1;
         return f <= kRkF1 ? 1 : f <= kRkF2 ? 2 : f <= kRkF3 ? 3 : f <= kRkF4 ? 4 : 5;
     }
     if (k <= kRkMaxK)
-        return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f > kRkF4 ? -1 : f <= range ? 9 : 7;
+        return f <= kRkF0 ? -1 : f <= kRkF2 ? 6 : f > kRkF4 ? -1 : f <= range && rows >= kRkSplitRows ? 9 : 7;
     return f > kRkF0 && f <= kRkF8 && k <= kRkSegMaxK && range < (1ll << kRkRangeBits8) ? 8 : -1;
 }
 // Rows of more than kMgF and at most kMg2F products that no rank class takes
@@ -112,16 +120,21 @@ __host__ __device__ inline int rank_class(long long f, int k, long long range)
 //   100 x 35          range 401: 1.11, 1.50      1201: 1.09, 1.05
 // But a group's thread merges ceil(f / 128) products, and where that is 32 its
 // reads meet in one bank (57 % slower): those are cut whatever their range.
+// A group takes about 120 us for a row, so a matrix of few rows (two or three for a
+// group) is cut too: R-MAT n=1500, 8 entries a row, numeric phase 0.15 and 0.27 ms.
 // Rows that reach into a second planning chunk pay for the planning of both, which
 // up to kMg2WideF products costs more than it saves where it is not reused: 40 x 90
 // products over 2^19 columns, merged against segments: symbolic 0.48, 0.62, one call
 // 1.05, 1.13, Upper 1.10, 1.34 (numeric phase alone 0.83, 0.49).
 constexpr int kMg2Share = 3;
 constexpr int kMg2WideF = 31 * 128;
-__host__ __device__ inline bool merge_group2(long long f, long long range)
+constexpr int kMg2Rows = 2048;
+__host__ __device__ inline bool merge_group2(long long f, long long range, int rows)
 {
-    return f <= kMgF || (f >= kMg2Share * (range + 1) && (f + 127) / 128 != 32) ||
-           (f <= kMg2WideF && range >= (1ll << kRkRangeBits8));
+    return f <= kMgF ||
+           (rows >= kMg2Rows &&
+            ((f >= kMg2Share * (range + 1) && (f + 127) / 128 != 32) ||
+             (f <= kMg2WideF && range >= (1ll << kRkRangeBits8))));
 }
 // Subsets of the mid-row kernels (they can run on different streams).
 constexpr int kMidGroups = 1;     // the batched mid rows and the four-warp group rows

@@ -23,6 +23,7 @@ def check(oracle_mod, A, B):
 
 
 def csr(rows, ncols, cols, rng, dtype):
+    cols = list(cols) + [np.zeros(0, np.int64)] * (rows - len(cols))  # empty rows
     rpt = np.concatenate([[0], np.cumsum([len(c) for c in cols])]).astype(np.int32)
     return brm.CSR(rows, ncols, rpt, np.concatenate(cols).astype(np.int32),
                    rng.uniform(-1, 1, rpt[-1])).astype(dtype)
@@ -34,7 +35,7 @@ def spread(ncols, n, rng):
     return np.sort(np.r_[0, inner, ncols - 1][:n]).astype(np.int64)
 
 
-@pytest.mark.parametrize("rows", [3, 9000])
+@pytest.mark.parametrize("rows", [3, 16383, 16384])
 @pytest.mark.parametrize("ncols", [1 << 16, (1 << 16) + 1025, 1 << 17, (1 << 17) + 1, 1 << 18,
                                    (1 << 18) + 1])
 def test_short_rows(oracle_mod, ncols, rows):
@@ -51,13 +52,14 @@ def test_short_rows(oracle_mod, ncols, rows):
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("rows", [4095, 4096])
 @pytest.mark.parametrize("lists,products", [(33, 769), (64, 770), (40, 1600), (48, 2999), (64, 3072)])
-def test_columns_as_many_as_products(oracle_mod, lists, products, dtype):
+def test_columns_as_many_as_products(oracle_mod, lists, products, rows, dtype):
     rng = np.random.default_rng(products)
     for ncols in (products - 1, products, products + 1, products + 2, 3 * products):
         lens = np.full(lists, products // lists) + (np.arange(lists) < products % lists)
         B = csr(lists, ncols, [spread(ncols, n, rng) for n in lens], rng, dtype)
-        A = csr(1, lists, [np.arange(lists)], rng, dtype)
+        A = csr(rows, lists, [np.arange(lists)], rng, dtype)
         check(oracle_mod, A, B)
 
 
@@ -67,4 +69,5 @@ def test_second_planning_chunk(oracle_mod, ncols, products):
     rng = np.random.default_rng(products)
     lens = np.full(40, products // 40) + (np.arange(40) < products % 40)
     B = csr(40, ncols, [spread(ncols, n, rng) for n in lens], rng, np.float64)
-    check(oracle_mod, csr(1, 40, [np.arange(40)], rng, np.float64), B)
+    for rows in (2047, 2048):
+        check(oracle_mod, csr(rows, 40, [np.arange(40)], rng, np.float64), B)

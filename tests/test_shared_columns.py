@@ -1,7 +1,8 @@
 """Rows of 3073 to 5888 products and 33 to 255 lists: merged by a group of warps
 where the column range holds at most a third as many columns as the row has
-products (and a thread's share is not 32 products), cut into segments elsewhere;
-both sides of every line, against the oracle, bit for bit."""
+products (and a thread's share is not 32 products) and the matrix has 2048 rows,
+cut into segments elsewhere; both sides of every line, against the oracle, bit for
+bit."""
 import numpy as np
 import pytest
 
@@ -19,16 +20,17 @@ ROWS = [(60, 3600, 1200, True), (60, 3600, 1201, False), (33, 3073, 1024, True),
         (100, 5000, 401, True), (200, 4600, 100000, False)]
 
 
-def one_row(lists, products, ncols, dtype, seed):
-    """A of one row with a B row of its own for each entry; the first and the
-    last column are used."""
+def one_row(lists, products, ncols, dtype, seed, rows=2048):
+    """A of one row (and empty ones) with a B row of its own for each entry; the
+    first and the last column are used."""
     rng = np.random.default_rng(seed)
     lens = np.full(lists, products // lists) + (np.arange(lists) < products % lists)
     cols = [np.sort(rng.choice(ncols, n, replace=False)) for n in lens]
     cols[0][0], cols[0][-1] = 0, ncols - 1
     rpt = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
-    A = brm.CSR(1, lists, np.array([0, lists], np.int32), np.arange(lists, dtype=np.int32),
-                rng.uniform(-1, 1, lists))
+    a_rpt = np.full(rows + 1, lists, np.int32)
+    a_rpt[0] = 0
+    A = brm.CSR(rows, lists, a_rpt, np.arange(lists, dtype=np.int32), rng.uniform(-1, 1, lists))
     B = brm.CSR(lists, ncols, rpt, np.concatenate(cols).astype(np.int32),
                 rng.uniform(-1, 1, products))
     return A.astype(dtype), B.astype(dtype)
@@ -49,4 +51,16 @@ def test_both_routes(oracle_mod, lists, products, ncols, merged, dtype):
     assert (launches <= 4) == merged, launches
     assert_same_csr(ctx.precise(dA, dB).to_host(), R, "split")
     assert_same_csr(ctx.upper(dA, dB).to_host(), R, "upper")
+    ctx.close()
+
+
+def test_few_rows_are_cut(oracle_mod):
+    A, B = one_row(60, 3600, 1200, np.float64, seed=1, rows=2047)
+    R = oracle_mod.precise(A, B)
+    ctx = brm.Context()
+    dA, dB = brm.DeviceCSR.from_host(A), brm.DeviceCSR.from_host(B)
+    before = _native.lib().brm_kernel_launches()
+    C = ctx.precise_device(dA, dB)
+    assert _native.lib().brm_kernel_launches() - before > 4
+    assert_same_csr(C.to_host(), R, "one call")
     ctx.close()
