@@ -110,6 +110,11 @@ struct brm_context_s {
     // ordered by part (device), and a second stream that copies finished
     // parts of C back while the next part computes
     DevBuf partbuf;
+    // table and stacked operands of a batch: in use by a call, or kept for the next
+    // one up to batch_keep bytes
+    DevBuf batchbuf;
+    bool batch_busy = false;
+    size_t batch_keep = 4ull << 30;
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t part_ev[brm::kMaxParts] = {};
     // a second compute stream: the mid rows run on it beside the heavy-row
@@ -150,6 +155,18 @@ int cuda_status(cudaError_t e)
 
 size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// cudaMallocAsync on the context's stream; a kept batch buffer makes room.
+cudaError_t pool_alloc(brm_context ctx, void **p, size_t bytes)
+{
+    cudaError_t e = cudaMallocAsync(p, bytes, ctx->stream);
+    if (e == cudaErrorMemoryAllocation && ctx->batchbuf.p && !ctx->batch_busy) {
+        (void)cudaGetLastError();
+        brm::batch_release(ctx);
+        e = cudaMallocAsync(p, bytes, ctx->stream);
+    }
+    return e;
+}
+
 // Grows a context buffer to at least `bytes` (25 % headroom when it grows
 // again), stream-ordered on the context's stream: the old block is released
 // after the work queued before it, and neither call waits for the device, so
@@ -167,7 +184,7 @@ int grow(brm_context ctx, DevBuf &b, size_t bytes)
         b.p = nullptr;
         b.cap = 0;
     }
-    BRM_CK(cudaMallocAsync(&b.p, want, ctx->stream));
+    BRM_CK(pool_alloc(ctx, &b.p, want));
     b.cap = want;
     return BRM_SUCCESS;
 }
@@ -218,7 +235,7 @@ int ensure_workspace(brm_context ctx, int M)
         ctx->ws = nullptr;
     }
     size_t bytes = workspace_bytes(M);
-    BRM_CK(cudaMallocAsync(&ctx->ws, bytes, ctx->stream));
+    BRM_CK(pool_alloc(ctx, &ctx->ws, bytes));
     ctx->ws_bytes = bytes;
     ctx->ws_M = M;
     size_t m = (size_t)(M > 0 ? M : 1);
@@ -1003,6 +1020,30 @@ int host_call(bool upper, const int *arpt, const int *acol, const T *aval, const
 
 cudaStream_t brm::context_stream(brm_context ctx) { return ctx->stream; }
 
+int brm::batch_scratch(brm_context ctx, size_t bytes, void **p)
+{
+    ctx->batch_busy = true;
+    BRM_TRY(grow(ctx, ctx->batchbuf, bytes));
+    *p = ctx->batchbuf.p;
+    return BRM_SUCCESS;
+}
+
+void brm::batch_done(brm_context ctx, bool idle)
+{
+    ctx->batch_busy = false;
+    if (!idle || ctx->batchbuf.cap > ctx->batch_keep)
+        batch_release(ctx);
+}
+
+void brm::batch_release(brm_context ctx)
+{
+    if (ctx->batchbuf.p)  // behind the work queued so far
+        cudaFreeAsync(ctx->batchbuf.p, ctx->stream);
+    ctx->batchbuf = DevBuf();
+}
+
+void brm::set_context_keep(brm_context ctx, size_t bytes) { ctx->batch_keep = bytes; }
+
 int brm::context_num_sms(brm_context ctx) { return ctx->num_sms; }
 
 int brm::numeric_async(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
@@ -1269,6 +1310,7 @@ int brm_destroy(brm_context ctx)
     if (ctx->fork.join)
         cudaEventDestroy(ctx->fork.join);
     release(ctx->partbuf);
+    release(ctx->batchbuf);
     delete ctx;
     return BRM_SUCCESS;
 }
@@ -1428,7 +1470,7 @@ static int precise_device_once(brm_context ctx, brm_dtype dtype, const brm_csr *
     const bool timed = timing != nullptr;
     double t0 = now_sec();
     int *crpt = nullptr;
-    BRM_CK(cudaMallocAsync((void **)&crpt, 4 * ((size_t)A->M + 1), ctx->stream));
+    BRM_CK(pool_alloc(ctx, (void **)&crpt, 4 * ((size_t)A->M + 1)));
     double t1 = now_sec();
     ctx->planned = false;
     int st = plan_phase(ctx, A, B, crpt, false, timed, dtype, true, any_order);
@@ -1442,9 +1484,9 @@ static int precise_device_once(brm_context ctx, brm_dtype dtype, const brm_csr *
     int *ccol = nullptr;
     void *cval = nullptr;
     double t2 = now_sec();
-    cudaError_t e = cudaMallocAsync((void **)&ccol, 4 * (size_t)(cnnz > 0 ? cnnz : 1), ctx->stream);
+    cudaError_t e = pool_alloc(ctx, (void **)&ccol, 4 * (size_t)(cnnz > 0 ? cnnz : 1));
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&cval, vsize(dtype) * (size_t)(cnnz > 0 ? cnnz : 1), ctx->stream);
+        e = pool_alloc(ctx, &cval, vsize(dtype) * (size_t)(cnnz > 0 ? cnnz : 1));
     if (e != cudaSuccess) {
         ctx->planned = ctx->planned && !deferred;
         cudaFreeAsync(crpt, ctx->stream);
@@ -1512,7 +1554,7 @@ static int upper_device_once(brm_context ctx, brm_dtype dtype, const brm_csr *A,
     BRM_TRY(grow(ctx, ctx->bar_val, (size_t)ctx->h_cnt->total_flop * vsize(dtype)));
     double t2 = now_sec();
     int *crpt = nullptr;
-    BRM_CK(cudaMallocAsync((void **)&crpt, 4 * ((size_t)A->M + 1), ctx->stream));
+    BRM_CK(pool_alloc(ctx, (void **)&crpt, 4 * ((size_t)A->M + 1)));
     ev_record(ctx, timed, kEvNum0);
     int st = numeric_launch(ctx, dtype, true, A, B, nullptr, (int *)ctx->bar_col.p, ctx->bar_val.p);
     ev_record(ctx, timed, kEvNum1);
@@ -1537,9 +1579,9 @@ static int upper_device_once(brm_context ctx, brm_dtype dtype, const brm_csr *A,
     double t3 = now_sec();
     int *ccol = nullptr;
     void *cval = nullptr;
-    cudaError_t e = cudaMallocAsync((void **)&ccol, 4 * (size_t)(cnnz > 0 ? cnnz : 1), ctx->stream);
+    cudaError_t e = pool_alloc(ctx, (void **)&ccol, 4 * (size_t)(cnnz > 0 ? cnnz : 1));
     if (e == cudaSuccess)
-        e = cudaMallocAsync(&cval, vsize(dtype) * (size_t)(cnnz > 0 ? cnnz : 1), ctx->stream);
+        e = pool_alloc(ctx, &cval, vsize(dtype) * (size_t)(cnnz > 0 ? cnnz : 1));
     if (e != cudaSuccess) {
         cudaFreeAsync(crpt, ctx->stream);
         if (ccol)

@@ -195,16 +195,13 @@ __global__ void __launch_bounds__(256) k_batch_local_rpt(const BatchDims *dims,
 
 namespace {
 
-// A block of the stream-ordered pool that goes back when the call ends, behind
-// the work queued so far.
-struct StreamBlock {
-    void *p = nullptr;
-    cudaStream_t s = nullptr;
-    ~StreamBlock()
-    {
-        if (p)
-            cudaFreeAsync(p, s);
-    }
+// The context's batch buffer in use by a call (batch_scratch .. batch_done).
+struct BatchHold {
+    brm_context ctx;
+    bool idle = false;  // the call has waited for its work
+    explicit BatchHold(brm_context c) : ctx(c) {}
+    BatchHold(const BatchHold &) = delete;
+    ~BatchHold() { brm::batch_done(ctx, idle); }
 };
 
 size_t a256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -379,23 +376,20 @@ int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A,
         return BRM_SUCCESS;
     cudaStream_t s = brm::context_stream(ctx);
     const size_t vb = dtype == BRM_F64 ? 8 : 4;
-    // the table, A_bd and B_bd, in one block: three of their own took the pool
-    // 10 ms of remapping a call (4096 pairs, 3.7 GB) where it had fragmented.  Kept
-    // in the context between calls the block saved no time (32.6 ms either way)
+    // the table, A_bd and B_bd, in a buffer that the context keeps up to a bound:
+    // allocated on each call they take the pool 2 to 10 ms of remapping where it has
+    // fragmented (4096 pairs, 3.7 GB: 36.3 ms against 33.3)
     const size_t a_rpt = a256(4 * (size_t)(ra + 1)), a_col = a256(4 * (size_t)std::max(na, 1LL));
     const size_t b_rpt = a256(4 * (size_t)(rb + 1)), b_col = a256(4 * (size_t)std::max(nb, 1LL));
     const size_t a_val = a256(vb * (size_t)std::max(na, 1LL)), t_all = a256(h.t.bytes);
-    StreamBlock buf;
-    buf.s = s;
-    if (cudaMallocAsync(&buf.p,
-                        t_all + a_rpt + a_col + a_val + b_rpt + b_col +
-                            vb * (size_t)std::max(nb, 1LL),
-                        s) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return BRM_ERR_ALLOC;
-    }
-    char *abd = (char *)buf.p + t_all, *bbd = abd + a_rpt + a_col + a_val;
-    const BatchTable t = table_layout(buf.p, n);
+    void *buf = nullptr;
+    BatchHold hold(ctx);
+    int st = brm::batch_scratch(
+        ctx, t_all + a_rpt + a_col + a_val + b_rpt + b_col + vb * (size_t)std::max(nb, 1LL), &buf);
+    if (st != BRM_SUCCESS)
+        return st;
+    char *abd = (char *)buf + t_all, *bbd = abd + a_rpt + a_col + a_val;
+    const BatchTable t = table_layout(buf, n);
     int *A_rpt = (int *)abd, *A_col = (int *)(abd + a_rpt);
     void *A_val = abd + a_rpt + a_col;
     int *B_rpt = (int *)bbd, *B_col = (int *)(bbd + b_rpt);
@@ -417,7 +411,7 @@ int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A,
     int *crpt = nullptr, *ccol = nullptr;
     void *cval = nullptr;
     int cnnz = 0;
-    int st = brm_precise_device(ctx, dtype, &Abd, &Bbd, &crpt, &ccol, &cval, &cnnz, nullptr);
+    st = brm_precise_device(ctx, dtype, &Abd, &Bbd, &crpt, &ccol, &cval, &cnnz, nullptr);
     if (st != BRM_SUCCESS)
         return st;
     int *lrpt = nullptr;
@@ -443,6 +437,7 @@ int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A,
         brm_device_free(ctx, lrpt);
         return (!hf || !hr) ? BRM_ERR_ALLOC : BRM_ERR_CUDA;
     }
+    hold.idle = true;
     std::memcpy(hr, h.t.off, sizeof(long long) * (size_t)(n + 1));
     out->row_off = hr;
     out->nnz_off = hf;
@@ -785,6 +780,7 @@ int brm_batch_caps_for(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A
     BRM_STATUS_TRY(brm_batch_precise(ctx, dtype, n, A, B, &b));  // plans the sample
     const brm::Counters c = brm::last_plan_counters(ctx);
     brm_batch_free(ctx, &b);
+    brm::batch_release(ctx);  // the batches go through the pipeline's own buffers
     const brm::BatchDims d = *h.t.dims;
     auto up = [&](long long x, long long lo) {
         const double v = std::ceil((double)x * headroom);

@@ -14,6 +14,14 @@ namespace brm {
 // The stream and SM count of a context (brm_api.cu).
 cudaStream_t context_stream(brm_context ctx);
 int context_num_sms(brm_context ctx);
+// The context's buffer for a batch's table and stacked operands, at least
+// `bytes`, until batch_done.  An idle one (no work queued on it) is kept for the
+// next batch up to the context's bound (4 GiB; set_context_keep) and until another
+// allocation of the context fails; batch_release gives it back.
+int batch_scratch(brm_context ctx, size_t bytes, void **p);
+void batch_done(brm_context ctx, bool idle);
+void batch_release(brm_context ctx);
+void set_context_keep(brm_context ctx, size_t bytes);
 
 // brm_numeric without its closing synchronisation (it only enqueues work on
 // the context stream, so it can be captured into a CUDA graph once every

@@ -509,6 +509,7 @@ int brm_server_create(const brm_server_config *cfg, brm_server *out)
             break;
         }
         brm_set_stream(c, s);
+        brm::set_context_keep(c, 0);  // the memory cap counts what a batch holds
         if (xw)
             st = brm::set_context_priority(c, hi);
         if (st == BRM_SUCCESS && srv->partitioned)

@@ -265,7 +265,9 @@ typedef struct brm_batch {
  * bit-identical to brm_precise_device(A_i, B_i).  No counterpart in the
  * reference (one pair per call).  The concatenated rows and entries must
  * each fit int32 (else BRM_ERR_CAPACITY); nnz of all C_i together must fit
- * int32 (else BRM_ERR_OVERFLOW). */
+ * int32 (else BRM_ERR_OVERFLOW).  The stacked operands are a copy of all A_i and
+ * B_i; of at most 4 GiB, the context keeps their memory for its next batch, until
+ * it is destroyed or another of its allocations needs it. */
 int brm_batch_precise(brm_context ctx, brm_dtype dtype, int n, const brm_csr *A, const brm_csr *B,
                       brm_batch *out);
 int brm_batch_free(brm_context ctx, brm_batch *batch);

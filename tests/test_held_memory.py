@@ -1,5 +1,6 @@
-"""What a call leaves allocated in the device's memory pool once its results are
-released: a batch's stacked operands go back with the call, when it fails too;
+"""What calls leave allocated in the device's memory pool once their results are
+released: a batch's stacked operands up to a bound, none of them in a server's
+workers, after an error or after a pipeline's capacities were taken from a sample;
 and what a small result keeps: at most twice its size, or 8 MiB more."""
 import ctypes as C
 import gc
@@ -13,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 
 def pool_used():
-    """Bytes in use in the current device's default pool (driver API)."""
+    """Bytes in use in the current device's default pool (driver API); what a
+    plain cudaFree gives back stays in this count."""
     import torch
     torch.cuda.synchronize()
     gc.collect()
@@ -24,10 +26,10 @@ def pool_used():
     return used.value
 
 
-def test_stacked_operands_go_back():
+@pytest.fixture(scope="module")
+def pair():
+    """16 rows of A use 4 rows of a B of 96 MB: 5120 products."""
     import torch
-    ctx = brm.Context()
-    # 16 rows of A use 4 rows of a B of 96 MB, twice: 192 MB stacked, 10240 products
     rows, per = 100_000, 80
     rpt = torch.arange(rows + 1, device="cuda", dtype=torch.int32) * per
     col = torch.arange(per, device="cuda", dtype=torch.int32).repeat(rows)
@@ -35,17 +37,44 @@ def test_stacked_operands_go_back():
     A = brm.CSR(16, rows, np.arange(17, dtype=np.int32) * 4,
                 np.tile(np.arange(4, dtype=np.int32), 16), np.ones(64))
     bad = brm.CSR(16, rows, A.rpt, A.col.copy(), A.val)
-    bad.col[63] = 2 * rows + 5
-    dA, dbad = brm.DeviceCSR.from_host(A), brm.DeviceCSR.from_host(bad)
+    bad.col[63] = 100 * rows
+    return brm.DeviceCSR.from_host(A), brm.DeviceCSR.from_host(bad), B
+
+
+SMALL = 64 << 20  # what else the context may hold here
+
+
+def test_stacked_operands_of_a_context(pair):
+    A, bad, B = pair
     before = pool_used()
-    res = ctx.batch_precise([(dA, B), (dA, B)])
-    assert float(res[1].val.sum()) == 16 * 4 * per
-    del res
-    assert pool_used() - before < 64 << 20
+    ctx = brm.Context()
+    for n, kept in ((2, 192_000_000), (60, 0), (2, 192_000_000)):  # 5.8 GB: above the bound
+        res = ctx.batch_precise([(A, B)] * n)
+        assert float(res[-1].val.sum()) == 16 * 4 * 80
+        del res
+        assert 0 <= pool_used() - before - kept < SMALL, n
     with pytest.raises(brm.BrmError):
-        ctx.batch_precise([(dA, B), (dbad, B)])
-    assert pool_used() - before < 64 << 20
+        ctx.batch_precise([(A, B), (bad, B)])
+    assert pool_used() - before < SMALL
+    ctx.batch_precise([(A, B)] * 2)
+    held = pool_used()
+    # (the pipeline's own pool buffers are 64 MiB of spill scratch and small ones)
+    pipe = ctx.batch_pipe([(A, B)] * 2)
+    assert pool_used() - held < -192_000_000 + (64 << 20) + SMALL
+    pipe.close()
     ctx.close()
+
+
+def test_stacked_operands_of_a_server(pair):
+    A, _, B = pair
+    before = pool_used()
+    srv = brm.Server(workers=1)
+    for t in [srv.submit(A, B) for _ in range(3)]:
+        C_, _ = srv.wait(t, timeout=60.0)
+        assert float(C_.val.sum()) == 16 * 4 * 80
+        del C_
+    assert pool_used() - before < SMALL
+    srv.close()
 
 
 @pytest.mark.parametrize("dtype", [np.float64, np.float32])
