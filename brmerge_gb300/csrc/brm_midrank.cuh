@@ -33,7 +33,7 @@
 // warp), so the merge kernels' partly filled warps of additions cost as much
 // as their instructions.  The 27-point stencil on 61x47x53, numeric phase
 // (152 k rows, 729 products and 125 columns inside): merge kernel 2.08 ms,
-// 16 warp instructions a product; this one 0.85 ms, 7 a product, the FP64
+// 16 warp instructions a product; this one 0.85 ms, 8 a product, the FP64
 // unit 57 % busy.  Rows of 3..128 products of 512 uneven pairs: 1.84 ->
 // 0.91 ms.
 //

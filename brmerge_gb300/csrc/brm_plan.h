@@ -41,9 +41,9 @@ constexpr int kMidMaxRows = kMidCap / (kWarpMaxFlop + 1) + 2;
 // kMidMaxK A entries) in their own class.  All take precedence over the
 // batched mid rows and over the segmented heavy rows.  Holding the first two
 // classes to 64 lists keeps their merge-tree stacks at seven levels and
-// their kernels within 80 registers without spills.  Longer rows are cut into
-// segments (merged in one piece up to 5888 products they took 178 us of R-MAT
-// n=2^18, the whole call 2.24 -> 2.18 ms without).
+// their kernels within 80 registers without spills.  Rows of more than kMgF
+// products are merged only where merge_group2 says so; in R-MAT n=2^18 they
+// are cut (merged they took 178 us, the whole call 2.24 -> 2.18 ms without).
 constexpr int kMwF = 768;
 constexpr int kMwMaxK = 64;
 constexpr int kMwRangeBits = 22;
@@ -56,9 +56,9 @@ constexpr int kMg2F = 5888;       // second group class (two groups a CTA fit 2 
 constexpr int kMg2RangeBits = 19;
 // Rank rows (brm_midrank.cuh): rows of at most 64 lists whose products are
 // placed by population counts instead of sorted; they take precedence over the
-// tile, warp and group rows above, which keep the wide ranges (the bitmap's
-// summary outgrows a row's shared memory there).  Class 8 takes the rows of 65
-// to 255 lists through the segment kernel, a row a segment.
+// tile, warp and group rows above, which keep the wide ranges (one level of
+// summary words outgrows a row's shared memory there).  Class 8 takes the rows
+// of 65 to 255 lists through the segment kernel, a row a segment.
 // R-MAT n=2^18: rows of 769..3072 products 0.35 -> 0.28 ms.
 // The most products of a row of each class:
 constexpr int kRkF0 = 128;

@@ -40,7 +40,7 @@
 // 17.9 k segments: 1147 us when every product's column, value, leaf, rank and
 // turn were staged in shared memory (111 KB, two CTAs an SM), 915 with the
 // columns in registers, 747 with columns of up to 32 products reduced in
-// place by groups of lanes (825 since rows of 3073 to 5888 products are cut
+// place by groups of lanes (825 since its rows of 3073 to 5888 products are cut
 // into segments too, 178 us less elsewhere).  A lane a column instead of a group
 // took 979 us with 12 % fewer instructions, the size lists claimed once a warp by
 // ballots 883, the next segment's split entries prefetched 831.
