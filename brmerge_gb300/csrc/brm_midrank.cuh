@@ -703,8 +703,9 @@ __global__ void __launch_bounds__(S::THREADS, S::CTAS)
 // The classes from 1 on (their limits: kRk* in brm_plan.h; class 0:
 // brm_rankpack.cuh).  CTAs an SM by shared memory
 // or by registers, whichever ends first.  Most columns have several products
-// where rows are long and lists many (class 2: stencils, finite elements), few
-// where lists are long and few (power-law graphs).  Rows of 33 to 64 lists are
+// where rows are long and lists many (class 2: stencils, finite elements; of
+// distinct columns, 20 lists of 30 products over 2^17 columns, it takes 0.20 ms,
+// merged 0.29), few where lists are long and few (power-law graphs).  Rows of 33 to 64 lists are
 // both: class 7 holds those of more products than columns in their range, class
 // 9 the others.  Numeric phase, as class 7 and as class 9: 64 lists of 20 products
 // over 2^17 columns 0.82 and 0.67 ms (merged, before the rank rows: 0.71), 48 of 48
