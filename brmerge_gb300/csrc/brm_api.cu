@@ -386,9 +386,9 @@ void plan_times_upper(brm_context ctx, brm_upper_timing *t)
 constexpr unsigned long long kDeferProducts = 2ull << 20;
 // Such a C is handed over as it is while at most half of it, or less than
 // this many bytes, is room to spare; else it is copied to arrays of its size.
-// The copy takes the 15 us that not waiting has saved (27-point stencil on 8^3
-// points, 2.4 MB to spare of 2.9: 100 -> 115 us), so small results keep their room.
-constexpr size_t kDeferSpare = 8 << 20;
+// The copy takes the 15 us that not waiting has saved (27-point stencil on 12^3
+// points, 9.4 MB to spare of 11.3: 147 -> 162 us), so most results keep their room.
+constexpr size_t kDeferSpare = 16 << 20;
 
 // Few rows: the smaller rank classes go along in the launch of the largest
 // that has rows, as long as its groups of warps hold all rows at once (a

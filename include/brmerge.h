@@ -187,7 +187,7 @@ int brm_numeric(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_cs
 /* BRMerge-Precise: symbolic then numeric.  Outputs are allocated from the
  * context's stream-ordered pool; release them with brm_device_free.  Of a
  * product of at most 2^21 products *ccol and *cval may have room for more than
- * *cnnz entries: at most twice as many, or less than 8 MiB more.
+ * *cnnz entries: at most twice as many, or less than 16 MiB more.
  * Mirrors brmerge_precise (spgemm.h:468-471).  timing may be NULL. */
 int brm_precise_device(brm_context ctx, brm_dtype dtype, const brm_csr *A, const brm_csr *B,
                        int **crpt, int **ccol, void **cval, int *cnnz,
