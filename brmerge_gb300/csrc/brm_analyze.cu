@@ -185,7 +185,7 @@ __device__ __forceinline__ void analyze_row(const CsrDev &A, const CsrDev &B, co
             ((bin == kBinMidTile || bin == kBinMidTile2) &&
              (long long)mx - mn >= (1ll << kMtRangeBits)) ||
             (bin == kBinMidGroup2 && ((long long)mx - mn >= (1ll << kMg2RangeBits) ||
-                                      !merge_group2(f, (long long)mx - mn, M))))
+                                      !merge_group2(f, (long long)mx - mn, M, A.nnz))))
             bin = (f <= P.mid_limit && 2 * nl <= P.mid_limit) ? kBinBatch : kBinHeavy;
         if (bin == kBinHeavy && a1 - a0 > kSegMaxK)
             bin = kBinMid;

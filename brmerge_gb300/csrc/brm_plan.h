@@ -120,8 +120,10 @@ __host__ __device__ inline int rank_class(long long f, int k, long long range, i
 //   100 x 35          range 401: 1.11, 1.50      1201: 1.09, 1.05
 // But a group's thread merges ceil(f / 128) products, and where that is 32 its
 // reads meet in one bank (57 % slower): those are cut whatever their range.
-// A group takes about 120 us for a row, so a matrix of few rows (two or three for a
-// group) is cut too: R-MAT n=1500, 8 entries a row, numeric phase 0.15 and 0.27 ms.
+// A group takes about 120 us for a row, so a few such rows among others are cut too:
+// R-MAT n=1500, 8 entries a row, numeric phase 0.15 and 0.27 ms.  Merged are those of
+// matrices of many rows or of rows that long on average (kMg2MeanK entries: 1143 rows of
+// 100 x 35 products, numeric phase 0.19 ms merged, 0.23 cut).
 // Rows that reach into a second planning chunk pay for the planning of both, which
 // up to kMg2WideF products costs more than it saves where it is not reused: 40 x 90
 // products over 2^19 columns, merged against segments: symbolic 0.48, 0.62, one call
@@ -129,10 +131,11 @@ __host__ __device__ inline int rank_class(long long f, int k, long long range, i
 constexpr int kMg2Share = 3;
 constexpr int kMg2WideF = 31 * 128;
 constexpr int kMg2Rows = 2048;
-__host__ __device__ inline bool merge_group2(long long f, long long range, int rows)
+constexpr int kMg2MeanK = 32;
+__host__ __device__ inline bool merge_group2(long long f, long long range, int rows, int nnz)
 {
     return f <= kMgF ||
-           (rows >= kMg2Rows &&
+           ((rows >= kMg2Rows || nnz > (long long)kMg2MeanK * rows) &&
             ((f >= kMg2Share * (range + 1) && (f + 127) / 128 != 32) ||
              (f <= kMg2WideF && range >= (1ll << kRkRangeBits8))));
 }

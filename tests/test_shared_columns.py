@@ -1,7 +1,7 @@
 """Rows of 3073 to 5888 products and 33 to 255 lists: merged by a group of warps
 where the column range holds at most a third as many columns as the row has
-products (and a thread's share is not 32 products) and the matrix has 2048 rows,
-cut into segments elsewhere; both sides of every line, against the oracle, bit for
+products (and a thread's share is not 32 products) and the matrix has 2048 rows or
+more than 32 entries a row, cut into segments elsewhere; both sides of every line, against the oracle, bit for
 bit."""
 import numpy as np
 import pytest
@@ -54,13 +54,14 @@ def test_both_routes(oracle_mod, lists, products, ncols, merged, dtype):
     ctx.close()
 
 
-def test_few_rows_are_cut(oracle_mod):
-    A, B = one_row(60, 3600, 1200, np.float64, seed=1, rows=2047)
+@pytest.mark.parametrize("rows,merged", [(2047, False), (2, False), (1, True)])
+def test_few_rows(oracle_mod, rows, merged):
+    A, B = one_row(60, 3600, 1200, np.float64, seed=1, rows=rows)
     R = oracle_mod.precise(A, B)
     ctx = brm.Context()
     dA, dB = brm.DeviceCSR.from_host(A), brm.DeviceCSR.from_host(B)
     before = _native.lib().brm_kernel_launches()
     C = ctx.precise_device(dA, dB)
-    assert _native.lib().brm_kernel_launches() - before > 4
+    assert (_native.lib().brm_kernel_launches() - before <= 4) == merged
     assert_same_csr(C.to_host(), R, "one call")
     ctx.close()
